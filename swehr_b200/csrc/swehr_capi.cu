@@ -253,6 +253,14 @@ static void make_devparams(const swehr_params *p, const swehr_inputs *in, const 
         P.a13[k] = 13.95 * p->nu / in->ds[k];
         P.a13sq[k] = P.a13[k] * P.a13[k];
     }
+    {
+        auto in_range = [](double c) { return c >= 0x1p-100 && c <= 0x1p100; };
+        bool ok = P.divk_ok && in_range(P.g) && in_range(P.rhos) && in_range(P.rhow) && in_range(P.h0) && P.F >= 0 &&
+                  P.F <= 0x1p100;
+        for (int k = 0; k < p->sclass; k++)
+            ok = ok && in_range(P.a13sq[k]) && in_range(P.ds[k]) && P.c109s >= 0 && P.c109s <= 0x1p100;
+        P.fast_ok = ok;
+    }
     fill_realc(P, P.kd);
     fill_realc(P, P.kf);
 }

@@ -64,7 +64,8 @@ __global__ void __launch_bounds__(NB_THREADS) k_cfl_noalloc(const DevParams P, c
     double smax = 0;
     for (int64_t c = first + threadIdx.x; c < first + NOALLOC_CELLS_PER_BLOCK && c < total; c += blockDim.x) {
         const int i = (int)(c / P.ny) + 1, j = (int)(c % P.ny) + 1;
-        const double s = wave_cell_g<PolicyF64, double>(P, src, i, j, inh, inhv, lagged_gz<PolicyF64>(P, zp, i, j));
+        PolicyF64 pp;
+        const double s = wave_cell_g<PolicyF64, double>(pp, P, src, i, j, inh, inhv, lagged_gz<PolicyF64>(P, zp, i, j));
         smax = (s > smax) ? s : smax;
     }
     __shared__ double red[NB_THREADS / 32];

@@ -62,7 +62,10 @@ struct DevParams {
      * thetas - theta0, for exact division by remainder correction (divk);
      * divk_ok: every constant divisor lies in [2^-100, 2^100] */
     double inv_J, inv_h0x6, inv_p2, inv_dtheta;
-    int32_t divk_ok, pad_divk;
+    int32_t divk_ok;
+    /* every constant a branch-free sequence takes untested is positive and of
+     * middling size (FastF64); 0: the plain operators throughout */
+    int32_t fast_ok;
     double storm_peak, storm_r2, storm_x0, storm_y0, storm_vx, storm_vy;
     double ds[16], pf[16], a13[16], a13sq[16];
     RealC<double> kd;     /* the constants above, for templated kernels */

@@ -13,6 +13,8 @@
  */
 #include <cuda_runtime.h>
 
+#include "swehr_ieee.h"
+
 static const int PROBE_THREADS = 256;
 static const int PROBE_CHAINS = 8;
 
@@ -63,4 +65,43 @@ extern "C" int swehr_probe_fp64_peak(double *tflops)
     const cudaError_t err = cudaGetLastError();
     *tflops = best;
     return err == cudaSuccess ? 0 : 4;
+}
+
+/* swehr_probe_ieee: the branch-free sequences of swehr_ieee.h beside the
+ * compiler's operators and the plain bodies of swehr_math.h, element by
+ * element, for the tests.  op: 0 a/b, 1 root of a, 2 exp(a), 3 a^b, 4
+ * cos(atan a); host arrays of n doubles.  refused: 1 where the operands are
+ * not ones the sequences take. */
+__global__ void k_ieee(int op, const double *__restrict__ a, const double *__restrict__ b, long long n, double *fast,
+                       double *plain, double *refused)
+{
+    for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x) {
+        const double x = a[q], y = b[q];
+        bool ok = true;
+        switch (op) {
+        case 0: fast[q] = sw_quot(x, y, sw_rcp(y)); plain[q] = x / y; ok = sw_mid_or_zero(x) && sw_mid_pos(y); break;
+        case 1: fast[q] = sw_sqrt_mid(x); plain[q] = sw_sqrt_pow(x); ok = sw_mid_pos(x) || sw_zero(x); break;
+        case 2: fast[q] = sw_exp_mid(x, 0.0); plain[q] = sw_exp(x); ok = sw_exp_fits(x); break;
+        case 3: fast[q] = sw_pow_mid(x, y, &ok); plain[q] = sw_pow(x, y); break;
+        default: fast[q] = sw_cos_atan_mid(x, &ok); plain[q] = sw_cos_atan(x); break;
+        }
+        refused[q] = !ok;
+    }
+}
+
+extern "C" int swehr_probe_ieee(int op, const double *a, const double *b, long long n, double *fast, double *plain,
+                                double *refused)
+{
+    if (!a || !b || !fast || !plain || !refused || n < 1 || op < 0 || op > 4) return 1;
+    const size_t bytes = (size_t)n * sizeof(double);
+    double *d = nullptr;
+    if (cudaMalloc(&d, 5 * bytes) != cudaSuccess) return 2;
+    cudaMemcpy(d, a, bytes, cudaMemcpyHostToDevice);
+    cudaMemcpy(d + n, b, bytes, cudaMemcpyHostToDevice);
+    k_ieee<<<592, 256>>>(op, d, d + n, n, d + 2 * n, d + 3 * n, d + 4 * n);
+    cudaMemcpy(fast, d + 2 * n, bytes, cudaMemcpyDeviceToHost);
+    cudaMemcpy(plain, d + 3 * n, bytes, cudaMemcpyDeviceToHost);
+    cudaMemcpy(refused, d + 4 * n, bytes, cudaMemcpyDeviceToHost);
+    cudaFree(d);
+    return cudaGetLastError() == cudaSuccess ? 0 : 3;
 }

@@ -33,6 +33,7 @@
 #include "swehr_device.cuh"
 #include "swehr_faces.cuh"
 #include "swehr_kernels.h"
+#include "swehr_ieee.h"
 #include "swehr_tma.cuh"
 
 #include <cuda_pipeline_primitives.h>
@@ -63,15 +64,28 @@ inline namespace SWEHR_TILE_NS {
 #define N_FY (T_I * (T_J + 1))
 #define TILE_THREADS 256
 
-/* ------------------------------------------------------------ policies --- */
+/* ------------------------------------------------------------ policies ---
+ * A policy is the arithmetic of a form: PolicyF64 and PolicyF32 name the two
+ * forms' kernels; Fast is the arithmetic their cells, faces and wave speeds
+ * run on.  Fast of the plain form collects in ok whether every operand was
+ * one its branch-free sequences are exact for; where it was not, the caller
+ * computes the cell (face, vector) again with Plain. */
+struct FastF64;
 struct PolicyF64 {
     typedef double R;
+    typedef FastF64 Fast;
+    typedef PolicyF64 Plain;
+    static constexpr bool kGuarded = false;
+    static constexpr bool ok = true;
     static constexpr int kMinBlocks = 2;      /* CTAs per SM the update kernel is register-budgeted for */
     static constexpr int kBatchMinBlocks = 2; /* ... and the batched update kernel */
-    /* the class loop of the cell update kept rolled: its unrolled body (eight
-     * inline exp and division sequences) costs more in instruction fetch
-     * than unrolling gains (measured: update -4 % rolled) */
-    static constexpr bool kRollClasses = true;
+    static constexpr bool kRollClasses = true;    /* one division and exp sequence in the code, not eight */
+    typedef double Recip;
+    static __device__ __forceinline__ R recip(R b) { return b; }
+    static __device__ __forceinline__ R quot(R a, R b) { return a / b; }
+    static __device__ __forceinline__ R quotz(R a, R b) { return divz(a, b); }
+    static __device__ __forceinline__ R quotn(R a, R b) { return divz(a, b); }
+    static __device__ __forceinline__ R root1(R x) { return sw_sqrt_pow(x); }
     /* wave pass: two cells per thread (16-byte loads) at 3 CTAs per SM (80
      * registers); measured against one cell per thread at 5 CTAs: wet steps
      * -0.06 ms, early steps +0.03 ms per 4096^2 step */
@@ -156,8 +170,115 @@ struct PolicyF64 {
     }
 };
 
+/* The plain form's arithmetic for ordinary operands: the IEEE results of
+ * PolicyF64 from the branch-free sequences of swehr_ieee.h, so that the
+ * compiler interleaves a cell's independent quotients, roots and exponentials
+ * and quotients by one divisor share its reciprocal.  ok is cleared by an
+ * operand outside [2^-500, 2^501) that is not a zero dividend or radicand, a
+ * divisor that is not positive, an exponent beyond 700 or a NaN; the caller
+ * then computes again with PolicyF64.  Constants need no test here:
+ * DevParams::fast_ok says that the run's are in range (ok starts as it). */
+struct FastF64 {
+    typedef double R;
+    typedef FastF64 Fast;
+    typedef PolicyF64 Plain;
+    static constexpr bool kGuarded = true;
+    /* rolled where the class count is not the kernel's own: sixteen unrolled
+     * bodies would not fit the instruction cache */
+    static constexpr bool kRollClasses = false;
+    static constexpr bool kKnownResults = true;
+    bool ok;
+    struct Recip {
+        R b, y;
+    };
+    static __device__ __forceinline__ Recip recip(R b) { return Recip{b, sw_rcp(b)}; }
+    __device__ __forceinline__ R quot(R a, const Recip &r)
+    {
+        ok &= sw_mid_pos(r.b) & sw_mid_or_zero(a);
+        return sw_quot(a, r.b, r.y);
+    }
+    __device__ __forceinline__ R quotz(R a, const Recip &r) { return quot(a, r); }
+    /* a quotient whose dividend may be a NaN that is there to stay (the
+     * deposit of the inflow row, which the reference's 0/0 at t = 0 makes) */
+    __device__ __forceinline__ R quotn(R a, const Recip &r)
+    {
+        ok &= sw_mid_pos(r.b) & (sw_mid_or_zero(a) | (a != a));
+        return sw_quot(a, r.b, r.y);
+    }
+    __device__ __forceinline__ R div(R a, R b) { return quot(a, recip(b)); }
+    __device__ __forceinline__ R divz(R a, R b) { return div(a, b); }
+    __device__ __forceinline__ R divk(R a, R c, R yc, int)
+    {
+        ok &= sw_mid_or_zero(a);
+        return sw_quot(a, c, yc);
+    }
+    __device__ __forceinline__ R sqrtp(R x)
+    {
+        ok &= sw_mid_pos(x) | sw_zero(x);
+        return sw_sqrt_mid(x);
+    }
+    __device__ __forceinline__ R sqrtz(R x) { return sqrtp(x); }
+    /* root of a sum of squares plus one */
+    __device__ __forceinline__ R root1(R x)
+    {
+        ok &= sw_small(x);
+        return sw_sqrt_mid(x);
+    }
+    __device__ __forceinline__ R pow(R x, R y)
+    {
+        if (y == 0.5) return sqrtp(x);
+        if (y == 1.0) return x;
+        if (y == 2.0) return x * x;
+        if (y == 4.0) {
+            const R ax = fabs(x);
+            ok &= (ax >= 0x1p-250) & (ax <= 0x1p250);
+            return sw_pow4(x);
+        }
+        return sw_pow_mid(x, y, &ok);
+    }
+    __device__ __forceinline__ R exp(R x)
+    {
+        ok &= sw_exp_fits(x);
+        return sw_exp_mid(x, 0.0);
+    }
+    __device__ __forceinline__ R cos_atan(R x)
+    {
+        return sw_cos_atan_mid(x, &ok);
+    }
+    static __device__ __forceinline__ R qnan() { return PolicyF64::qnan(); }
+    /* E3 and E4 as in PolicyF64: an exact zero m gives the zero of the
+     * quotient's sign without the quotient */
+    __device__ __forceinline__ R e3_term(R num, R J, R yJ, int, R m)
+    {
+        ok &= sw_small(num);
+        if (m == 0)
+            return PolicyF64::zero_xor(__double_as_longlong(num) ^ __double_as_longlong(m));
+        return divk(num, J, yJ, 1) * m;
+    }
+    __device__ __forceinline__ R e4_term(R A, const Recip &T, R F, const Recip &e, R m)
+    {
+        if (m == 0) {
+            ok &= sw_small(A) & sw_mid_pos(T.b) & sw_mid_pos(e.b);
+            return PolicyF64::zero_xor(__double_as_longlong(A) ^ __double_as_longlong(F) ^ __double_as_longlong(m));
+        }
+        return quot(quot(A, T) * F, e) * m;
+    }
+    /* A^2 and c = 1.09 (rhos/rhow - 1) gz d are in range with the run's
+     * constants: gz = g / root, root >= 1 tested where it was formed */
+    static __device__ __forceinline__ R settle(R A, R A2, R c) { return sw_sqrt_mid(A2 + c) - A; }
+    __device__ __forceinline__ double dep_of(double M, const DevParams &P)
+    {
+        ok &= sw_mid_or_zero(M) | (M != M);
+        return sw_quot(M, P.rhos, P.inv_rhos);
+    }
+};
+
 struct PolicyF32 {
     typedef float R;
+    typedef PolicyF32 Fast;
+    typedef PolicyF32 Plain;
+    static constexpr bool kGuarded = false;
+    static constexpr bool ok = true;
     static constexpr int kMinBlocks = 3;
     /* the batched update reads its scenario's parameters from shared memory,
      * not the constant bank, and needs more registers: at 3 CTAs per SM it
@@ -199,6 +320,12 @@ struct PolicyF32 {
     static __device__ __forceinline__ R cos_atan(R x) { return rsqrtf(1.f + x * x); }
     static __device__ __forceinline__ R sin_atan(R x) { return x * rsqrtf(1.f + x * x); }
     static __device__ __forceinline__ R div(R a, R b) { return __fdividef(a, b); }
+    typedef float Recip;
+    static __device__ __forceinline__ R recip(R b) { return b; }
+    static __device__ __forceinline__ R quot(R a, R b) { return div(a, b); }
+    static __device__ __forceinline__ R quotz(R a, R b) { return div(a, b); }
+    static __device__ __forceinline__ R quotn(R a, R b) { return div(a, b); }
+    static __device__ __forceinline__ R root1(R x) { return sqrtp(x); }
     static __device__ __forceinline__ R divz(R a, R b) { return div(a, b); }
     static __device__ __forceinline__ R sqrtz(R x) { return sqrtp(x); }
     static __device__ __forceinline__ R divk(R a, R c, R, int) { return div(a, c); }
@@ -213,22 +340,30 @@ struct PolicyF32 {
     static __device__ __forceinline__ double dep_of(double M, const DevParams &P) { return M * P.inv_rhos; }
 };
 
+/* the arithmetic of a routine that recomputes with Plain where it has to */
+template <class F>
+__device__ __forceinline__ F make_fast(const DevParams &P)
+{
+    if constexpr (F::kGuarded) return F{P.fast_ok != 0};
+    else return F{};
+}
+
 /* hllc of SWEHR.c:327-409 with the velocities already formed
  * (nl = normal/ul, tl = tangential/vl; both 0 for a dry side) and the left
  * side's sqrt(g hl) given.  Same operations as hllc(). */
 template <class PP>
-__device__ __forceinline__ typename PP::R hllc_v(typename PP::R hl, typename PP::R hr, typename PP::R nl,
+__device__ __forceinline__ typename PP::R hllc_v(PP &pp, typename PP::R hl, typename PP::R hr, typename PP::R nl,
                                                  typename PP::R nr, typename PP::R tl, typename PP::R tr,
                                                  typename PP::R g, typename PP::R cl, typename PP::R hfilm,
                                                  typename PP::R &T0, typename PP::R &T1, typename PP::R &T2)
 {
     typedef typename PP::R R;
     const R half = R(0.5);
-    const R cr = PP::sqrtp(g * hr);
+    const R cr = pp.sqrtp(g * hr);
     const R d = nl + 2 * cl - nr - 2 * cr;
-    const R hs = PP::divz(d * d, 16 * g);
+    const R hs = pp.divz(d * d, 16 * g);
     const R us = half * (nl + nr) + cl - cr;
-    const R cs = PP::sqrtz(g * hs);
+    const R cs = pp.sqrtz(g * hs);
     R sl = nl - cl;
     if (us - cs < sl) sl = us - cs;
     R sm = us;
@@ -237,19 +372,20 @@ __device__ __forceinline__ typename PP::R hllc_v(typename PP::R hl, typename PP:
     if (hl <= hfilm) { sl = nr - 2 * cr; sm = sl; sr = nr + cr; }
     if (hr <= hfilm) { sl = nl - cl; sr = nl + 2 * cl; sm = sr; }
     R f0 = PP::qnan(), f1 = f0;
-    if (sl >= 0) {
-        f0 = hl * nl;
-        f1 = hl * nl * nl + half * g * hl * hl;
-    }
-    if (sl <= 0 && sr >= 0) {
-        f0 = PP::divz(sr * (hl * nl) - sl * (hr * nr) + sl * sr * (hr - hl), sr - sl);
-        f1 = PP::div(sr * (hl * nl * nl + half * g * hl * hl) - sl * (hr * nr * nr + half * g * hr * hr)
-                         + sl * sr * (hr * nr - hl * nl),
-                     sr - sl);
-    }
+    /* the reference tests sl >= 0, then sl <= 0 <= sr, then sr <= 0, the last
+     * one met deciding; in this order the star state's divisor is positive */
     if (sr <= 0) {
         f0 = hr * nr;
         f1 = hr * nr * nr + half * g * hr * hr;
+    } else if (sl <= 0 && sr >= 0) {
+        const typename PP::Recip w = pp.recip(sr - sl);
+        f0 = pp.quot(sr * (hl * nl) - sl * (hr * nr) + sl * sr * (hr - hl), w);
+        f1 = pp.quot(sr * (hl * nl * nl + half * g * hl * hl) - sl * (hr * nr * nr + half * g * hr * hr)
+                         + sl * sr * (hr * nr - hl * nl),
+                     w);
+    } else if (sl >= 0) {
+        f0 = hl * nl;
+        f1 = hl * nl * nl + half * g * hl * hl;
     }
     T0 = f0;
     T1 = f1;
@@ -271,18 +407,55 @@ __device__ __forceinline__ typename PP::R mirror_v(typename PP::R vel, typename 
     return h > hfilm ? -vel : typename PP::R(0);
 }
 
+/* The states of a face beside a solid cell (var 1: the left or lower side
+ * is solid, 2: the right or upper one): the flow side's state on both sides,
+ * its normal velocity mirrored, with the GZ of the face's left cell */
+template <class PP>
+__device__ __forceinline__ void mirror_face(int var, typename PP::R hfilm, typename PP::R &hl, typename PP::R &hr,
+                                            typename PP::R &nl, typename PP::R &nr, typename PP::R &tl,
+                                            typename PP::R &tr, typename PP::R g, typename PP::R &cl)
+{
+    if (var == 1) {
+        hl = hr;
+        nl = mirror_v<PP>(nr, hr, hfilm);
+        tl = tr;
+        cl = PP::sqrtp(g * hr);
+    } else if (var == 2) {
+        hr = hl;
+        nr = mirror_v<PP>(nl, hl, hfilm);
+        tr = tl;
+    }
+}
+
+/* the three fluxes of a face with plain operators, for the rare face that
+ * FastF64 does not take */
+template <class R>
+struct Flux {
+    R a, b, c;
+};
+template <class PP>
+__device__ __noinline__ Flux<typename PP::R> hllc_plain(typename PP::R hl, typename PP::R hr, typename PP::R nl,
+                                                        typename PP::R nr, typename PP::R tl, typename PP::R tr,
+                                                        typename PP::R g, typename PP::R cl, typename PP::R hfilm)
+{
+    PP pp;
+    Flux<typename PP::R> w;
+    hllc_v<PP>(pp, hl, hr, nl, nr, tl, tr, g, cl, hfilm, w.a, w.b, w.c);
+    return w;
+}
+
 /* wave speed only (the same sl, sr, sm as hllc_v) */
 template <class PP>
-__device__ __forceinline__ typename PP::R hll_speed(typename PP::R hl, typename PP::R hr, typename PP::R nl,
+__device__ __forceinline__ typename PP::R hll_speed(PP &pp, typename PP::R hl, typename PP::R hr, typename PP::R nl,
                                                     typename PP::R nr, typename PP::R g, typename PP::R cl,
                                                     typename PP::R hfilm)
 {
     typedef typename PP::R R;
-    const R cr = PP::sqrtp(g * hr);
+    const R cr = pp.sqrtp(g * hr);
     const R d = nl + 2 * cl - nr - 2 * cr;
-    const R hs = PP::divz(d * d, 16 * g);
+    const R hs = pp.divz(d * d, 16 * g);
     const R us = R(0.5) * (nl + nr) + cl - cr;
-    const R cs = PP::sqrtz(g * hs);
+    const R cs = pp.sqrtz(g * hs);
     R sl = nl - cl;
     if (us - cs < sl) sl = us - cs;
     R sm = us;
@@ -568,6 +741,7 @@ __device__ __forceinline__ void stage_derive(const DevParams &P, const SetV<RS> 
                                              typename PP::R insed)
 {
     typedef typename PP::R R;
+    typedef typename PP::Fast F;
     const int S = NS ? NS : P.S;
     const RealC<R> &K = kc<R>(P);
     const RS *halo = reinterpret_cast<const RS *>(smb + L.halo);
@@ -597,16 +771,35 @@ __device__ __forceinline__ void stage_derive(const DevParams &P, const SetV<RS> 
             if ((gi == 0 && P.bndry[0] == 1) || (gi == P.nx + 1 && P.bndry[2] == 1)) hu = -hu;
             if ((gj == 0 && P.bndry[1] == 1) || (gj == P.ny + 1 && P.bndry[3] == 1)) hv = -hv;
         }
+        F pp = make_fast<F>(P);
+        const bool flow = h > K.hfilm;
+        const typename F::Recip rh = F::recip(h);
         R u = 0, v = 0;
-        if (h > K.hfilm) { u = PP::div(hu, h); v = PP::div(hv, h); }
+        if (flow) { u = pp.quot(hu, rh); v = pp.quot(hv, rh); }
         if (gx || gy) {
             /* ghost cells are never read through the staged planes: keep h there */
             reinterpret_cast<RS *>(smb + L.halo)[HP_H * L.hps + hi * Cols<RS>::rj + hj + Cols<RS>::pad - 1] = (RS)h;
         }
-        su[idx] = u;
-        sv[idx] = v;
-        if (hi <= T_I && hj <= T_J) {
-            R g;
+        auto sed_k = [&](int k, R q) {            /* q = U_k / h of a flowing cell */
+            R s = 0;
+            if (inflow) s = insed;
+            else if (flow) {
+                s = q;
+                if (s < R(-1e-5)) s = 0;
+            }
+            ssed[k * N_H + idx] = s;
+        };
+        const RS *U = halo + HP_U * L.hps + so;
+        if constexpr (NS > 0) {
+#pragma unroll
+            for (int k = 0; k < NS; k++) sed_k(k, flow ? pp.quot((R)U[k * L.hps], rh) : R(0));
+        } else {
+#pragma unroll 4
+            for (int k = 0; k < S; k++) sed_k(k, flow ? pp.quot((R)U[k * L.hps], rh) : R(0));
+        }
+        R g = 0, c = 0, slope2 = 1;
+        const bool left = hi <= T_I && hj <= T_J;      /* the left or lower cell of a face of the tile */
+        if (left) {
             if (P.has_solid) {
                 /* the state's GZ plane: the previous step's GZ of a flow cell,
                  * the set-up GZ a solid cell keeps (SWEHR.c:1233) */
@@ -615,26 +808,29 @@ __device__ __forceinline__ void stage_derive(const DevParams &P, const SetV<RS> 
                 /* GZ of the previous step at the source cell, SWEHR.c:1279 via z_prev */
                 const int zr = si - (tc.i0 - 2);
                 const R sx = (R)sslope_x(P, zps, zr, zcol, si), sy = (R)sslope_y(P, zps, zr, zcol, sj);
-                g = PP::div(K.g, PP::sqrtp(sx * sx + sy * sy + 1));
+                slope2 = sx * sx + sy * sy + 1;
+                g = pp.div(K.g, pp.root1(slope2));
             }
-            sg[idx] = g;
-            sc[idx] = PP::sqrtp(g * h);
+            c = pp.sqrtp(g * h);
         }
-        auto sed_k = [&](int k) {
-            R s = 0;
-            if (inflow) s = insed;
-            else if (h > K.hfilm) {
-                s = PP::div((R)halo[(HP_U + k) * L.hps + so], h);
-                if (s < R(-1e-5)) s = 0;
-            }
-            ssed[k * N_H + idx] = s;
-        };
-        if (PP::kRollClasses) {          /* one division sequence in the code, not four */
+        if constexpr (F::kGuarded) {
+            if (!pp.ok) {                         /* an operand the branch-free sequences do not take */
+                typedef typename F::Plain Q;
+                u = v = 0;
+                if (flow) { u = Q::div(hu, h); v = Q::div(hv, h); }
 #pragma unroll 1
-            for (int k = 0; k < S; k++) sed_k(k);
-        } else {
-#pragma unroll
-            for (int k = 0; k < S; k++) sed_k(k);
+                for (int k = 0; k < S; k++) sed_k(k, flow ? Q::div((R)U[k * L.hps], h) : R(0));
+                if (left) {
+                    if (!P.has_solid) g = Q::div(K.g, Q::sqrtp(slope2));
+                    c = Q::sqrtp(g * h);
+                }
+            }
+        }
+        su[idx] = u;
+        sv[idx] = v;
+        if (left) {
+            sg[idx] = g;
+            sc[idx] = c;
         }
     }
 }
@@ -675,7 +871,7 @@ __device__ __forceinline__ typename PP::R lagged_gz(const DevParams &P, const do
  * past the row at j = ny, see solid_at), with the GZ of the face's left
  * (lower) cell as every face does. */
 template <class PP, class RS>
-__device__ __forceinline__ typename PP::R wave_cell_g(const DevParams &P, const SetV<RS> &src, int i, int j,
+__device__ __forceinline__ typename PP::R wave_cell_g(PP &pp, const DevParams &P, const SetV<RS> &src, int i, int j,
                                                       typename PP::R inh, typename PP::R inhv, typename PP::R g,
                                                       const uint8_t *__restrict__ solid = nullptr)
 {
@@ -685,24 +881,25 @@ __device__ __forceinline__ typename PP::R wave_cell_g(const DevParams &P, const 
     const R h = (R)src.h[q], hu = (R)src.hu[q], hv = (R)src.hv[q];
     R u = 0, v = 0;
     if (h > K.hfilm) {
-        u = PP::div(hu, h);
-        v = PP::div(hv, h);
+        const typename PP::Recip rh = PP::recip(h);
+        u = pp.quot(hu, rh);
+        v = pp.quot(hv, rh);
     }
-    const R c = PP::sqrtp(g * h);
+    const R c = pp.sqrtp(g * h);
     const bool here_solid = solid && solid_at(P, solid, i, j);
     R smax = 0, s;
     /* x face i+1/2 */
     if (i < P.nx) {
         const int64_t qr = q + P.pitch;
         const R hr = (R)src.h[qr];
-        const R ur = hr > K.hfilm ? PP::div((R)src.hu[qr], hr) : R(0);
+        const R ur = hr > K.hfilm ? pp.div((R)src.hu[qr], hr) : R(0);
         const bool right_solid = solid && solid_at(P, solid, i + 1, j);
         if (here_solid && !right_solid)
-            s = hll_speed<PP>(hr, hr, mirror_v<PP>(ur, hr, K.hfilm), ur, g, PP::sqrtp(g * hr), K.hfilm);
-        else if (!here_solid && right_solid) s = hll_speed<PP>(h, h, u, mirror_v<PP>(u, h, K.hfilm), g, c, K.hfilm);
-        else s = hll_speed<PP>(h, hr, u, ur, g, c, K.hfilm);
+            s = hll_speed<PP>(pp, hr, hr, mirror_v<PP>(ur, hr, K.hfilm), ur, g, pp.sqrtp(g * hr), K.hfilm);
+        else if (!here_solid && right_solid) s = hll_speed<PP>(pp, h, h, u, mirror_v<PP>(u, h, K.hfilm), g, c, K.hfilm);
+        else s = hll_speed<PP>(pp, h, hr, u, ur, g, c, K.hfilm);
     } else {
-        s = hll_speed<PP>(h, h, u, P.bndry[2] == 1 ? -u : u, g, c, K.hfilm);
+        s = hll_speed<PP>(pp, h, h, u, P.bndry[2] == 1 ? -u : u, g, c, K.hfilm);
     }
     smax = (s > smax) ? s : smax;
     /* y face j+1/2: the right state is cell (i, j+1), or at j = ny the ghost
@@ -712,31 +909,41 @@ __device__ __forceinline__ typename PP::R wave_cell_g(const DevParams &P, const 
         if (j < P.ny) {
             const int64_t qr = q + 1;
             hr = (R)src.h[qr];
-            vr = hr > K.hfilm ? PP::div((R)src.hv[qr], hr) : R(0);
+            vr = hr > K.hfilm ? pp.div((R)src.hv[qr], hr) : R(0);
         } else if (P.inflow) {
             hr = (R)(RS)inh;                     /* the ghost's depth as the tile pass staged it */
-            vr = inh > K.hfilm ? PP::div(inhv, inh) : R(0);
+            vr = inh > K.hfilm ? pp.div(inhv, inh) : R(0);
         } else {
             hr = h;
             vr = P.bndry[3] == 1 ? -v : v;
         }
         const bool right_solid = solid && solid_at(P, solid, i, j + 1);
         if (here_solid && !right_solid)
-            s = hll_speed<PP>(hr, hr, mirror_v<PP>(vr, hr, K.hfilm), vr, g, PP::sqrtp(g * hr), K.hfilm);
-        else if (!here_solid && right_solid) s = hll_speed<PP>(h, h, v, mirror_v<PP>(v, h, K.hfilm), g, c, K.hfilm);
-        else s = hll_speed<PP>(h, hr, v, vr, g, c, K.hfilm);
+            s = hll_speed<PP>(pp, hr, hr, mirror_v<PP>(vr, hr, K.hfilm), vr, g, pp.sqrtp(g * hr), K.hfilm);
+        else if (!here_solid && right_solid) s = hll_speed<PP>(pp, h, h, v, mirror_v<PP>(v, h, K.hfilm), g, c, K.hfilm);
+        else s = hll_speed<PP>(pp, h, hr, v, vr, g, c, K.hfilm);
     }
     smax = (s > smax) ? s : smax;
     /* the domain's faces 1/2: ghost on the left, this cell on the right */
     if (i == 1) {
-        s = hll_speed<PP>(h, h, P.bndry[0] == 1 ? -u : u, u, g, c, K.hfilm);
+        s = hll_speed<PP>(pp, h, h, P.bndry[0] == 1 ? -u : u, u, g, c, K.hfilm);
         smax = (s > smax) ? s : smax;
     }
     if (j == 1) {
-        s = hll_speed<PP>(h, h, P.bndry[1] == 1 ? -v : v, v, g, c, K.hfilm);
+        s = hll_speed<PP>(pp, h, h, P.bndry[1] == 1 ? -v : v, v, g, c, K.hfilm);
         smax = (s > smax) ? s : smax;
     }
     return smax;
+}
+
+/* the same with plain operators, for the rare cell that FastF64 does not take */
+template <class PP, class RS>
+__device__ __noinline__ typename PP::R wave_cell_plain(const DevParams &P, const SetV<RS> src, int i, int j,
+                                                       typename PP::R inh, typename PP::R inhv,
+                                                       const uint8_t *__restrict__ solid)
+{
+    PP pp;
+    return wave_cell_g<PP, RS>(pp, P, src, i, j, inh, inhv, (typename PP::R)src.gz[cidx(P, i, j)], solid);
 }
 
 template <class PP, class RS>
@@ -744,8 +951,14 @@ __device__ __forceinline__ typename PP::R wave_cell(const DevParams &P, const Se
                                                     typename PP::R inh, typename PP::R inhv,
                                                     const uint8_t *__restrict__ solid)
 {
+    typedef typename PP::Fast F;
+    F pp = make_fast<F>(P);
     /* GZ of the previous step, written by its update */
-    return wave_cell_g<PP, RS>(P, src, i, j, inh, inhv, (typename PP::R)src.gz[cidx(P, i, j)], solid);
+    const typename PP::R s =
+        wave_cell_g<F, RS>(pp, P, src, i, j, inh, inhv, (typename PP::R)src.gz[cidx(P, i, j)], solid);
+    if constexpr (F::kGuarded)
+        if (!pp.ok) return wave_cell_plain<typename F::Plain, RS>(P, src, i, j, inh, inhv, solid);
+    return s;
 }
 
 /* V = 16 / sizeof(RS) consecutive elements of a plane with one 16-byte
@@ -769,7 +982,7 @@ __device__ __forceinline__ void load_vec(const RS *__restrict__ p, R *out)
  * V cells per load.  A cell's normal velocity towards its right neighbour in
  * the vector is that neighbour's own velocity, formed once. */
 template <class PP, class RS>
-__device__ __forceinline__ typename PP::R wave_vec(const DevParams &P, const SetV<RS> &src, int i, int j0,
+__device__ __forceinline__ typename PP::R wave_vec(PP &pp, const DevParams &P, const SetV<RS> &src, int i, int j0,
                                                    typename PP::R inh, typename PP::R inhv)
 {
     typedef typename PP::R R;
@@ -798,8 +1011,9 @@ __device__ __forceinline__ typename PP::R wave_vec(const DevParams &P, const Set
         u[k] = 0;
         v[k] = 0;
         if (h[k] > K.hfilm) {
-            u[k] = PP::div(hu[k], h[k]);
-            v[k] = PP::div(hv[k], h[k]);
+            const typename PP::Recip rh = PP::recip(h[k]);
+            u[k] = pp.quot(hu[k], rh);
+            v[k] = pp.quot(hv[k], rh);
         }
     }
     R smax = 0, s;
@@ -807,13 +1021,13 @@ __device__ __forceinline__ typename PP::R wave_vec(const DevParams &P, const Set
     for (int k = 0; k < V; k++) {
         const int j = j0 + k;
         if (j > P.ny) break;
-        const R c = PP::sqrtp(g[k] * h[k]);
+        const R c = pp.sqrtp(g[k] * h[k]);
         /* x face i+1/2 */
         if (below) {
-            const R ur = hd[k] > K.hfilm ? PP::div(hud[k], hd[k]) : R(0);
-            s = hll_speed<PP>(h[k], hd[k], u[k], ur, g[k], c, K.hfilm);
+            const R ur = hd[k] > K.hfilm ? pp.div(hud[k], hd[k]) : R(0);
+            s = hll_speed<PP>(pp, h[k], hd[k], u[k], ur, g[k], c, K.hfilm);
         } else {
-            s = hll_speed<PP>(h[k], h[k], u[k], P.bndry[2] == 1 ? -u[k] : u[k], g[k], c, K.hfilm);
+            s = hll_speed<PP>(pp, h[k], h[k], u[k], P.bndry[2] == 1 ? -u[k] : u[k], g[k], c, K.hfilm);
         }
         smax = (s > smax) ? s : smax;
         /* y face j+1/2 */
@@ -824,24 +1038,24 @@ __device__ __forceinline__ typename PP::R wave_vec(const DevParams &P, const Set
                 vr = v[k + 1];
             } else {
                 hr = hn;
-                vr = hn > K.hfilm ? PP::div(hvn, hn) : R(0);
+                vr = hn > K.hfilm ? pp.div(hvn, hn) : R(0);
             }
         } else if (P.inflow) {
             hr = (R)(RS)inh;
-            vr = inh > K.hfilm ? PP::div(inhv, inh) : R(0);
+            vr = inh > K.hfilm ? pp.div(inhv, inh) : R(0);
         } else {
             hr = h[k];
             vr = P.bndry[3] == 1 ? -v[k] : v[k];
         }
-        s = hll_speed<PP>(h[k], hr, v[k], vr, g[k], c, K.hfilm);
+        s = hll_speed<PP>(pp, h[k], hr, v[k], vr, g[k], c, K.hfilm);
         smax = (s > smax) ? s : smax;
         /* the domain's faces 1/2 */
         if (i == 1) {
-            s = hll_speed<PP>(h[k], h[k], P.bndry[0] == 1 ? -u[k] : u[k], u[k], g[k], c, K.hfilm);
+            s = hll_speed<PP>(pp, h[k], h[k], P.bndry[0] == 1 ? -u[k] : u[k], u[k], g[k], c, K.hfilm);
             smax = (s > smax) ? s : smax;
         }
         if (j == 1) {
-            s = hll_speed<PP>(h[k], h[k], P.bndry[1] == 1 ? -v[k] : v[k], v[k], g[k], c, K.hfilm);
+            s = hll_speed<PP>(pp, h[k], h[k], P.bndry[1] == 1 ? -v[k] : v[k], v[k], g[k], c, K.hfilm);
             smax = (s > smax) ? s : smax;
         }
     }
@@ -880,9 +1094,10 @@ __device__ __forceinline__ void wave_finalize(const DevParams &P, Ctl *ctl)
 }
 
 template <class PP, class RS>
-__global__ void __launch_bounds__(TILE_THREADS, PP::kWaveMinBlocks) k_wave_cells(const DevParams P, const BufsT<RS> B, Ctl *ctl)
+__global__ void __launch_bounds__(TILE_THREADS, PP::kWaveMinBlocks) k_wave_cells(const __grid_constant__ DevParams P, const BufsT<RS> B, Ctl *ctl)
 {
     typedef typename PP::R R;
+    typedef typename PP::Fast F;
     if (!ctl->active) return;
     __shared__ double red8[TILE_THREADS / 32];
     __shared__ bool last;
@@ -905,7 +1120,17 @@ __global__ void __launch_bounds__(TILE_THREADS, PP::kWaveMinBlocks) k_wave_cells
         for (int64_t c = c0; c < total; c += stride) {
             const int r = (int)(c / nv);
             const int i = r + P.own_lo, j0 = (int)(c - (int64_t)r * nv) * V + 1;
-            const R s = wave_vec<PP, RS>(P, src, i, j0, (R)inh, (R)inhv);
+            F pp = make_fast<F>(P);
+            R s = wave_vec<F, RS>(pp, P, src, i, j0, (R)inh, (R)inhv);
+            if constexpr (F::kGuarded)
+                if (!pp.ok) {
+                    s = 0;
+#pragma unroll 1
+                    for (int j = j0; j < j0 + V && j <= P.ny; j++) {
+                        const R sj = wave_cell_plain<typename F::Plain, RS>(P, src, i, j, (R)inh, (R)inhv, nullptr);
+                        s = (sj > s) ? sj : s;
+                    }
+                }
             smax = (s > smax) ? s : smax;
         }
     } else {
@@ -1023,13 +1248,13 @@ __device__ __noinline__ typename PP::R fail_exact(const FailArgs A, const RS *__
 
 /* moving storm in the form's arithmetic (positions in FP64) */
 template <class PP>
-__device__ __forceinline__ typename PP::R storm_r(const DevParams &P, double t, int i, int j)
+__device__ __forceinline__ typename PP::R storm_r(PP &pp, const DevParams &P, double t, int i, int j)
 {
     typedef typename PP::R R;
     const double x = ((double)(i + P.row0) - 0.5) * P.dx - (P.storm_x0 + P.storm_vx * t);
     const double y = ((double)j - 0.5) * P.dx - (P.storm_y0 + P.storm_vy * t);
     const double r2 = (x * x + y * y) / P.storm_r2;
-    return (R)P.storm_peak * PP::exp(R(-0.5 * r2));
+    return (R)P.storm_peak * pp.exp(R(-0.5 * r2));
 }
 
 /* A solid cell in the update (SWEHR.c:1421 false branch, 1566-1574): no
@@ -1066,8 +1291,11 @@ __device__ __forceinline__ void solid_cell(const DevParams &P, const SetV<RS> &s
     zn[q] = zc[q];
 }
 
-template <class PP, class RS, int MAXS, bool BUDGET, int NS = 0>
-__device__ __forceinline__ void tile_cell(const DevParams &P, const SetV<RS> &src, const SetV<RS> &dst,
+/* One cell of the tile with the arithmetic PP.  FRESH: U_k and M_k are read
+ * from the source set instead of their staged slots (a cell computed again,
+ * whose slots already hold new values). */
+template <class PP, class RS, int MAXS, bool BUDGET, int NS, bool FRESH>
+__device__ __forceinline__ void tile_cell_pp(PP &pp, const DevParams &P, const SetV<RS> &src, const SetV<RS> &dst,
                                           const double *__restrict__ zp, const double *__restrict__ zc,
                                           double *__restrict__ zn, const unsigned char *smb, const StagedLayout &L,
                                           TileCoord tc, double t, double dt, double Rr, Acc2<MAXS, BUDGET> &acc,
@@ -1077,14 +1305,10 @@ __device__ __forceinline__ void tile_cell(const DevParams &P, const SetV<RS> &sr
     const RealC<R> &K = kc<R>(P);
     const int ti = threadIdx.x / T_J, tj = threadIdx.x % T_J;
     const int i = tc.i0 + ti, j = tc.j0 + tj;
-    if (i > P.own_hi || j > P.ny) return;
     const int64_t pl = P.plane;
     const int64_t q = cidx(P, i, j);
-    if (P.has_solid && solid[q]) {
-        solid_cell<PP, RS, MAXS, BUDGET>(P, src, dst, zc, zn, q, acc);
-        return;
-    }
     const int S = NS ? NS : P.S;
+    const bool stage_m = !FRESH && L.stage_m;
     const R hfilm = K.hfilm, rhos = K.rhos, rhow = K.rhow, one = 1, half = R(0.5);
     const int hs = (ti + 1) * H_J + (tj + 1);                      /* this cell in halo coords */
     constexpr int RJ = Cols<RS>::rj;
@@ -1100,7 +1324,7 @@ __device__ __forceinline__ void tile_cell(const DevParams &P, const SetV<RS> &sr
     const R totm0 = (R)cellr[CR_TOTM * T_I * T_J + cs];
     R rho0c = rhow * (1 - totsed0) + rhos * totsed0;
     if (rho0c > K.rhos08) rho0c = K.rhos08;
-    const R Rc = P.storm ? storm_r<PP>(P, t, i, j) : (R)Rr;
+    const R Rc = P.storm ? storm_r<PP>(pp, P, t, i, j) : (R)Rr;
     const R dtr = (R)dt;
 
     /* faces of this cell (computed in stage B) */
@@ -1123,12 +1347,13 @@ __device__ __forceinline__ void tile_cell(const DevParams &P, const SetV<RS> &sr
     const double *zps = reinterpret_cast<const double *>(smb + L.zp), *zcs = reinterpret_cast<const double *>(smb + L.zc);
     const R sx = (R)sslope_x(P, zcs, ti + 1, tj + 2, i), sy = (R)sslope_y(P, zcs, ti + 1, tj + 2, j);
     const R syl = (R)sslope_y(P, zps, ti + 2, tj + 2, j);
-    const R gx = PP::div(g * sx, PP::sqrtp(sx * sx + syl * syl + 1));
+    const R gx = pp.div(g * sx, pp.root1(sx * sx + syl * syl + 1));
     const R SXf = -gx * h0v;
-    const R gy = PP::div(g * sy, PP::sqrtp(sx * sx + sy * sy + 1));
+    const typename PP::Recip rroot = PP::recip(pp.root1(sx * sx + sy * sy + 1));
+    const R gy = pp.quot(g * sy, rroot);
     const R SYf = -gy * h0v;
-    const R gz = PP::div(g, PP::sqrtp(sx * sx + sy * sy + 1));
-    const R slope = PP::sqrtp(sx * sx + sy * sy);
+    const R gz = pp.quot(g, rroot);
+    const R slope = pp.sqrtp(sx * sx + sy * sy);
     /* variable-density forcing (SWEHR.c:1283-1290).  Where the TOTSED
      * difference is an exact zero the term is a zero times a finite
      * quotient, and 0 - (+-0) = +0: the FP64 form keeps gamma = +0 without
@@ -1139,10 +1364,10 @@ __device__ __forceinline__ void tile_cell(const DevParams &P, const SetV<RS> &sr
                2 * rho0c >= R(0x1p-100);
     };
     if (i > 1 && i < P.nx && !zero_gradient(so + RJ, so - RJ))
-        gammax -= PP::div((rhos - rho0c) * gz * h0v * h0v, 2 * rho0c) * half * K.oneoverdx
+        gammax -= pp.div((rhos - rho0c) * gz * h0v * h0v, 2 * rho0c) * half * K.oneoverdx
                   * ((R)sTS[so + RJ] - (R)sTS[so - RJ]);
     if (j > 1 && j < P.ny && !zero_gradient(so + 1, so - 1))
-        gammay -= PP::div((rhos - rho0c) * gz * h0v * h0v, 2 * rho0c) * half * K.oneoverdx
+        gammay -= pp.div((rhos - rho0c) * gz * h0v * h0v, 2 * rho0c) * half * K.oneoverdx
                   * ((R)sTS[so + 1] - (R)sTS[so - 1]);
     /* slope stability: provable "no failure" first, exact test otherwise */
     R fail = 0;
@@ -1164,10 +1389,10 @@ __device__ __forceinline__ void tile_cell(const DevParams &P, const SetV<RS> &sr
             fa.oneoverdx = P.oneoverdx; fa.half_odx = P.half_odx; fa.rho0 = P.rho0; fa.rhow = P.rhow;
             fa.cohesion = P.cohesion; fa.fa = P.fa;
             fa.solid = P.has_solid ? solid : nullptr; fa.z0 = z0;
-            fail = fail_exact<PP, RS>(fa, src.dep, zp, zc, i, j, sx, sy, gz, dep0, rho0c, h0v);
+            fail = fail_exact<typename PP::Plain, RS>(fa, src.dep, zp, zc, i, j, sx, sy, gz, dep0, rho0c, h0v);
         }
     }
-    R dfmask = fmin(one, PP::divk(totsed0 - R(0.2), R(0.2), (R)P.inv_p2, P.divk_ok));
+    R dfmask = fmin(one, pp.divk(totsed0 - R(0.2), R(0.2), (R)P.inv_p2, P.divk_ok));
     if (h0v < K.h0x9 || totsed0 < R(0.2)) dfmask = 0;
     R betax = K.neg1ml * gz * h0v * K.fa;
     R betay = K.neg1ml * gz * h0v * K.fa;
@@ -1175,29 +1400,30 @@ __device__ __forceinline__ void tile_cell(const DevParams &P, const SetV<RS> &sr
     if (hv0 < 0) betay = -1 * betay;
 
     /* Hairsine-Rose, class-independent parts (SWEHR.c:1330-1382) */
-    const R hvert = PP::div(h0v, PP::cos_atan(fabs(slope)));
+    const R hvert = pp.div(h0v, pp.cos_atan(fabs(slope)));
     R mtstar = K.mtstar0;
     const bool deepv = hvert > K.h0;
     R depthfac = 1;
     if (deepv) {
-        depthfac = PP::pow(PP::div(K.h0, hvert), K.b);
+        depthfac = pp.pow(pp.div(K.h0, hvert), K.b);
         mtstar = K.mtstar0 * depthfac;
     }
-    const R Hs = fmin(one, PP::divz(totm0, mtstar));
+    const R Hs = fmin(one, pp.quotn(totm0, PP::recip(mtstar)));
     const bool swash = (h0v > K.hfx10 && totsed0 < R(0.6));
     R E3b = 0, E4b = 0, e4den = 1;
     if (swash) {
-        const R manning = (h0v <= K.hc) ? K.roughness * PP::pow(PP::div(h0v, K.hc), K.dde) : K.roughness;
-        const R qq = PP::sqrtp(hu0 * hu0 + hv0 * hv0);
-        const R SF = PP::div(manning * manning * qq * qq, PP::pow(h0v, R(3.333)));
+        const R manning = (h0v <= K.hc) ? K.roughness * pp.pow(pp.div(h0v, K.hc), K.dde) : K.roughness;
+        const R qq = pp.sqrtp(hu0 * hu0 + hv0 * hv0);
+        const R SF = pp.div(manning * manning * qq * qq, pp.pow(h0v, R(3.333)));
         /* streampowererosion (SWEHR.c:412-426): omega is the same for every
          * class; only the h > d_k condition differs */
         const R omega = rho0c * gz * SF * qq;
         if (omega > K.uc && totsed0 < R(0.6)) E3b = K.af * (omega - K.uc);
         if (omega > K.uc2 && totsed0 < R(0.6)) E4b = K.afr * (omega - K.uc2);
-        e4den = PP::divk(rhos - rho0c, rhos, (R)P.inv_rhos, P.divk_ok) * gz * h0v;
+        e4den = pp.divk(rhos - rho0c, rhos, (R)P.inv_rhos, P.divk_ok) * gz * h0v;
     }
-    const R vfconc = PP::pow(1 - fmin(totsed0, R(0.99)), R(4.0));
+    const typename PP::Recip rtotm = PP::recip(totm0), re4 = PP::recip(e4den);
+    const R vfconc = pp.pow(1 - fmin(totsed0, R(0.99)), R(4.0));
     const bool debris = (h0v > K.h0x9 && totsed0 > K.cthreshold);
 
     /* conservative update, SWEHR.c:1424-1446 */
@@ -1208,9 +1434,16 @@ __device__ __forceinline__ void tile_cell(const DevParams &P, const SetV<RS> &sr
     /* Green-Ampt in FP64 (SWEHR.c:1449-1452) */
     const double ks = P.has_ks ? (double)cellr[CR_KS * T_I * T_J + cs] : P.ks;
     const double vinf0 = celld[CD_VINF * T_I * T_J + cs];
-    const double zf = PolicyF64::divk(vinf0, P.thetas - P.theta0, P.inv_dtheta, P.divk_ok);
     const double hd = (double)h;
-    const double infl = fmin(hd - P.hfilm, dt * ks * (zf + P.hf + hd) / zf);
+    double zf, need;
+    if constexpr (PP::kGuarded) {
+        zf = pp.divk(vinf0, P.thetas - P.theta0, P.inv_dtheta, 1);
+        need = pp.div(dt * ks * (zf + P.hf + hd), zf);
+    } else {
+        zf = PolicyF64::divk(vinf0, P.thetas - P.theta0, P.inv_dtheta, P.divk_ok);
+        need = dt * ks * (zf + P.hf + hd) / zf;
+    }
+    const double infl = fmin(hd - P.hfilm, need);
     const double vinf = vinf0 + infl;
     h = (R)(hd - infl);
 
@@ -1220,7 +1453,7 @@ __device__ __forceinline__ void tile_cell(const DevParams &P, const SetV<RS> &sr
      * of the staged U_k plane (no other thread reads that slot once the faces
      * are solved), so no per-class array stays live in registers; the mixed
      * form's unrolled loops keep them in registers (faster there). */
-    constexpr bool kSlot = PP::kRollClasses;
+    constexpr bool kSlot = PP::kRollClasses || (PP::kGuarded && NS == 0);
     static_assert(sizeof(R) == sizeof(RS), "the staged U_k slot holds a U_k value");
     const R *SED = reinterpret_cast<const R *>(smb + L.sed);
     RS *Uslot = reinterpret_cast<RS *>(const_cast<unsigned char *>(smb) + L.halo) + HP_U * L.hps + so;
@@ -1243,13 +1476,13 @@ __device__ __forceinline__ void tile_cell(const DevParams &P, const SetV<RS> &sr
         if (k >= S) break;
         const int64_t qm = k * pl + q;
         const R *sk = SED + k * N_H;
-        const RS u_in = Uslot[k * hps];
+        const RS u_in = FRESH ? src.U[qm] : Uslot[k * hps];
         R uflux;
         if constexpr (kSlot)
             uflux = (R)u_in - dtdx * (fxr0 * sk[uxr] - fxl0 * sk[uxl]) - dtdx * (fyr0 * sk[uyr] - fyl0 * sk[uyl]);
         else
             uflux = Ureg[kSlot ? 0 : k];
-        const double Mk0 = L.stage_m ? celld[(CD_M + k) * T_I * T_J + cs] : __ldg(src.M + qm);
+        const double Mk0 = stage_m ? celld[(CD_M + k) * T_I * T_J + cs] : __ldg(src.M + qm);
         const R Mk0r = (R)Mk0;
         /* Rain-splash detachment of the original soil is the only source the
          * shallow branch uses; the other sources and the settling velocity
@@ -1271,23 +1504,23 @@ __device__ __forceinline__ void tile_cell(const DevParams &P, const SetV<RS> &sr
         } else {
             R E2 = 0, E3 = 0, E4 = 0, VF = 0;
             if (swash && !debris) {
-                if (totm0 > R(1e-8) && Mk0r > R(1e-8)) E2 = PP::div(Hs * Mk0r, totm0) * K.ad * Rc;
+                if (totm0 > R(1e-8) && Mk0r > R(1e-8)) E2 = pp.quot(Hs * Mk0r, rtotm) * K.ad * Rc;
                 if (deepv) E2 = E2 * depthfac;
-                E3 = PP::e3_term((1 - Hs) * K.pf[k] * K.F, K.J, (R)P.inv_J, P.divk_ok, h0v > K.ds[k] ? E3b : R(0));
+                E3 = pp.e3_term((1 - Hs) * K.pf[k] * K.F, K.J, (R)P.inv_J, P.divk_ok, h0v > K.ds[k] ? E3b : R(0));
                 if (totm0 > R(1e-6) && Mk0r > 0)
-                    E4 = PP::e4_term(K.one_m_bb * Hs * Mk0r, totm0, K.F, e4den, h0v > K.ds[k] ? E4b : R(0));
+                    E4 = pp.e4_term(K.one_m_bb * Hs * Mk0r, rtotm, K.F, re4, h0v > K.ds[k] ? E4b : R(0));
             }
             if (!debris) {
-                VF = PP::settle(K.a13[k], K.a13sq[k], K.c109s * gz * K.ds[k]);
+                VF = pp.settle(K.a13[k], K.a13sq[k], K.c109s * gz * K.ds[k]);
                 VF = VF * vfconc;
                 if (K.ds[k] > R(0.0001) && h0v < K.h0x9)
-                    VF = R(2e-3) + PP::divk(fmax(h0v - K.h0x3, R(0)) * (VF - R(2e-3)), K.h0x6, (R)P.inv_h0x6, P.divk_ok);
+                    VF = R(2e-3) + pp.divk(fmax(h0v - K.h0x3, R(0)) * (VF - R(2e-3)), K.h0x6, (R)P.inv_h0x6, P.divk_ok);
                 if (K.ds[k] > R(0.002) && h0v < K.h0x9)
-                    VF = R(2e-3) + PP::divk(fmax(h0v - K.h0x3, R(0)) * (VF - R(2e-3)), K.h0x6, (R)P.inv_h0x6, P.divk_ok);
+                    VF = R(2e-3) + pp.divk(fmax(h0v - K.h0x3, R(0)) * (VF - R(2e-3)), K.h0x6, (R)P.inv_h0x6, P.divk_ok);
             }
             chtemp = u;
             const R redetach = fmin(Mk0r, dtr * (E2 + E4));
-            const R dec = PP::exp(PP::div(-VF, h) * (half * dtr));
+            const R dec = pp.exp(pp.div(-VF, h) * (half * dtr));
             u = dec * u;
             u = u + dtr * (E1 + E3) + redetach;
             u = dec * u;
@@ -1302,16 +1535,16 @@ __device__ __forceinline__ void tile_cell(const DevParams &P, const SetV<RS> &sr
                 dep = 0;
             }
         }
-        const R dh = PP::divk(u - chtemp, K.porod, (R)P.invporo, P.divk_ok);
+        const R dh = pp.divk(u - chtemp, K.porod, (R)P.invporo, P.divk_ok);
         h = h + dh;
         bulk += dh;
         totm += Mk;
-        dep += PP::dep_of(Mk, P);
+        dep += pp.dep_of(Mk, P);
         if constexpr (kSlot)
             Uslot[k * hps] = (RS)u;
         else
             Ureg[kSlot ? 0 : k] = u;
-        if (L.stage_m)         /* the cell's own staged slot: read back below, no global round trip */
+        if (stage_m)         /* the cell's own staged slot: read back below, no global round trip */
             const_cast<double *>(celld)[(CD_M + k) * T_I * T_J + cs] = Mk;
         else
             dst.M[qm] = Mk;
@@ -1329,13 +1562,14 @@ __device__ __forceinline__ void tile_cell(const DevParams &P, const SetV<RS> &sr
     /* derived fields and the dry clamp, SWEHR.c:1513-1551 */
     R totsed = 0, clamp = 0;
     if (h > hfilm) {
+        const typename PP::Recip rh = PP::recip(h);
 #pragma unroll
         for (int k = 0; k < MAXS; k++) {
             if (k >= S) break;
             const R uk = kSlot ? (R)Uslot[k * hps] : Ureg[kSlot ? 0 : k];
-            totsed += PP::divk(PP::divz(uk, h), rhos, (R)P.inv_rhos, P.divk_ok);
+            totsed += pp.divk(pp.quotz(uk, rh), rhos, (R)P.inv_rhos, P.divk_ok);
             dst.U[k * pl + q] = (RS)uk;
-            if (L.stage_m) dst.M[k * pl + q] = celld[(CD_M + k) * T_I * T_J + cs];
+            if (stage_m) dst.M[k * pl + q] = celld[(CD_M + k) * T_I * T_J + cs];
         }
     } else {
         clamp = hfilm - h;
@@ -1348,7 +1582,7 @@ __device__ __forceinline__ void tile_cell(const DevParams &P, const SetV<RS> &sr
             const int64_t qm = k * pl + q;
             const R uk = kSlot ? (R)Uslot[k * hps] : Ureg[kSlot ? 0 : k];
             z = z + P.invporo * (double)uk;
-            const double mk = L.stage_m ? celld[(CD_M + k) * T_I * T_J + cs] : dst.M[qm];
+            const double mk = stage_m ? celld[(CD_M + k) * T_I * T_J + cs] : dst.M[qm];
             dst.M[qm] = mk + (double)uk;
             dst.U[qm] = (RS)0;
         }
@@ -1356,15 +1590,16 @@ __device__ __forceinline__ void tile_cell(const DevParams &P, const SetV<RS> &sr
     /* implicit friction, SWEHR.c:1553-1565 */
     R vel1 = 0, vel2 = 0;
     if (h > hfilm) {
-        const R manning = (h <= K.hc) ? K.roughness * PP::pow(PP::div(h, K.hc), K.dde) : K.roughness;
-        const R SFf = PP::div(manning * manning * gz * PP::sqrtp(hu * hu + hv * hv) * 1, PP::pow(h, R(2.333)));
-        hu = PP::div(hu, 1 + dtr * SFf);
-        hv = PP::div(hv, 1 + dtr * SFf);
-        vel1 = PP::div(hu, h);
-        vel2 = PP::div(hv, h);
+        const R manning = (h <= K.hc) ? K.roughness * pp.pow(pp.div(h, K.hc), K.dde) : K.roughness;
+        const R SFf = pp.div(manning * manning * gz * pp.sqrtp(hu * hu + hv * hv) * 1, pp.pow(h, R(2.333)));
+        const typename PP::Recip rf = PP::recip(1 + dtr * SFf), rh = PP::recip(h);
+        hu = pp.quot(hu, rf);
+        hv = pp.quot(hv, rf);
+        vel1 = pp.quot(hu, rh);
+        vel2 = pp.quot(hv, rh);
     }
     R maxvel = (R)cellr[CR_MAXVEL * T_I * T_J + cs], maxdep = (R)cellr[CR_MAXDEP * T_I * T_J + cs];
-    const R vmag = PP::sqrtz(vel1 * vel1 + vel2 * vel2);
+    const R vmag = pp.sqrtz(vel1 * vel1 + vel2 * vel2);
     if (vmag > maxvel) maxvel = vmag;
     if (h > maxdep) maxdep = h;
     dst.h[q] = (RS)h;
@@ -1406,6 +1641,66 @@ __device__ __forceinline__ void tile_cell(const DevParams &P, const SetV<RS> &sr
             if (j == 1) acc.out -= dtdx_d * (double)fyl0;
             if (j == P.ny) acc.out += dtdx_d * (double)fyr0;
         }
+    }
+}
+
+/* what a cell computed again needs, by value (rarely built) */
+template <class RS>
+struct CellArgs {
+    SetV<RS> src, dst;
+    const double *zp, *zc, *z0;
+    double *zn;
+    const unsigned char *smb;
+    const uint8_t *solid;
+    StagedLayout L;
+    TileCoord tc;
+    double t, dt, Rr;
+};
+
+/* A cell whose operands FastF64 does not take, with plain operators: every
+ * output is written again.  Its inputs are the source set and what the block
+ * staged for it; of those only its own U_k and M_k slots have changed. */
+template <class PP, class RS>
+__device__ __noinline__ void tile_cell_again(const DevParams &P, const CellArgs<RS> &a)
+{
+    PP pp;
+    Acc2<16, false> none;
+    tile_cell_pp<PP, RS, 16, false, 0, true>(pp, P, a.src, a.dst, a.zp, a.zc, a.zn, a.smb, a.L, a.tc, a.t, a.dt, a.Rr,
+                                             none, a.solid, a.z0);
+}
+
+/* One thread's cell of the tile.  The budget variant of the plain form adds
+ * to its sums as it goes, so it keeps the plain operators. */
+template <class PP, class RS, int MAXS, bool BUDGET, int NS = 0>
+__device__ __forceinline__ void tile_cell(const DevParams &P, const SetV<RS> &src, const SetV<RS> &dst,
+                                          const double *__restrict__ zp, const double *__restrict__ zc,
+                                          double *__restrict__ zn, const unsigned char *smb, const StagedLayout &L,
+                                          TileCoord tc, double t, double dt, double Rr, Acc2<MAXS, BUDGET> &acc,
+                                          const uint8_t *__restrict__ solid, const double *__restrict__ z0)
+{
+    const int i = tc.i0 + (int)threadIdx.x / T_J, j = tc.j0 + (int)threadIdx.x % T_J;
+    if (i > P.own_hi || j > P.ny) return;
+    if (P.has_solid) {
+        const int64_t q = cidx(P, i, j);
+        if (solid[q]) {
+            solid_cell<PP, RS, MAXS, BUDGET>(P, src, dst, zc, zn, q, acc);
+            return;
+        }
+    }
+    typedef typename PP::Fast F;
+    if constexpr (F::kGuarded && !BUDGET) {
+        F pp = make_fast<F>(P);
+        tile_cell_pp<F, RS, MAXS, BUDGET, NS, false>(pp, P, src, dst, zp, zc, zn, smb, L, tc, t, dt, Rr, acc, solid, z0);
+        if (!pp.ok) {
+            CellArgs<RS> a;
+            a.src = src; a.dst = dst; a.zp = zp; a.zc = zc; a.z0 = z0; a.zn = zn; a.smb = smb; a.solid = solid;
+            a.L = L; a.tc = tc; a.t = t; a.dt = dt; a.Rr = Rr;
+            tile_cell_again<typename F::Plain, RS>(P, a);
+        }
+    } else {
+        typename PP::Plain pp;
+        tile_cell_pp<typename PP::Plain, RS, MAXS, BUDGET, NS, false>(pp, P, src, dst, zp, zc, zn, smb, L, tc, t, dt, Rr,
+                                                                     acc, solid, z0);
     }
 }
 
@@ -1472,6 +1767,7 @@ __device__ __forceinline__ void update_tile(const DevParams &P, const BufsT<RS> 
                                             uint64_t *bar = nullptr, uint32_t *phase = nullptr, Ctl *ctl = nullptr)
 {
     typedef typename PP::R R;
+    typedef typename PP::Fast F;
     const RealC<R> &K = kc<R>(P);
     const SetV<RS> src = B.set[n & 1];
     const SetV<RS> dst = B.set[(n + 1) & 1];
@@ -1503,56 +1799,55 @@ __device__ __forceinline__ void update_tile(const DevParams &P, const BufsT<RS> 
     const RS *sh = staged_h<RS>(smb, L);
     /* stage B: every face of the tile (SWEHR.c:1099-1230) */
     for (int f = threadIdx.x; f < N_FX + N_FY; f += TILE_THREADS) {
-        R T0, T1, T2;
+        R hl, hr, nl, nr, tl, tr, g, cl;
+        R *face;
+        bool yface;
         if (f < N_FX) {
             const int fi = f / T_J, fj = f - fi * T_J;
             const int gi = tc.i0 - 1 + fi, gj = tc.j0 + fj;
             if (gj > P.ny || gi > P.nx) continue;
             const int Lh = fi * H_J + fj + 1, Rh = Lh + H_J;
-            const R hl = (R)sh[fi * Cols<RS>::rj + fj + Cols<RS>::pad], hr = (R)sh[(fi + 1) * Cols<RS>::rj + fj + Cols<RS>::pad];
+            hl = (R)sh[fi * Cols<RS>::rj + fj + Cols<RS>::pad];
+            hr = (R)sh[(fi + 1) * Cols<RS>::rj + fj + Cols<RS>::pad];
+            nl = su[Lh]; nr = su[Rh]; tl = sv[Lh]; tr = sv[Rh]; g = sg[Lh]; cl = sc[Lh];
             int var = 0;                 /* 1: solid left, 2: solid right (SWEHR.c:1137-1146) */
             if (P.has_solid && gi >= 1 && gi < P.nx) {
                 const bool sl = solid_at(P, B.solid, gi, gj), sr = solid_at(P, B.solid, gi + 1, gj);
                 var = (sl && !sr) ? 1 : ((!sl && sr) ? 2 : 0);
             }
-            /* the mirrored normal velocity is (-hu)/h when wet (a zero keeps its
-             * negated sign, as in the reference) and +0 when dry */
-            if (var == 1)
-                hllc_v<PP>(hr, hr, mirror_v<PP>(su[Rh], hr, K.hfilm), su[Rh], sv[Rh], sv[Rh], sg[Lh],
-                           PP::sqrtp(sg[Lh] * hr), K.hfilm, T0, T1, T2);
-            else if (var == 2)
-                hllc_v<PP>(hl, hl, su[Lh], mirror_v<PP>(su[Lh], hl, K.hfilm), sv[Lh], sv[Lh], sg[Lh], sc[Lh], K.hfilm,
-                           T0, T1, T2);
-            else
-                hllc_v<PP>(hl, hr, su[Lh], su[Rh], sv[Lh], sv[Rh], sg[Lh], sc[Lh], K.hfilm, T0, T1, T2);
-            R *F = sfx + 3 * f;
-            F[0] = T0; F[1] = T1; F[2] = T2;
-            upb[f] = (T0 > 0) ? 0 : 1;
+            mirror_face<typename PP::Plain>(var, K.hfilm, hl, hr, nl, nr, tl, tr, g, cl);
+            face = sfx + 3 * f;
+            yface = false;
         } else {
             const int f2 = f - N_FX;
             const int fi = f2 / (T_J + 1), fj = f2 - fi * (T_J + 1);
             const int gi = tc.i0 + fi, gj = tc.j0 - 1 + fj;
             if (gi > P.nx || gj > P.ny) continue;
             const int Lh = (fi + 1) * H_J + fj, Rh = Lh + 1;
-            const R hl = (R)sh[(fi + 1) * Cols<RS>::rj + fj + Cols<RS>::pad - 1],
-                    hr = (R)sh[(fi + 1) * Cols<RS>::rj + fj + Cols<RS>::pad];
+            hl = (R)sh[(fi + 1) * Cols<RS>::rj + fj + Cols<RS>::pad - 1];
+            hr = (R)sh[(fi + 1) * Cols<RS>::rj + fj + Cols<RS>::pad];
+            nl = sv[Lh]; nr = sv[Rh]; tl = su[Lh]; tr = su[Rh]; g = sg[Lh]; cl = sc[Lh];
             int var = 0;                 /* 1: solid below, 2: solid above (SWEHR.c:1205-1214) */
             if (P.has_solid && gj >= 1) {
                 const bool sl = solid_at(P, B.solid, gi, gj), sr = solid_at(P, B.solid, gi, gj + 1);
                 var = (sl && !sr) ? 1 : ((!sl && sr) ? 2 : 0);
             }
-            if (var == 1)
-                hllc_v<PP>(hr, hr, mirror_v<PP>(sv[Rh], hr, K.hfilm), sv[Rh], su[Rh], su[Rh], sg[Lh],
-                           PP::sqrtp(sg[Lh] * hr), K.hfilm, T0, T1, T2);
-            else if (var == 2)
-                hllc_v<PP>(hl, hl, sv[Lh], mirror_v<PP>(sv[Lh], hl, K.hfilm), su[Lh], su[Lh], sg[Lh], sc[Lh], K.hfilm,
-                           T0, T1, T2);
-            else
-                hllc_v<PP>(hl, hr, sv[Lh], sv[Rh], su[Lh], su[Rh], sg[Lh], sc[Lh], K.hfilm, T0, T1, T2);
-            R *F = sfy + 3 * f2;
-            F[0] = T0; F[1] = T2; F[2] = T1;
-            upb[f] = (T0 > 0) ? 0 : 1;
+            mirror_face<typename PP::Plain>(var, K.hfilm, hl, hr, nl, nr, tl, tr, g, cl);
+            face = sfy + 3 * f2;
+            yface = true;
         }
+        R T0, T1, T2;
+        F pp = make_fast<F>(P);
+        hllc_v<F>(pp, hl, hr, nl, nr, tl, tr, g, cl, K.hfilm, T0, T1, T2);
+        if constexpr (F::kGuarded)
+            if (!pp.ok) {
+                const Flux<R> w = hllc_plain<typename F::Plain>(hl, hr, nl, nr, tl, tr, g, cl, K.hfilm);
+                T0 = w.a; T1 = w.b; T2 = w.c;
+            }
+        face[0] = T0;
+        face[1] = yface ? T2 : T1;
+        face[2] = yface ? T1 : T2;
+        upb[f] = (T0 > 0) ? 0 : 1;
     }
     __syncthreads();
     tile_cell<PP, RS, MAXS, BUDGET, NS>(P, src, dst, zp, zc, zn, smb, L, tc, t, dt, Rr, acc, B.solid, B.z0);
@@ -1638,7 +1933,7 @@ __device__ __forceinline__ void budget_fold(Ctl *ctl, int m, double hi, double l
 }
 
 template <class PP, class RS, int MAXS, bool BUDGET, bool STAGE_M, bool TMA, int NS>
-__global__ void __launch_bounds__(TILE_THREADS, PP::kMinBlocks) k_update_tile(const DevParams P, const BufsT<RS> B, Ctl *ctl,
+__global__ void __launch_bounds__(TILE_THREADS, PP::kMinBlocks) k_update_tile(const __grid_constant__ DevParams P, const BufsT<RS> B, Ctl *ctl,
                                                                   const double *__restrict__ rain, double *partials,
                                                                   double *stage, double *saveflow,
                                                                   const __grid_constant__ TmaMaps tm)
