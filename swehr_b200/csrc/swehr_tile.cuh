@@ -489,9 +489,13 @@ __device__ __forceinline__ TileCoord tile_coord(const DevParams &P, int64_t tile
  * (cp.async of 16 bytes, or one tensor-map box per plane) into shared memory,
  * so the arithmetic never waits on HBM and other CTAs on the SM compute while
  * this one's copies fly.
- *   halo planes  h hu hv totsed dep U_1..U_S   10 rows x (32 + 2 pad) columns
+ *   halo planes  h hu hv totsed dep gz U_1..U_S   10 rows x (32 + 2 pad) columns
  *   cell planes  totm maxvel maxdep [ks] (RS), vinf M_1..M_S (double)   8 x 32
- *   topography   z_prev 12 x 36, z 10 x 36 (double)
+ *   topography   z_prev 8 x 36, z 10 x 36 (double)
+ * gz is the previous step's GZ of the faces' left and lower cells: a plane of
+ * the state since the wave pass reads it, so staging it replaces four
+ * topography reads, a root and a quotient per halo cell by one load (8 bytes
+ * more per FP64 cell, 4 mixed; the z_prev window loses four of its rows).
  * A staged row of a plane of T starts pad = 16 / sizeof(T) columns left of
  * the tile: row r is grid row i0-1+r, column c is grid column (0-based)
  * j0-1-pad+c, so every staged row starts 16-byte aligned in HBM and halo
@@ -505,15 +509,18 @@ struct Cols {
 };
 #define R_J (T_J + 4)       /* staged columns of the (double) topography windows */
 #define HALO_ROWS H_I
-#define ZP_ROWS (T_I + 4)
+#define ZP_ROWS T_I
 #define ZC_ROWS (T_I + 2)
 
-static_assert((size_t)(TILE_THREADS / 32) * B_NTERMS * sizeof(double) <= 4 * N_H * sizeof(float),
+static_assert((size_t)(TILE_THREADS / 32) * B_NTERMS * sizeof(double) <= 4 * (size_t)N_H * sizeof(float),
               "budget reduction fits in the face-state arrays it reuses");
+
+/* halo planes, in staging order */
+enum { HP_H = 0, HP_HU, HP_HV, HP_TS, HP_DEP, HP_GZ, HP_U };
 
 struct StagedLayout {
     /* byte offsets from the start of dynamic shared memory */
-    size_t halo, cell_r, cell_d, zp, zc, u, v, g, c, sed, fx, fy, up, red, total;
+    size_t halo, cell_r, cell_d, zp, zc, u, v, c, sed, fx, fy, up, red, total;
     int nhalo, ncellr, ncelld;
     int hps;              /* elements from one halo plane to the next (rows x staged columns, rounded to 128 bytes) */
     int stage_m;          /* M_k staged here (else read from global memory by the cell stage) */
@@ -529,7 +536,7 @@ struct StagedLayout {
         const size_t rj = (size_t)T_J + 2 * (16 / rs);
         L.hps = (int)(((size_t)HALO_ROWS * rj * rs + 127) / 128 * 128 / rs);
         L.stage_m = stage_m;
-        L.nhalo = 5 + S;
+        L.nhalo = HP_U + S;
         L.ncellr = 4;
         L.ncelld = L.stage_m ? 1 + S : 1;
         L.halo = take((size_t)L.nhalo * L.hps * rs);
@@ -539,22 +546,19 @@ struct StagedLayout {
         L.zc = take((size_t)ZC_ROWS * R_J * sizeof(double));
         L.u = take((size_t)N_H * rs);
         L.v = take((size_t)N_H * rs);
-        L.g = take((size_t)N_H * rs);
         L.c = take((size_t)N_H * rs);
         L.sed = take((size_t)S * N_H * rs);
         L.fx = take((size_t)3 * N_FX * rs);
         L.fy = take((size_t)3 * N_FY * rs);
         L.up = take((size_t)(N_FX + N_FY));
         /* the budget reduction runs after a tile's cells are done, when the
-         * face states u, v, g, c are dead: it reuses their space */
+         * face states u, v, c and SED_k are dead: it reuses their space */
         L.red = L.u;
         L.total = o;
         return L;
     }
 };
 
-/* halo planes, in staging order */
-enum { HP_H = 0, HP_HU, HP_HV, HP_TS, HP_DEP, HP_U };
 /* cell planes: RS then double */
 enum { CR_TOTM = 0, CR_MAXVEL, CR_MAXDEP, CR_KS };
 enum { CD_VINF = 0, CD_M };
@@ -568,6 +572,7 @@ __device__ __forceinline__ const RS *halo_plane_src(const SetV<RS> &s, int p, in
     case HP_HV: return s.hv;
     case HP_TS: return s.totsed;
     case HP_DEP: return s.dep;
+    case HP_GZ: return s.gz;
     default: return s.U + (int64_t)(p - HP_U) * pl;
     }
 }
@@ -614,20 +619,21 @@ __device__ __forceinline__ void stage_load(const DevParams &P, const SetV<RS> &s
             cp16(d + HP_HV * ps, src.hv + go);
             cp16(d + HP_TS * ps, src.totsed + go);
             cp16(d + HP_DEP * ps, src.dep + go);
+            cp16(d + HP_GZ * ps, src.gz + go);
             const RS *u = src.U + go;
             for (int k = 0; k < S; k++) cp16(d + (HP_U + k) * ps, u + (int64_t)k * pl);
         }
     }
-    /* topography: z_prev 12 rows, z 10 rows, 18 pairs each */
+    /* topography: z_prev 8 rows, z 10 rows, 18 pairs each */
     {
         constexpr int NHS = HALO_ROWS * NV;
         const int slot = tid < NHS ? tid + (TILE_THREADS - NHS) : tid - NHS;
-        const int nzs = (ZP_ROWS + ZC_ROWS) * (R_J / 2);                   /* 396 */
+        const int nzs = (ZP_ROWS + ZC_ROWS) * (R_J / 2);                   /* 324 */
         for (int s = slot; s < nzs; s += TILE_THREADS) {
             const bool isp = s < ZP_ROWS * (R_J / 2);
             const int s2 = isp ? s : s - ZP_ROWS * (R_J / 2);
             const int r = s2 / (R_J / 2), k2 = s2 - r * (R_J / 2);
-            const int gi = (isp ? tc.i0 - 2 : tc.i0 - 1) + r, col = tc.j0 - 3 + 2 * k2;   /* double windows: pad 2 */
+            const int gi = (isp ? tc.i0 : tc.i0 - 1) + r, col = tc.j0 - 3 + 2 * k2;   /* double windows: pad 2 */
             if (gi < 1 || gi > P.nx || col < 0 || col >= P.ny) continue;
             double *d = reinterpret_cast<double *>(smb + (isp ? L.zp : L.zc)) + r * R_J + 2 * k2;
             cp16(d, (isp ? zp : zc) + (int64_t)(gi - 1) * P.pitch + col);
@@ -666,19 +672,19 @@ struct SetPlanes;
 template <>
 struct SetPlanes<double> {
     enum { h = P_H, hu = P_HU, hv = P_HV, maxvel = P_MAXVEL, maxdep = P_MAXDEP, totm = P_TOTM, dep = P_DEP,
-           totsed = P_TOTSED, U = P_FIXED, d_vinf = P_VINF };
+           totsed = P_TOTSED, gz = P_GZ, U = P_FIXED, d_vinf = P_VINF };
     static __device__ __forceinline__ int d_M(int S) { return P_FIXED + S; }
 };
 template <>
 struct SetPlanes<float> {
-    enum { h = 0, hu = 1, hv = 2, maxvel = 3, maxdep = 4, totm = 5, dep = 6, totsed = 7, U = 9, d_vinf = 0 };
+    enum { h = 0, hu = 1, hv = 2, maxvel = 3, maxdep = 4, totm = 5, dep = 6, totsed = 7, gz = 8, U = 9, d_vinf = 0 };
     static __device__ __forceinline__ int d_M(int) { return 1; }
 };
 
 /* The same staging as stage_load as tensor-map box copies (planes of one
  * domain), issued by one thread onto the tile's mbarrier: halo boxes of
  * Cols<RS>::rj columns x halo rows at column j0-1-pad, row i0-2 (0-based),
- * the z_prev window one row higher and taller (doubles, column j0-3), cell
+ * the z_prev window of the tile's rows (doubles, column j0-3), cell
  * boxes T_J x T_I at (j0-1, i0-1).  j0-1 is a multiple of T_J and pad is 16
  * bytes of the plane's type, so every box starts on a 16-byte column
  * boundary; rows or columns outside the grid arrive as zeros. */
@@ -690,7 +696,7 @@ __device__ __forceinline__ void stage_load_tma(const DevParams &P, const TmaMaps
     typedef SetPlanes<RS> SP;
     const uint32_t hb = (uint32_t)(HALO_ROWS * Cols<RS>::rj * sizeof(RS));
     const uint32_t cbr = (uint32_t)(T_I * T_J * sizeof(RS)), cbd = (uint32_t)(T_I * T_J * sizeof(double));
-    const uint32_t bytes = (uint32_t)(5 + P.S) * hb + (uint32_t)((ZP_ROWS + ZC_ROWS) * R_J * sizeof(double)) +
+    const uint32_t bytes = (uint32_t)(HP_U + P.S) * hb + (uint32_t)((ZP_ROWS + ZC_ROWS) * R_J * sizeof(double)) +
                            (3u + (P.has_ks ? 1u : 0u)) * cbr + (1u + (L.stage_m ? (uint32_t)P.S : 0u)) * cbd;
     mbar_expect_tx(bar, bytes);
     const CUtensorMap *mh = &tm.m[TM_HALO0 + set], *mc = &tm.m[TM_CELL0 + set], *md = &tm.m[TM_CELLD0 + set];
@@ -701,8 +707,9 @@ __device__ __forceinline__ void stage_load_tma(const DevParams &P, const TmaMaps
     tma_load_3d(halo + HP_HV * L.hps, mh, bar, hx, hy, SP::hv);
     tma_load_3d(halo + HP_TS * L.hps, mh, bar, hx, hy, SP::totsed);
     tma_load_3d(halo + HP_DEP * L.hps, mh, bar, hx, hy, SP::dep);
+    tma_load_3d(halo + HP_GZ * L.hps, mh, bar, hx, hy, SP::gz);
     for (int k = 0; k < P.S; k++) tma_load_3d(halo + (HP_U + k) * L.hps, mh, bar, hx, hy, SP::U + k);
-    tma_load_3d(smb + L.zp, &tm.m[TM_ZP], bar, zx, tc.i0 - 3, (int)((n + 2) % 3));
+    tma_load_3d(smb + L.zp, &tm.m[TM_ZP], bar, zx, cy, (int)((n + 2) % 3));
     tma_load_3d(smb + L.zc, &tm.m[TM_ZC], bar, zx, hy, (int)(n % 3));
     RS *cr = reinterpret_cast<RS *>(smb + L.cell_r);
     double *cd = reinterpret_cast<double *>(smb + L.cell_d);
@@ -733,8 +740,7 @@ __device__ __forceinline__ double sslope_y(const DevParams &P, const double *zs,
 }
 
 /* Derived halo values from the staged planes: h, u = hu/h, v = hv/h (0 when
- * dry), GZ of the previous step and sqrt(GZ h) for left/lower face cells,
- * SED_k.  Ghost cells read their source cell (SWEHR.c:816-1035). */
+ * dry), sqrt(GZ h) with GZ of the previous step, SED_k.  Ghost cells read their source cell (SWEHR.c:816-1035). */
 template <class PP, class RS, int NS = 0>
 __device__ __forceinline__ void stage_derive(const DevParams &P, const SetV<RS> &src, TileCoord tc, unsigned char *smb,
                                              const StagedLayout &L, typename PP::R inh, typename PP::R inhv,
@@ -745,9 +751,8 @@ __device__ __forceinline__ void stage_derive(const DevParams &P, const SetV<RS> 
     const int S = NS ? NS : P.S;
     const RealC<R> &K = kc<R>(P);
     const RS *halo = reinterpret_cast<const RS *>(smb + L.halo);
-    const double *zps = reinterpret_cast<const double *>(smb + L.zp);
     R *su = reinterpret_cast<R *>(smb + L.u), *sv = reinterpret_cast<R *>(smb + L.v);
-    R *sg = reinterpret_cast<R *>(smb + L.g), *sc = reinterpret_cast<R *>(smb + L.c);
+    R *sc = reinterpret_cast<R *>(smb + L.c);
     R *ssed = reinterpret_cast<R *>(smb + L.sed);
     for (int idx = threadIdx.x; idx < N_H; idx += TILE_THREADS) {
         const int hi = idx / H_J, hj = idx - hi * H_J;
@@ -757,9 +762,8 @@ __device__ __forceinline__ void stage_derive(const DevParams &P, const SetV<RS> 
         if (hcorner || gi > P.nx + 1 || gj > P.ny + 1 || (gx && gy)) continue;
         const int si = gi < 1 ? 1 : (gi > P.nx ? P.nx : gi);
         const int sj = gj < 1 ? 1 : (gj > P.ny ? P.ny : gj);
-        /* staged position of the source in the RS planes, and its column in the topography windows */
-        const int sr = si - (tc.i0 - 1), scol = sj - tc.j0 + Cols<RS>::pad, zcol = sj - tc.j0 + 2;
-        const int so = sr * Cols<RS>::rj + scol;
+        /* staged position of the source cell */
+        const int so = (si - (tc.i0 - 1)) * Cols<RS>::rj + sj - tc.j0 + Cols<RS>::pad;
         const bool inflow = gj == P.ny + 1 && P.inflow;
         R h, hu, hv;
         if (inflow) {
@@ -777,8 +781,10 @@ __device__ __forceinline__ void stage_derive(const DevParams &P, const SetV<RS> 
         R u = 0, v = 0;
         if (flow) { u = pp.quot(hu, rh); v = pp.quot(hv, rh); }
         if (gx || gy) {
-            /* ghost cells are never read through the staged planes: keep h there */
-            reinterpret_cast<RS *>(smb + L.halo)[HP_H * L.hps + hi * Cols<RS>::rj + hj + Cols<RS>::pad - 1] = (RS)h;
+            /* no cell reads a ghost's staged planes: keep its h and GZ there */
+            RS *ghost = reinterpret_cast<RS *>(smb + L.halo) + hi * Cols<RS>::rj + hj + Cols<RS>::pad - 1;
+            ghost[HP_H * L.hps] = (RS)h;
+            ghost[HP_GZ * L.hps] = halo[HP_GZ * L.hps + so];
         }
         auto sed_k = [&](int k, R q) {            /* q = U_k / h of a flowing cell */
             R s = 0;
@@ -797,22 +803,8 @@ __device__ __forceinline__ void stage_derive(const DevParams &P, const SetV<RS> 
 #pragma unroll 4
             for (int k = 0; k < S; k++) sed_k(k, flow ? pp.quot((R)U[k * L.hps], rh) : R(0));
         }
-        R g = 0, c = 0, slope2 = 1;
-        const bool left = hi <= T_I && hj <= T_J;      /* the left or lower cell of a face of the tile */
-        if (left) {
-            if (P.has_solid) {
-                /* the state's GZ plane: the previous step's GZ of a flow cell,
-                 * the set-up GZ a solid cell keeps (SWEHR.c:1233) */
-                g = (R)src.gz[cidx(P, si, sj)];
-            } else {
-                /* GZ of the previous step at the source cell, SWEHR.c:1279 via z_prev */
-                const int zr = si - (tc.i0 - 2);
-                const R sx = (R)sslope_x(P, zps, zr, zcol, si), sy = (R)sslope_y(P, zps, zr, zcol, sj);
-                slope2 = sx * sx + sy * sy + 1;
-                g = pp.div(K.g, pp.root1(slope2));
-            }
-            c = pp.sqrtp(g * h);
-        }
+        const R g = (R)halo[HP_GZ * L.hps + so];
+        R c = pp.sqrtp(g * h);
         if constexpr (F::kGuarded) {
             if (!pp.ok) {                         /* an operand the branch-free sequences do not take */
                 typedef typename F::Plain Q;
@@ -820,18 +812,12 @@ __device__ __forceinline__ void stage_derive(const DevParams &P, const SetV<RS> 
                 if (flow) { u = Q::div(hu, h); v = Q::div(hv, h); }
 #pragma unroll 1
                 for (int k = 0; k < S; k++) sed_k(k, flow ? Q::div((R)U[k * L.hps], h) : R(0));
-                if (left) {
-                    if (!P.has_solid) g = Q::div(K.g, Q::sqrtp(slope2));
-                    c = Q::sqrtp(g * h);
-                }
+                c = Q::sqrtp(g * h);
             }
         }
         su[idx] = u;
         sv[idx] = v;
-        if (left) {
-            sg[idx] = g;
-            sc[idx] = c;
-        }
+        sc[idx] = c;
     }
 }
 
@@ -1346,7 +1332,7 @@ __device__ __forceinline__ void tile_cell_pp(PP &pp, const DevParams &P, const S
     const R g = K.g;
     const double *zps = reinterpret_cast<const double *>(smb + L.zp), *zcs = reinterpret_cast<const double *>(smb + L.zc);
     const R sx = (R)sslope_x(P, zcs, ti + 1, tj + 2, i), sy = (R)sslope_y(P, zcs, ti + 1, tj + 2, j);
-    const R syl = (R)sslope_y(P, zps, ti + 2, tj + 2, j);
+    const R syl = (R)sslope_y(P, zps, ti, tj + 2, j);
     const R gx = pp.div(g * sx, pp.root1(sx * sx + syl * syl + 1));
     const R SXf = -gx * h0v;
     const typename PP::Recip rroot = PP::recip(pp.root1(sx * sx + sy * sy + 1));
@@ -1777,7 +1763,7 @@ __device__ __forceinline__ void update_tile(const DevParams &P, const BufsT<RS> 
     if (P.inflow) inflow_ghost(t, inh, inhv, insed);
     unsigned char *upb = smb + L.up;
     const R *su = reinterpret_cast<const R *>(smb + L.u), *sv = reinterpret_cast<const R *>(smb + L.v);
-    const R *sg = reinterpret_cast<const R *>(smb + L.g), *sc = reinterpret_cast<const R *>(smb + L.c);
+    const R *sc = reinterpret_cast<const R *>(smb + L.c);
     R *sfx = reinterpret_cast<R *>(smb + L.fx), *sfy = reinterpret_cast<R *>(smb + L.fy);
     if constexpr (TMA) {
         /* the previous tile's reads and writes of these buffers are done
@@ -1798,7 +1784,7 @@ __device__ __forceinline__ void update_tile(const DevParams &P, const BufsT<RS> 
     }
     stage_derive<PP, RS, NS>(P, src, tc, smb, L, (R)inh, (R)inhv, (R)insed);
     __syncthreads();
-    const RS *sh = staged_h<RS>(smb, L);
+    const RS *sh = staged_h<RS>(smb, L), *sg = sh + HP_GZ * L.hps;
     /* stage B: every face of the tile (SWEHR.c:1099-1230) */
     for (int f = threadIdx.x; f < N_FX + N_FY; f += TILE_THREADS) {
         R hl, hr, nl, nr, tl, tr, g, cl;
@@ -1809,9 +1795,9 @@ __device__ __forceinline__ void update_tile(const DevParams &P, const BufsT<RS> 
             const int gi = tc.i0 - 1 + fi, gj = tc.j0 + fj;
             if (gj > P.ny || gi > P.nx) continue;
             const int Lh = fi * H_J + fj + 1, Rh = Lh + H_J;
-            hl = (R)sh[fi * Cols<RS>::rj + fj + Cols<RS>::pad];
-            hr = (R)sh[(fi + 1) * Cols<RS>::rj + fj + Cols<RS>::pad];
-            nl = su[Lh]; nr = su[Rh]; tl = sv[Lh]; tr = sv[Rh]; g = sg[Lh]; cl = sc[Lh];
+            const int Ls = fi * Cols<RS>::rj + fj + Cols<RS>::pad;
+            hl = (R)sh[Ls]; hr = (R)sh[Ls + Cols<RS>::rj];
+            nl = su[Lh]; nr = su[Rh]; tl = sv[Lh]; tr = sv[Rh]; g = (R)sg[Ls]; cl = sc[Lh];
             int var = 0;                 /* 1: solid left, 2: solid right (SWEHR.c:1137-1146) */
             if (P.has_solid && gi >= 1 && gi < P.nx) {
                 const bool sl = solid_at(P, B.solid, gi, gj), sr = solid_at(P, B.solid, gi + 1, gj);
@@ -1826,9 +1812,9 @@ __device__ __forceinline__ void update_tile(const DevParams &P, const BufsT<RS> 
             const int gi = tc.i0 + fi, gj = tc.j0 - 1 + fj;
             if (gi > P.nx || gj > P.ny) continue;
             const int Lh = (fi + 1) * H_J + fj, Rh = Lh + 1;
-            hl = (R)sh[(fi + 1) * Cols<RS>::rj + fj + Cols<RS>::pad - 1];
-            hr = (R)sh[(fi + 1) * Cols<RS>::rj + fj + Cols<RS>::pad];
-            nl = sv[Lh]; nr = sv[Rh]; tl = su[Lh]; tr = su[Rh]; g = sg[Lh]; cl = sc[Lh];
+            const int Ls = (fi + 1) * Cols<RS>::rj + fj + Cols<RS>::pad - 1;
+            hl = (R)sh[Ls]; hr = (R)sh[Ls + 1];
+            nl = sv[Lh]; nr = sv[Rh]; tl = su[Lh]; tr = su[Rh]; g = (R)sg[Ls]; cl = sc[Lh];
             int var = 0;                 /* 1: solid below, 2: solid above (SWEHR.c:1205-1214) */
             if (P.has_solid && gj >= 1) {
                 const bool sl = solid_at(P, B.solid, gi, gj), sr = solid_at(P, B.solid, gi, gj + 1);

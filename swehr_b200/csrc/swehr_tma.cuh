@@ -30,7 +30,7 @@ enum {
     TM_HALO1,        /* state set 1 */
     TM_CELL0,        /* state set 0, every plane; box tile columns x tile rows x 1 */
     TM_CELL1,        /* state set 1 */
-    TM_ZP,           /* the three topography planes; box R_J x (tile rows + 4) x 1 */
+    TM_ZP,           /* the three topography planes; box R_J x tile rows x 1 */
     TM_ZC,           /* the three topography planes; box R_J x (tile rows + 2) x 1 */
     TM_KS,           /* the Ks plane; box tile columns x tile rows x 1 */
     TM_CELLD0,       /* state set 0, its FP64 planes (vinf, M_k); box tile columns x tile rows x 1 */
