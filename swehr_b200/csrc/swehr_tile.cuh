@@ -289,16 +289,54 @@ struct PolicyF32 {
     static constexpr bool kRollClasses = false;
     static constexpr int kWaveMinBlocks = 5;      /* 48 registers: four cells per thread without spills */
     static constexpr bool kKnownResults = false;
-    /* sqrt on the SFU, x * rsqrt(x) (~3 ulp): the mixed form's ~25 square
-     * roots per cell (wave speeds, gravity, settling, friction) cost a third
-     * of the IEEE sequence; +0 for x <= 0 (the reference's pow(x, 0.5) of a
-     * zero).  The product is rounded on its own (never fused into a later
-     * add), so the single-domain and batched kernels compute the same value. */
-    static __device__ __forceinline__ R sqrtp(R x) { return x > 0.f ? __fmul_rn(x, rsqrtf(x)) : 0.f; }
-    /* x^y for x > 0 as x^n * 2^(f log2 x), n = floor(y), f = y - n in [0,1):
-     * the integer power by multiplication (|n| <= 4), the fractional one on
-     * the SFU.  The SFU's log2 error is then scaled by f < 1 instead of y, so
-     * x^3.333 of a 10 um film errs ~1e-6 instead of ~1e-5 (about 12
+    /* The SFU's functions in the form that takes no denormal operand.  The
+     * other form tests every operand and scales it there and back (two
+     * multiplications and a compare around each of a wet cell's ~100 uses, a
+     * fifth of the mixed update's instructions).  The divisors and radicands
+     * here are depths above the film, sums with one or with such a depth's
+     * wave speed, and constants: normal numbers, for which both forms are the
+     * same.  A quotient keeps a denormal dividend (the reciprocal is what the
+     * SFU computes); roots and powers below 1e-19 and exponentials below 1e-38
+     * come out as (near) zero. */
+    static __device__ __forceinline__ R rcp(R b)
+    {
+        R y;
+        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(b));
+        return y;
+    }
+    static __device__ __forceinline__ R rsqrt(R x)
+    {
+        R y;
+        asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+        return y;
+    }
+    static __device__ __forceinline__ R exp2(R x)
+    {
+        R y;
+        asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+        return y;
+    }
+    static __device__ __forceinline__ R log2(R x)
+    {
+        R y;
+        asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+        return y;
+    }
+    /* sqrt on the SFU, x * rsqrt(x) (~3 ulp), +0 for x <= 0 (the reference's
+     * pow(x, 0.5) of a zero).  The product is rounded on its own (never fused
+     * into a later add), so the single-domain and batched kernels compute the
+     * same value. */
+    static __device__ __forceinline__ R sqrtp(R x)
+    {
+        const R c = fmaxf(x, 0.f);
+        return __fmul_rn(c, rsqrt(fmaxf(c, 1.17549435e-38f)));
+    }
+    /* root of a sum of squares plus one */
+    static __device__ __forceinline__ R root1(R x) { return __fmul_rn(x, rsqrt(x)); }
+    /* x^y for x > 0 as x^n * 2^(f log2 x), n the integer part of y, f = y - n:
+     * the integer power by multiplication (0 <= n <= 4), the fractional one on
+     * the SFU.  The SFU's log2 error is then scaled by |f| < 1 instead of y,
+     * so x^3.333 of a 10 um film errs ~1e-6 instead of ~1e-5 (about 12
      * instructions against ~50 for powf).  Other exponents use powf. */
     static __device__ __forceinline__ R pow(R x, R y)
     {
@@ -306,36 +344,34 @@ struct PolicyF32 {
         if (y == 1.f) return x;
         if (y == 2.f) return x * x;
         if (y == 4.f) { const float x2 = x * x; return x2 * x2; }
-        const float n = floorf(y);
-        if (x > 0.f && x < 3.0e38f && n >= -4.f && n <= 4.f) {
+        const float n = truncf(y);
+        if (x >= 1.17549435e-38f && x < 3.0e38f && y > -1.f && n <= 4.f) {
             const float f = y - n;
             float p = 1.f;
-            const float b = n < 0.f ? __frcp_rn(x) : x;
-            for (int k = 0; k < (int)fabsf(n); k++) p *= b;
-            return f == 0.f ? p : p * exp2f(f * __log2f(x));
+            for (int k = 0; k < (int)n; k++) p *= x;
+            return f == 0.f ? p : p * exp2(f * log2(x));
         }
         return powf(x, y);
     }
-    static __device__ __forceinline__ R exp(R x) { return __expf(x); }
-    static __device__ __forceinline__ R cos_atan(R x) { return rsqrtf(1.f + x * x); }
-    static __device__ __forceinline__ R sin_atan(R x) { return x * rsqrtf(1.f + x * x); }
-    static __device__ __forceinline__ R div(R a, R b) { return __fdividef(a, b); }
-    typedef float Recip;
-    static __device__ __forceinline__ R recip(R b) { return b; }
-    static __device__ __forceinline__ R quot(R a, R b) { return div(a, b); }
-    static __device__ __forceinline__ R quotz(R a, R b) { return div(a, b); }
-    static __device__ __forceinline__ R quotn(R a, R b) { return div(a, b); }
-    static __device__ __forceinline__ R root1(R x) { return sqrtp(x); }
+    static __device__ __forceinline__ R exp(R x) { return exp2(__fmul_rn(x, 1.4426950408889634f)); }
+    static __device__ __forceinline__ R cos_atan(R x) { return rsqrt(1.f + x * x); }
+    static __device__ __forceinline__ R sin_atan(R x) { return x * rsqrt(1.f + x * x); }
+    typedef R Recip;                                /* the reciprocal */
+    static __device__ __forceinline__ R recip(R b) { return rcp(b); }
+    static __device__ __forceinline__ R quot(R a, R y) { return __fmul_rn(a, y); }
+    static __device__ __forceinline__ R quotz(R a, R y) { return quot(a, y); }
+    static __device__ __forceinline__ R quotn(R a, R y) { return quot(a, y); }
+    static __device__ __forceinline__ R div(R a, R b) { return quot(a, rcp(b)); }
     static __device__ __forceinline__ R divz(R a, R b) { return div(a, b); }
     static __device__ __forceinline__ R sqrtz(R x) { return sqrtp(x); }
     static __device__ __forceinline__ R divk(R a, R c, R, int) { return div(a, c); }
     static __device__ __forceinline__ R e3_term(R num, R J, R yJ, int ok, R m) { return divk(num, J, yJ, ok) * m; }
-    static __device__ __forceinline__ R e4_term(R A, R T, R F, R e, R m) { return div(div(A, T) * F, e) * m; }
+    static __device__ __forceinline__ R e4_term(R A, R T, R F, R e, R m) { return quot(quot(A, T) * F, e) * m; }
     static __device__ __forceinline__ R qnan() { return __int_as_float(0x7fc00000); }
     /* settling velocity sqrt(A^2 + c) - A rewritten as c / (sqrt(A^2 + c) + A):
      * equal in exact arithmetic, but for fine classes (d = 2 um: A = 8.37,
      * c = 3e-5) the reference's difference cancels ~7 digits, all of FP32's */
-    static __device__ __forceinline__ R settle(R A, R A2, R c) { return __fdividef(c, sqrtp(A2 + c) + A); }
+    static __device__ __forceinline__ R settle(R A, R A2, R c) { return div(c, sqrtp(A2 + c) + A); }
     /* DEP is stored in FP32 here: a reciprocal multiply is exact enough */
     static __device__ __forceinline__ double dep_of(double M, const DevParams &P) { return M * P.inv_rhos; }
 };
@@ -1426,8 +1462,14 @@ __device__ __forceinline__ void tile_cell_pp(PP &pp, const DevParams &P, const S
         zf = pp.divk(vinf0, P.thetas - P.theta0, P.inv_dtheta, 1);
         need = pp.div(dt * ks * (zf + P.hf + hd), zf);
     } else {
-        zf = PolicyF64::divk(vinf0, P.thetas - P.theta0, P.inv_dtheta, P.divk_ok);
-        need = dt * ks * (zf + P.hf + hd) / zf;
+        zf = sw_quot(vinf0, P.thetas - P.theta0, P.inv_dtheta);
+        double num = dt * ks * (zf + P.hf + hd);
+        need = sw_quot(num, zf, sw_rcp(zf));
+        if (!(P.fast_ok & sw_mid_pos(vinf0) & sw_mid_pos(zf) & sw_mid_or_zero(num))) {
+            zf = vinf0 / (P.thetas - P.theta0);
+            num = dt * ks * (zf + P.hf + hd);
+            need = num / zf;
+        }
     }
     const double infl = fmin(hd - P.hfilm, need);
     const double vinf = vinf0 + infl;
@@ -1773,7 +1815,7 @@ __device__ __forceinline__ void update_tile(const DevParams &P, const BufsT<RS> 
             stage_load_tma<RS>(P, *tm, (int)(n & 1), n, tc, smb, L, bar);
         }
         /* one warp polls, the others wait at the block's barrier: eight polling
-         * warps took issue slots from the SM's other blocks (FP64 update -1.3 %) */
+         * warps take issue slots from the SM's other blocks */
         if (threadIdx.x < 32 && !mbar_wait_bounded(bar, *phase & 1u) && threadIdx.x == 0) ctl->dev_error = 1;
         *phase += 1;
         __syncthreads();
@@ -1933,8 +1975,8 @@ __global__ void __launch_bounds__(TILE_THREADS, PP::kMinBlocks) k_update_tile(co
      * the launch adds 128 bytes and the staging starts at the next boundary.
      * The boundary is an offset from the array, never a rebuilt pointer: from
      * that the compiler no longer knows the address is shared memory, and the
-     * ~125 staged reads of a cell become generic loads (4096^2, ponded flow:
-     * FP64 update 4.70 ms with them, 4.00 ms without; mixed 2.16 and 2.05) */
+     * ~125 staged reads of a cell become generic loads (4096^2, ponded flow,
+     * with the polling below: FP64 update 4.24 -> 4.04 ms, mixed 2.24 -> 2.12) */
     unsigned char *smb = smb_raw + (TMA ? (128u - (smem_addr(smb_raw) & 127u)) & 127u : 0u);
     __shared__ bool last;
     __shared__ __align__(8) uint64_t tma_bar;
