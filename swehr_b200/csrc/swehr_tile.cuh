@@ -1084,6 +1084,27 @@ __device__ __forceinline__ typename PP::R wave_vec(PP &pp, const DevParams &P, c
     return smax;
 }
 
+/* wave_vec with its rare cells computed again */
+template <class PP, class RS>
+__device__ __forceinline__ typename PP::R wave_vec_any(const DevParams &P, const SetV<RS> &src, int i, int j0,
+                                                       typename PP::R inh, typename PP::R inhv)
+{
+    typedef typename PP::R R;
+    typedef typename PP::Fast F;
+    F pp = make_fast<F>(P);
+    R s = wave_vec<F, RS>(pp, P, src, i, j0, inh, inhv);
+    if constexpr (F::kGuarded)
+        if (!pp.ok) {
+            s = 0;
+#pragma unroll 1
+            for (int j = j0; j < j0 + Cols<RS>::pad && j <= P.ny; j++) {
+                const R sj = wave_cell_plain<typename F::Plain, RS>(P, src, i, j, inh, inhv, nullptr);
+                s = (sj > s) ? sj : s;
+            }
+        }
+    return s;
+}
+
 /* block maximum of the threads' partial maxima (result valid in thread 0) */
 __device__ __forceinline__ double block_max(double v, double *red8)
 {
@@ -1119,7 +1140,6 @@ template <class PP, class RS>
 __global__ void __launch_bounds__(TILE_THREADS, PP::kWaveMinBlocks) k_wave_cells(const __grid_constant__ DevParams P, const BufsT<RS> B, Ctl *ctl)
 {
     typedef typename PP::R R;
-    typedef typename PP::Fast F;
     if (!ctl->active) return;
     __shared__ double red8[TILE_THREADS / 32];
     __shared__ bool last;
@@ -1142,17 +1162,7 @@ __global__ void __launch_bounds__(TILE_THREADS, PP::kWaveMinBlocks) k_wave_cells
         for (int64_t c = c0; c < total; c += stride) {
             const int r = (int)(c / nv);
             const int i = r + P.own_lo, j0 = (int)(c - (int64_t)r * nv) * V + 1;
-            F pp = make_fast<F>(P);
-            R s = wave_vec<F, RS>(pp, P, src, i, j0, (R)inh, (R)inhv);
-            if constexpr (F::kGuarded)
-                if (!pp.ok) {
-                    s = 0;
-#pragma unroll 1
-                    for (int j = j0; j < j0 + V && j <= P.ny; j++) {
-                        const R sj = wave_cell_plain<typename F::Plain, RS>(P, src, i, j, (R)inh, (R)inhv, nullptr);
-                        s = (sj > s) ? sj : s;
-                    }
-                }
+            const R s = wave_vec_any<PP, RS>(P, src, i, j0, (R)inh, (R)inhv);
             smax = (s > smax) ? s : smax;
         }
     } else {
@@ -2134,9 +2144,10 @@ __global__ void __launch_bounds__(TILE_THREADS) k_wave_batch(const BatchHdr<RS> 
     if (blockIdx.x == 0 && threadIdx.x == 0) hdr->grab[1] = 0ull;  /* the update pass's counter, for after us */
     for (;;) {
         if (!grab_chunk(hdr->grab, map, total, chunk)) break;
-        for (int c = 0; c < chunk.n; c++) {
-            const int64_t g = chunk.g0 + c;
+        for (int c = 0; c < chunk.n;) {
             const int sid = chunk.sid[c];                        /* uniform across the block */
+            int e = c + 1;                                       /* tiles c..e-1 of the chunk are this scenario's */
+            while (e < chunk.n && chunk.sid[e] == sid) e++;
             if (sid != cur) {
                 if (run) flush();
                 load_desc(tab, sid, sd, snap, false);
@@ -2145,16 +2156,35 @@ __global__ void __launch_bounds__(TILE_THREADS) k_wave_batch(const BatchHdr<RS> 
                 snap_inh = snap_inhv = 0;
                 if (sd.P.inflow) inflow_ghost(snap.t, snap_inh, snap_inhv, insed);
             }
-            if (!snap.go) continue;
-            const int64_t n = snap.n;
-            const TileCoord tc = tile_coord(sd.P, g - sd.tile0);
-            const int i = tc.i0 + (int)threadIdx.x / T_J, j = tc.j0 + (int)threadIdx.x % T_J;
-            if (i <= sd.P.nx && j <= sd.P.ny) {
-                const R s = wave_cell<PP, RS>(sd.P, sd.B.set[n & 1], i, j, (R)snap_inh, (R)snap_inhv,
-                                              sd.P.has_solid ? sd.B.solid : nullptr);
-                smax = (s > smax) ? s : smax;
+            if (snap.go) {
+                const SetV<RS> &src = sd.B.set[snap.n & 1];
+                /* vectors of V cells with 16-byte loads as in k_wave_cells,
+                 * V tiles of the run at a time; beside interior solid cells one
+                 * cell per thread */
+                constexpr int V = Cols<RS>::pad, VROW = T_J / V, VTILE = T_I * VROW;
+                if (!sd.P.has_solid) {
+                    for (int v = threadIdx.x; v < (e - c) * VTILE; v += TILE_THREADS) {
+                        const int r = v % VTILE;
+                        const TileCoord tc = tile_coord(sd.P, chunk.g0 + c + v / VTILE - sd.tile0);
+                        const int i = tc.i0 + r / VROW, j = tc.j0 + (r % VROW) * V;
+                        if (i <= sd.P.nx && j <= sd.P.ny) {
+                            const R s = wave_vec_any<PP, RS>(sd.P, src, i, j, (R)snap_inh, (R)snap_inhv);
+                            smax = (s > smax) ? s : smax;
+                        }
+                    }
+                } else {
+                    for (int k = c; k < e; k++) {
+                        const TileCoord tc = tile_coord(sd.P, chunk.g0 + k - sd.tile0);
+                        const int i = tc.i0 + (int)threadIdx.x / T_J, j = tc.j0 + (int)threadIdx.x % T_J;
+                        if (i <= sd.P.nx && j <= sd.P.ny) {
+                            const R s = wave_cell<PP, RS>(sd.P, src, i, j, (R)snap_inh, (R)snap_inhv, sd.B.solid);
+                            smax = (s > smax) ? s : smax;
+                        }
+                    }
+                }
+                run += e - c;
             }
-            run++;
+            c = e;
         }
     }
     if (run) flush();
