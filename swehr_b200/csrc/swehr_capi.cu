@@ -11,6 +11,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <cmath>
 #include <cstdio>
@@ -18,6 +19,7 @@
 #include <cstring>
 #include <mutex>
 #include <string>
+#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -288,13 +290,19 @@ static int upload_plane(swehr_ctx *c, PlaneRef d, const double *host, cudaStream
 }
 
 /* Rows of a device array (nrows x ncols elements of esize bytes, spitch
- * bytes apart) into contiguous host doubles.  Planes of 32 MB and more go
- * through two pinned 16 MB buffers, the device copy of one chunk overlapping
- * the host copy of the one before (a pageable destination is otherwise
- * filled at a fraction of the link's speed); smaller reads (a serving
- * request's) and pooled contexts return 0 without copying. */
-static const size_t kStageBytes = (size_t)16 << 20;
-static const size_t kStageMin = (size_t)32 << 20;
+ * bytes apart) into contiguous host doubles, through a pinned buffer: a
+ * pageable destination is filled by the driver at 3-4 GB/s.  Up to 32 MB every
+ * part is copied at once, one part per host thread, each thread filling its
+ * share of the destination as soon as its part has landed (the fresh pages of
+ * a destination are the slow half: their faults proceed in parallel).  Larger
+ * planes alternate between the buffer's two halves, the device copy of one
+ * chunk overlapping the host copy of the one before.
+ * Measured (B200 host): five fields of a 1024^2 domain 12.2 ms with pageable
+ * copies, 4.4-5.1 with parts; two fields of 16 pooled mixed catchments of
+ * 64-1024 cells a side 13.9 and 6.0; the 200 x 50 hillslope's five 0.17 and 0.15. */
+static const size_t kStageBytes = (size_t)16 << 20;      /* half of the pinned buffer */
+static const size_t kPartMin = (size_t)512 << 10;        /* device bytes that are worth a thread */
+static const int kStageThreadsMax = 8;
 
 static void stage_part(double *dst, const void *src, size_t n, size_t esize)
 {
@@ -306,17 +314,14 @@ static void stage_part(double *dst, const void *src, size_t n, size_t esize)
     for (size_t q = 0; q < n; q++) dst[q] = (double)f[q];
 }
 
-/* the host side of a chunk, split over a few threads: filling fresh pageable
- * pages is bound by page faults, which proceed in parallel (half the host's
- * hardware threads, 2..8) */
-static const int kStageThreadsMax = 8;
-
+/* host threads of a read: half the hardware threads, 2..8 */
 static int stage_threads()
 {
     static const int T = std::max(2, std::min(kStageThreadsMax, (int)std::thread::hardware_concurrency() / 2));
     return T;
 }
 
+/* the host side of a chunk, split over the threads */
 static void stage_out(double *dst, const void *src, size_t n, size_t esize)
 {
     const int T = stage_threads();
@@ -330,37 +335,46 @@ static void stage_out(double *dst, const void *src, size_t n, size_t esize)
     for (int t = 0; t < T - 1; t++) th[t].join();
 }
 
-static int d2h_staged_copy(swehr_ctx *c, double *host, const void *dev, size_t spitch, size_t esize,
-                           int64_t nrows, int64_t ncols);
-
-static int d2h_staged(swehr_ctx *c, double *host, const void *dev, size_t spitch, size_t esize, int64_t nrows,
-                      int64_t ncols, int *done)
+/* planes up to the pinned buffer's size, in parts */
+static int d2h_parts(swehr_ctx *c, char *stage, double *host, const void *dev, size_t spitch, size_t esize,
+                     int64_t nrows, int64_t ncols)
 {
-    *done = 0;
-    const size_t row_in = (size_t)ncols * esize;
-    if (c->host || row_in * (size_t)nrows < kStageMin || row_in > kStageBytes) return SWEHR_OK;
-    /* one pinned pair per process (pinning takes ~0.1 s), used by one read at a time */
-    static std::mutex mu;
-    static void *stage = nullptr;
-    std::lock_guard<std::mutex> lock(mu);
-    if (!stage) CK(cudaHostAlloc(&stage, 2 * kStageBytes, cudaHostAllocPortable));
-    if (!c->ev_stage[0])
-        for (int e = 0; e < 2; e++) CK(cudaEventCreateWithFlags(&c->ev_stage[e], cudaEventDisableTiming));
-    c->h_stage = stage;
-    const int rc = d2h_staged_copy(c, host, dev, spitch, esize, nrows, ncols);
-    if (rc != SWEHR_OK) {
-        /* a copy into the shared pinned pair may still be in flight: let it
-         * land before the lock is released and the next reader reuses the pair */
-        cudaStreamSynchronize(c->stream);
-        return rc;
+    const size_t row_in = (size_t)ncols * esize, total = row_in * (size_t)nrows;
+    const int T = (int)std::max<size_t>(1, std::min({(size_t)stage_threads(), total / kPartMin, (size_t)nrows}));
+    const int64_t per = (nrows + T - 1) / T;
+    for (int t = 0; t < T; t++) {
+        const int64_t r0 = t * per, n = std::min(per, nrows - r0);
+        if (n <= 0) break;
+        CK(cudaMemcpy2DAsync(stage + (size_t)r0 * row_in, row_in, (const char *)dev + (size_t)r0 * spitch, spitch, row_in,
+                             (size_t)n, cudaMemcpyDeviceToHost, c->stream));
+        CK(cudaEventRecord(c->ev_stage[t], c->stream));
     }
-    *done = 1;
+    std::atomic<int> bad{cudaSuccess};
+    auto part = [&](int t) {
+        const int64_t r0 = t * per, n = std::min(per, nrows - r0);
+        if (n <= 0) return;
+        const cudaError_t e = cudaEventSynchronize(c->ev_stage[t]);
+        if (e != cudaSuccess) bad = (int)e;
+        else stage_part(host + (size_t)r0 * ncols, stage + (size_t)r0 * row_in, (size_t)(n * ncols), esize);
+    };
+    std::thread th[kStageThreadsMax - 1];
+    int made = 0;
+    const int device = c->device;
+    try {
+        for (; made < T - 1; made++) th[made] = std::thread([&, made] { cudaSetDevice(device); part(made + 1); });
+    } catch (const std::system_error &) {
+        /* no more threads: this one fills what is left */
+    }
+    part(0);
+    for (int t = made + 1; t < T; t++) part(t);
+    for (int t = 0; t < made; t++) th[t].join();
+    if (bad) return set_err(SWEHR_CUDA_ERROR, std::string("field download: ") + cudaGetErrorString((cudaError_t)bad.load()));
     return SWEHR_OK;
 }
 
-/* the chunked copy of d2h_staged (its lock held, the pinned pair set up) */
-static int d2h_staged_copy(swehr_ctx *c, double *host, const void *dev, size_t spitch, size_t esize,
-                           int64_t nrows, int64_t ncols)
+/* planes above it, in chunks of half the buffer */
+static int d2h_chunks(swehr_ctx *c, char *stage, double *host, const void *dev, size_t spitch, size_t esize,
+                      int64_t nrows, int64_t ncols)
 {
     const size_t row_in = (size_t)ncols * esize;
     const int64_t per = (int64_t)(kStageBytes / row_in);
@@ -370,14 +384,12 @@ static int d2h_staged_copy(swehr_ctx *c, double *host, const void *dev, size_t s
     for (int64_t r0 = 0; r0 < nrows; r0 += per, k++) {
         const int64_t n = std::min(per, nrows - r0);
         const int b = (int)(k & 1);
-        char *buf = (char *)c->h_stage + (size_t)b * kStageBytes;
-        CK(cudaMemcpy2DAsync(buf, row_in, (const char *)dev + (size_t)r0 * spitch, spitch, row_in, (size_t)n,
-                             cudaMemcpyDeviceToHost, c->stream));
+        CK(cudaMemcpy2DAsync(stage + (size_t)b * kStageBytes, row_in, (const char *)dev + (size_t)r0 * spitch, spitch,
+                             row_in, (size_t)n, cudaMemcpyDeviceToHost, c->stream));
         CK(cudaEventRecord(c->ev_stage[b], c->stream));
         if (prev_r0 >= 0) {
             CK(cudaEventSynchronize(c->ev_stage[prev_b]));
-            stage_out(host + (size_t)prev_r0 * ncols, (char *)c->h_stage + (size_t)prev_b * kStageBytes,
-                      (size_t)prev_n * ncols, esize);
+            stage_out(host + (size_t)prev_r0 * ncols, stage + (size_t)prev_b * kStageBytes, (size_t)prev_n * ncols, esize);
         }
         prev_r0 = r0;
         prev_n = n;
@@ -385,10 +397,49 @@ static int d2h_staged_copy(swehr_ctx *c, double *host, const void *dev, size_t s
     }
     if (prev_r0 >= 0) {
         CK(cudaEventSynchronize(c->ev_stage[prev_b]));
-        stage_out(host + (size_t)prev_r0 * ncols, (char *)c->h_stage + (size_t)prev_b * kStageBytes,
-                  (size_t)prev_n * ncols, esize);
+        stage_out(host + (size_t)prev_r0 * ncols, stage + (size_t)prev_b * kStageBytes, (size_t)prev_n * ncols, esize);
     }
     return SWEHR_OK;
+}
+
+/* the rows are in host when it returns (SWEHR_OK) */
+static int d2h_rows(swehr_ctx *c, double *host, const void *dev, size_t spitch, size_t esize, int64_t nrows,
+                    int64_t ncols)
+{
+    const size_t row_in = (size_t)ncols * esize;
+    if (row_in > kStageBytes) {          /* a single row beyond the buffer: straight to the pageable destination */
+        std::vector<float> tmp(esize == sizeof(double) ? 0 : (size_t)(nrows * ncols));
+        void *dst = esize == sizeof(double) ? (void *)host : (void *)tmp.data();
+        CK(cudaMemcpy2DAsync(dst, row_in, dev, spitch, row_in, (size_t)nrows, cudaMemcpyDeviceToHost, c->stream));
+        CK(cudaStreamSynchronize(c->stream));
+        for (size_t q = 0; q < tmp.size(); q++) host[q] = (double)tmp[q];
+        return SWEHR_OK;
+    }
+    /* one pinned buffer per process, used by one read at a time, as large as
+     * the largest read needed (pinning 32 MB takes ~0.1 s) */
+    static std::mutex mu;
+    static char *stage = nullptr;
+    static size_t held = 0;
+    std::lock_guard<std::mutex> lock(mu);
+    const size_t need = std::min(row_in * (size_t)nrows, 2 * kStageBytes);
+    if (need > held) {
+        size_t want = (size_t)1 << 20;
+        while (want < need) want *= 2;
+        if (stage) CK(cudaFreeHost(stage));
+        stage = nullptr;
+        held = 0;
+        CK(cudaHostAlloc((void **)&stage, want, cudaHostAllocPortable));
+        held = want;
+    }
+    for (int e = 0; e < kStageThreadsMax; e++)
+        if (!c->ev_stage[e]) CK(cudaEventCreateWithFlags(&c->ev_stage[e], cudaEventDisableTiming));
+    const int rc = row_in * (size_t)nrows <= 2 * kStageBytes
+                       ? d2h_parts(c, stage, host, dev, spitch, esize, nrows, ncols)
+                       : d2h_chunks(c, stage, host, dev, spitch, esize, nrows, ncols);
+    /* after an error a copy into the shared buffer may still be in flight: let
+     * it land before the lock is released and the next reader reuses it */
+    if (rc != SWEHR_OK) cudaStreamSynchronize(c->stream);
+    return rc;
 }
 
 /* the lagged GZ the wave pass of step n reads, from z of step n-1 */
@@ -400,23 +451,9 @@ static int init_gz(swehr_ctx *c, int64_t n)
     return SWEHR_OK;
 }
 
-static int download_plane(swehr_ctx *c, double *host, PlaneRef d, cudaStream_t s)
+static int download_plane(swehr_ctx *c, double *host, PlaneRef d)
 {
-    const size_t N = (size_t)c->P.nx * c->P.ny;
-    int staged = 0;
-    int rc = d2h_staged(c, host, d.ptr, (size_t)c->P.pitch * d.esize, d.esize, c->P.nx, c->P.ny, &staged);
-    if (rc || staged) return rc;
-    if (d.esize == sizeof(double)) {
-        CK(cudaMemcpy2DAsync(host, (size_t)c->P.ny * sizeof(double), d.ptr, (size_t)c->P.pitch * sizeof(double),
-                             (size_t)c->P.ny * sizeof(double), (size_t)c->P.nx, cudaMemcpyDeviceToHost, s));
-        return SWEHR_OK;
-    }
-    std::vector<float> tmp(N);
-    CK(cudaMemcpy2DAsync(tmp.data(), (size_t)c->P.ny * sizeof(float), d.ptr, (size_t)c->P.pitch * sizeof(float),
-                         (size_t)c->P.ny * sizeof(float), (size_t)c->P.nx, cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
-    for (size_t q = 0; q < N; q++) host[q] = (double)tmp[q];
-    return SWEHR_OK;
+    return d2h_rows(c, host, d.ptr, (size_t)c->P.pitch * d.esize, d.esize, c->P.nx, c->P.ny);
 }
 
 template <class RS>
@@ -468,8 +505,8 @@ static void destroy_ctx(swehr_ctx *c)
     if (c->ev_stop) cudaEventDestroy(c->ev_stop);
     for (int e = 0; e < 2 * TIMING_RING; e++)
         if (c->ev_k[e]) cudaEventDestroy(c->ev_k[e]);
-    for (int e = 0; e < 2; e++)
-        if (c->ev_stage[e]) cudaEventDestroy(c->ev_stage[e]);
+    for (cudaEvent_t e : c->ev_stage)
+        if (e) cudaEventDestroy(e);
     if (c->host) {
         if (c->mem) c->host->release(c->host->self, c->mem);
         free(c->h_ctl);
@@ -869,17 +906,9 @@ static int read_derived(swehr_ctx *c, int field, int k, int cur, double *dst)
         k_derived<float><<<grid, threads, 0, c->stream>>>((const float *)h.ptr, (const float *)d.ptr,
                                                            (const float *)e.ptr, c->P.nx, c->P.ny, c->P.pitch,
                                                            c->P.hfilm, vel, tmp);
-    cudaError_t err = cudaGetLastError();
-    if (err == cudaSuccess) {
-        int staged = 0;
-        const int rc = d2h_staged(c, dst, tmp, (size_t)c->P.ny * sizeof(double), sizeof(double), c->P.nx, c->P.ny,
-                                  &staged);
-        if (rc) return rc;
-        if (!staged) err = cudaMemcpyAsync(dst, tmp, N * sizeof(double), cudaMemcpyDeviceToHost, c->stream);
-    }
+    const cudaError_t err = cudaGetLastError();
     if (err != cudaSuccess) return set_err(SWEHR_CUDA_ERROR, std::string("derived field: ") + cudaGetErrorString(err));
-    CK(cudaStreamSynchronize(c->stream));
-    return SWEHR_OK;
+    return d2h_rows(c, dst, tmp, (size_t)c->P.ny * sizeof(double), sizeof(double), c->P.nx, c->P.ny);
 }
 
 extern "C" int swehr_read_field(swehr_ctx *c, int field, int k, double *dst)
@@ -893,17 +922,14 @@ extern "C" int swehr_read_field(swehr_ctx *c, int field, int k, double *dst)
     if (rc) return rc;
     const int cur = (int)(step & 1);
     if (field == SWEHR_FIELD_Z) {
-        rc = download_plane(c, dst, z_plane(c, step), c->stream);
+        return download_plane(c, dst, z_plane(c, step));
     } else if (field == SWEHR_FIELD_VEL || field == SWEHR_FIELD_SED) {
         return read_derived(c, field, k, cur, dst);
     } else {
         PlaneRef src = field_plane(c, field, k, cur);
         if (!src.ptr) return set_err(SWEHR_INVALID, "unknown field");
-        rc = download_plane(c, dst, src, c->stream);
+        return download_plane(c, dst, src);
     }
-    if (rc) return rc;
-    CK(cudaStreamSynchronize(c->stream));
-    return SWEHR_OK;
 }
 
 extern "C" int swehr_write_field(swehr_ctx *c, int field, int k, const double *src)

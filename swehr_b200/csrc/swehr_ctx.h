@@ -43,8 +43,7 @@ struct swehr_ctx {
     cudaGraphExec_t graph = nullptr;
     cudaEvent_t ev_start = nullptr, ev_stop = nullptr;
     cudaEvent_t ev_k[2 * TIMING_RING] = {};
-    void *h_stage = nullptr;           /* the process's two pinned download buffers (set on the first large read) */
-    cudaEvent_t ev_stage[2] = {};
+    cudaEvent_t ev_stage[8] = {};      /* parts of a field download (made on the first read) */
     swehr::StepConfig cfg;
     swehr::TmaMaps tm;      /* tensor maps of the update's tile loads (when cfg.tma) */
     int timing = 0;

@@ -51,3 +51,20 @@ def test_large_plane_roundtrip_and_derived(precision):
     assert np.array_equal(got["vel"], vel)
     assert np.array_equal(got["sed"], sed)
     assert wet.any() and (~wet).any()
+
+
+# one part, the smallest plane of two parts and one row less, ragged parts, more threads' worth than rows
+PART_SIDES = [(3, 51), (256, 512), (255, 512), (701, 1531), (2, 200000), (2047, 2049)]
+
+
+@pytest.mark.parametrize("precision", [FP64, MIXED], ids=["fp64", "mixed"])
+@pytest.mark.parametrize("nx,ny", PART_SIDES)
+def test_planes_read_in_parts(nx, ny, precision):
+    from swehr_b200.lib import Simulation
+    case = W.tiny_case(nx=nx, ny=ny, S=1, per_cell_ks=False)
+    a = np.random.default_rng(nx + ny).uniform(0.0, 1.0, (nx, ny))
+    with Simulation(case, precision=precision) as s:
+        s.write_field("h", a)
+        assert np.array_equal(s.field("h"), a if precision == FP64 else a.astype(np.float32).astype(np.float64))
+        s.write_field("z", a)
+        assert np.array_equal(s.field("z"), a)
