@@ -708,6 +708,17 @@ static int launch_step(swehr_ctx *c, cudaEvent_t ev0, cudaEvent_t ev1)
                            c->cfg, c->stream, ev0, ev1);
 }
 
+static int launch_run(swehr_ctx *c, int steps)
+{
+    const int e = c->precision == SWEHR_MIXED
+                      ? launch_run_f32(c->P, c->B32, c->d_ctl, c->d_rain, c->d_stage, c->d_saveflow, c->tm,
+                                       c->cfg, steps, c->stream)
+                      : launch_run_f64(c->P, c->B64, c->d_ctl, c->d_rain, c->d_stage, c->d_saveflow, c->tm,
+                                       c->cfg, steps, c->stream);
+    if (e) return set_err(SWEHR_CUDA_ERROR, std::string("launch: ") + cudaGetErrorString((cudaError_t)e));
+    return SWEHR_OK;
+}
+
 static int build_graph(swehr_ctx *c)
 {
     if (c->graph) return SWEHR_OK;
@@ -769,6 +780,20 @@ extern "C" int swehr_advance(swehr_ctx *c, double t_stop, int64_t max_steps, swe
                 }
                 if (max_steps >= 0) left -= n;
                 if (!h->active || (max_steps >= 0 && left <= 0)) break;
+            }
+        } else if (c->cfg.fn_run) {
+            /* RUN_STEPS steps a launch; one that finds the run stopped returns at once */
+            int64_t left = max_steps;
+            for (;;) {
+                const int n = max_steps >= 0 && left < RUN_STEPS ? (int)left : RUN_STEPS;
+                const int rcr = launch_run(c, n);
+                if (rcr) return rcr;
+                launched++;
+                left -= n;
+                if (max_steps >= 0 && left > 0) continue;
+                CK(cudaMemcpyAsync(h, c->d_ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, c->stream));
+                CK(cudaStreamSynchronize(c->stream));
+                if (max_steps >= 0 || !h->active) break;
             }
         } else {
             int rcg = build_graph(c);

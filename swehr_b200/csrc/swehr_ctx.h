@@ -11,6 +11,7 @@
 #include "swehr_kernels.h"
 
 static const int GRAPH_STEPS = 32;
+static const int RUN_STEPS = 128;        /* steps of one k_run_tile launch */
 static const int TIMING_RING = 64;
 
 /* What a pool lends the contexts it creates: its stream and a device-memory

@@ -109,6 +109,9 @@ struct Ctl {
     double sed0[16];
     int32_t dev_error;                      /* a bounded device-side wait gave up (SWEHR_TIMEOUT) */
     int32_t pad_err;
+    /* k_run_tile: arrivals at its grid barriers, and the largest wave speed of
+     * even and odd steps (0 between launches) */
+    unsigned long long run_count, run_smax[2];
 };
 
 /* budget term slots */

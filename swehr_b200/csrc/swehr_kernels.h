@@ -88,6 +88,10 @@ struct StepConfig {
     size_t smem_wave = 0, smem_update = 0;
     void *fn_update = nullptr, *fn_wave = nullptr;
     int stage_m = 1;                    /* the update stages M_k in shared memory */
+    /* many steps a launch (k_run_tile), null where two kernels a step are faster;
+     * its grid is grid_update */
+    void *fn_run = nullptr;
+    size_t smem_run = 0;
     int tma = 0;                        /* in: tensor maps can be encoded; out: the update loads tiles through them */
 };
 
@@ -108,6 +112,9 @@ int launch_update_f64(const DevParams &P, const BufsT<double> &B, Ctl *ctl, cons
                       double *stage, double *saveflow, const TmaMaps &tm, const StepConfig &cfg, cudaStream_t s);
 int launch_update_f32(const DevParams &P, const BufsT<float> &B, Ctl *ctl, const double *rain, double *partials,
                       double *stage, double *saveflow, const TmaMaps &tm, const StepConfig &cfg, cudaStream_t s);
+/* Enqueue up to `steps` whole steps in one cooperative launch (cfg.fn_run) */
+int launch_run_f64(const DevParams &P, const BufsT<double> &B, Ctl *ctl, const double *rain, double *stage, double *saveflow, const TmaMaps &tm, const StepConfig &cfg, int steps, cudaStream_t s);
+int launch_run_f32(const DevParams &P, const BufsT<float> &B, Ctl *ctl, const double *rain, double *stage, double *saveflow, const TmaMaps &tm, const StepConfig &cfg, int steps, cudaStream_t s);
 /* the update kernel's tile loads through tensor maps (one domain): whether
  * the driver offers the encoder, and the maps of a simulation's planes (0
  * when all were encoded) */

@@ -55,6 +55,20 @@ static inline bool encode_planes(TensorMapEncodeFn enc, CUtensorMap *m, const vo
 
 inline namespace SWEHR_TILE_NS {
 
+/* Tiles per SM up to which a domain is stepped by k_run_tile.  Measured (B200,
+ * 7 classes, ponded flow, us a step, two kernels and many steps a launch):
+ *   tiles      1     64    175    384    750   1536   65536
+ *   FP64    35.0   32.4   33.7   48.6   74.0  139.1    4228
+ *           32.3   28.2   31.4   47.1   71.7  141.4    4346
+ *   mixed   22.5   21.2   23.8   26.2   37.1   60.0    1858
+ *           19.9   17.8   20.3   23.1   33.7   61.6    1884
+ * What a launch saves is the same at any size, but the wave pass runs at the
+ * update's occupancy and a block's tiles wait for the slowest block at every
+ * barrier.  With interior solid cells (the wave pass takes one cell a thread:
+ * 517 x 389, 10 classes 134 and 150 us) and with budgets (block 0 folds the
+ * sums between two barriers: 200 x 50 mixed 40 and 47 us) two kernels stay. */
+#define RUN_TILES_PER_SM 4
+
 template <class PP, class RS>
 struct FormLauncher {
     typedef typename PP::R R;
@@ -134,12 +148,30 @@ struct FormLauncher {
         /* the class counts of the benchmark configurations get kernels
          * built for exactly that many classes: their class loops have no
          * exit tests, so the compiler interleaves the classes' independent
-         * division chains (mixed form -7 %) */
-        if (S == 7) return update_fn<8, BUDGET, SM, TMA, 7>();
-        if (S == 10) return update_fn<16, BUDGET, SM, TMA, 10>();
+         * division chains (mixed form -7 %); not for the fallback without
+         * tensor maps */
+        if constexpr (TMA) {
+            if (S == 7) return update_fn<8, BUDGET, SM, TMA, 7>();
+            if (S == 10) return update_fn<16, BUDGET, SM, TMA, 10>();
+        }
         if (S <= 4) return update_fn<4, BUDGET, SM, TMA>();
         if (S <= 8) return update_fn<8, BUDGET, SM, TMA>();
         return update_fn<16, BUDGET, SM, TMA>();
+    }
+
+    template <int MAXS, int NS = 0>
+    static void *run_fn(bool sm)
+    {
+        return sm ? (void *)k_run_tile<PP, RS, MAXS, true, NS> : (void *)k_run_tile<PP, RS, MAXS, false, NS>;
+    }
+    /* the same class counts as pick_u */
+    static void *pick_run(int S, bool sm)
+    {
+        if (S == 7) return run_fn<8, 7>(sm);
+        if (S == 10) return run_fn<16, 10>(sm);
+        if (S <= 4) return run_fn<4>(sm);
+        if (S <= 8) return run_fn<8>(sm);
+        return run_fn<16>(sm);
     }
 
     template <bool TMA>
@@ -184,6 +216,21 @@ struct FormLauncher {
         cfg.fn_update = fu;
         cfg.fn_wave = fw;
         cfg.stage_m = stage_m;
+        cfg.fn_run = nullptr;
+        if (tma && !P.budget && !P.has_solid && ntiles <= (int64_t)RUN_TILES_PER_SM * num_sms) {
+            void *fr = pick_run(P.S, stage_m != 0);
+            int occ = 0, coop = 0, dev = 0;
+            e = cudaFuncSetAttribute(fr, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)su);
+            if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fr, TILE_THREADS, su);
+            if (e == cudaSuccess) e = cudaGetDevice(&dev);
+            if (e == cudaSuccess) e = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
+            if (e != cudaSuccess) return (int)e;
+            /* every block resident at once */
+            if (coop && (int64_t)num_sms * occ >= cfg.grid_update) {
+                cfg.fn_run = fr;
+                cfg.smem_run = su;
+            }
+        }
         return 0;
     }
 
@@ -261,6 +308,14 @@ struct FormLauncher {
         cudaLaunchKernel(cfg.fn_update, dim3(cfg.grid_update), dim3(TILE_THREADS), args, cfg.smem_update, s);
         if (ev1) cudaEventRecord(ev1, s);
         return (int)cudaGetLastError();
+    }
+
+    static int launch_run(const DevParams &P, const BufsT<RS> &B, Ctl *ctl, const double *rain, double *stage, double *saveflow, const TmaMaps &tm, const StepConfig &cfg, int steps,
+                          cudaStream_t s)
+    {
+        void *args[] = {(void *)&P, (void *)&B, (void *)&ctl, (void *)&rain, (void *)&stage,
+                        (void *)&saveflow, (void *)&tm, (void *)&steps};
+        return (int)cudaLaunchCooperativeKernel(cfg.fn_run, dim3(cfg.grid_update), dim3(TILE_THREADS), args, cfg.smem_run, s);
     }
 
     /* the two passes of a step one at a time (a slab of a split domain takes

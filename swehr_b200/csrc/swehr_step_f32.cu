@@ -25,6 +25,11 @@ int launch_update_f32(const DevParams &P, const BufsT<float> &B, Ctl *ctl, const
     return FormLauncher<PolicyF32, float>::launch_update(P, B, ctl, rain, partials, stage, saveflow, tm, cfg, s);
 }
 
+int launch_run_f32(const DevParams &P, const BufsT<float> &B, Ctl *ctl, const double *rain, double *stage, double *saveflow, const TmaMaps &tm, const StepConfig &cfg, int steps, cudaStream_t s)
+{
+    return FormLauncher<PolicyF32, float>::launch_run(P, B, ctl, rain, stage, saveflow, tm, cfg, steps, s);
+}
+
 int init_gz_f32(const DevParams &P, const BufsT<float> &B, int64_t n, cudaStream_t s)
 {
     return FormLauncher<PolicyF32, float>::init_gz(P, B, n, s);

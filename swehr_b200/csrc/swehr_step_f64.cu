@@ -38,6 +38,11 @@ int launch_update_f64(const DevParams &P, const BufsT<double> &B, Ctl *ctl, cons
     return FormLauncher<PolicyF64, double>::launch_update(P, B, ctl, rain, partials, stage, saveflow, tm, cfg, s);
 }
 
+int launch_run_f64(const DevParams &P, const BufsT<double> &B, Ctl *ctl, const double *rain, double *stage, double *saveflow, const TmaMaps &tm, const StepConfig &cfg, int steps, cudaStream_t s)
+{
+    return FormLauncher<PolicyF64, double>::launch_run(P, B, ctl, rain, stage, saveflow, tm, cfg, steps, s);
+}
+
 int init_gz_f64(const DevParams &P, const BufsT<double> &B, int64_t n, cudaStream_t s)
 {
     return FormLauncher<PolicyF64, double>::init_gz(P, B, n, s);

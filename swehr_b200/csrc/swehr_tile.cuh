@@ -986,14 +986,18 @@ __device__ __forceinline__ typename PP::R wave_cell(const DevParams &P, const Se
 /* V = 16 / sizeof(RS) consecutive elements of a plane with one 16-byte
  * load (p is 16-byte aligned: the vector starts on a column multiple of V
  * of a row whose pitch is a multiple of 32), converted to R */
-template <class RS, class R>
-__device__ __forceinline__ void load_vec(const RS *__restrict__ p, R *out)
+/* LIVE: the plane was written by this very launch (k_run_tile), so the load
+ * goes to L2 and not through the read-only path */
+template <class RS, class R, bool LIVE>
+__device__ __forceinline__ void load_vec(const RS *p, R *out)
 {
     if constexpr (sizeof(RS) == 4) {
-        const float4 a = __ldg(reinterpret_cast<const float4 *>(p));
+        const float4 *v = reinterpret_cast<const float4 *>(p);
+        const float4 a = LIVE ? __ldcg(v) : __ldg(v);
         out[0] = (R)a.x; out[1] = (R)a.y; out[2] = (R)a.z; out[3] = (R)a.w;
     } else {
-        const double2 a = __ldg(reinterpret_cast<const double2 *>(p));
+        const double2 *v = reinterpret_cast<const double2 *>(p);
+        const double2 a = LIVE ? __ldcg(v) : __ldg(v);
         out[0] = (R)a.x; out[1] = (R)a.y;
     }
 }
@@ -1003,7 +1007,7 @@ __device__ __forceinline__ void load_vec(const RS *__restrict__ p, R *out)
  * wave_cell_g for each cell (no interior solid cells), with every plane read
  * V cells per load.  A cell's normal velocity towards its right neighbour in
  * the vector is that neighbour's own velocity, formed once. */
-template <class PP, class RS>
+template <class PP, class RS, bool LIVE>
 __device__ __forceinline__ typename PP::R wave_vec(PP &pp, const DevParams &P, const SetV<RS> &src, int i, int j0,
                                                    typename PP::R inh, typename PP::R inhv)
 {
@@ -1012,21 +1016,21 @@ __device__ __forceinline__ typename PP::R wave_vec(PP &pp, const DevParams &P, c
     const RealC<R> &K = kc<R>(P);
     const int64_t q = cidx(P, i, j0);
     R h[V], hu[V], hv[V], g[V], u[V], v[V], hd[V], hud[V];
-    load_vec<RS, R>(src.h + q, h);
-    load_vec<RS, R>(src.hu + q, hu);
-    load_vec<RS, R>(src.hv + q, hv);
-    load_vec<RS, R>(src.gz + q, g);
+    load_vec<RS, R, LIVE>(src.h + q, h);
+    load_vec<RS, R, LIVE>(src.hu + q, hu);
+    load_vec<RS, R, LIVE>(src.hv + q, hv);
+    load_vec<RS, R, LIVE>(src.gz + q, g);
     const bool below = i < P.nx;
     if (below) {
-        load_vec<RS, R>(src.h + q + P.pitch, hd);
-        load_vec<RS, R>(src.hu + q + P.pitch, hud);
+        load_vec<RS, R, LIVE>(src.h + q + P.pitch, hd);
+        load_vec<RS, R, LIVE>(src.hu + q + P.pitch, hud);
     }
     /* the cell after the vector, for the last cell's y face */
     const int jl = j0 + V;
     R hn = 0, hvn = 0;
     if (jl <= P.ny) {
-        hn = (R)src.h[q + V];
-        hvn = (R)src.hv[q + V];
+        hn = (R)(LIVE ? __ldcg(src.h + q + V) : src.h[q + V]);
+        hvn = (R)(LIVE ? __ldcg(src.hv + q + V) : src.hv[q + V]);
     }
 #pragma unroll
     for (int k = 0; k < V; k++) {
@@ -1085,14 +1089,14 @@ __device__ __forceinline__ typename PP::R wave_vec(PP &pp, const DevParams &P, c
 }
 
 /* wave_vec with its rare cells computed again */
-template <class PP, class RS>
+template <class PP, class RS, bool LIVE = false>
 __device__ __forceinline__ typename PP::R wave_vec_any(const DevParams &P, const SetV<RS> &src, int i, int j0,
                                                        typename PP::R inh, typename PP::R inhv)
 {
     typedef typename PP::R R;
     typedef typename PP::Fast F;
     F pp = make_fast<F>(P);
-    R s = wave_vec<F, RS>(pp, P, src, i, j0, inh, inhv);
+    R s = wave_vec<F, RS, LIVE>(pp, P, src, i, j0, inh, inhv);
     if constexpr (F::kGuarded)
         if (!pp.ok) {
             s = 0;
@@ -1103,6 +1107,43 @@ __device__ __forceinline__ typename PP::R wave_vec_any(const DevParams &P, const
             }
         }
     return s;
+}
+
+/* This thread's share (of nthreads, number me) of the faces of the context's
+ * rows; every wave pass over one context. */
+template <class PP, class RS, bool LIVE>
+__device__ __forceinline__ typename PP::R wave_rows(const DevParams &P, const SetV<RS> &src, int64_t me, int64_t nthreads,
+                                                    typename PP::R inh, typename PP::R inhv, const uint8_t *solid)
+{
+    typedef typename PP::R R;
+    /* the cells of the rows this context updates; a face belongs to the
+     * row of its lower (left) cell, face 1/2 to row 1 */
+    R smax = 0;
+    if (!P.has_solid) {
+        /* V cells per thread and 16-byte loads (the pass is bound by load latency) */
+        constexpr int V = Cols<RS>::pad;
+        const int nv = (P.ny + V - 1) / V;
+        const int64_t total = (int64_t)(P.own_hi - P.own_lo + 1) * nv;
+        for (int64_t c = me; c < total; c += nthreads) {
+            const int r = (int)(c / nv);
+            const int i = r + P.own_lo, j0 = (int)(c - (int64_t)r * nv) * V + 1;
+            const R s = wave_vec_any<PP, RS, LIVE>(P, src, i, j0, inh, inhv);
+            smax = (s > smax) ? s : smax;
+        }
+    } else {
+        /* cells in i-major order, j contiguous; (i, j) advanced by the stride */
+        const int64_t total = (int64_t)(P.own_hi - P.own_lo + 1) * P.ny;
+        const int si = (int)(nthreads / P.ny), sj = (int)(nthreads - (int64_t)si * P.ny);
+        int i = (int)(me / P.ny) + P.own_lo, j = (int)(me - (int64_t)(i - P.own_lo) * P.ny) + 1;
+        for (int64_t c = me; c < total; c += nthreads) {
+            const R s = wave_cell<PP, RS>(P, src, i, j, inh, inhv, solid);
+            smax = (s > smax) ? s : smax;
+            i += si;
+            j += sj;
+            if (j > P.ny) { j -= P.ny; i++; }
+        }
+    }
+    return smax;
 }
 
 /* block maximum of the threads' partial maxima (result valid in thread 0) */
@@ -1118,26 +1159,37 @@ __device__ __forceinline__ double block_max(double v, double *red8)
     return m;
 }
 
-/* CFL time step once every face of the step is in (SWEHR.c:1409-1413); one thread */
+/* CFL time step from the largest wave speed (SWEHR.c:1409-1413) */
+struct StepSize {
+    double dt, courant;
+};
+__device__ __forceinline__ StepSize step_size(const DevParams &P, double t, double Smax)
+{
+    StepSize s;
+    s.dt = P.cstable * P.dx / Smax;
+    if (s.dt > P.maxstep) s.dt = P.maxstep;
+    if (t + s.dt > P.tend) s.dt = P.tend - t;
+    s.courant = Smax * s.dt * P.oneoverdx;
+    return s;
+}
+
+/* ... once every face of the step is in; one thread */
 __device__ __forceinline__ void wave_finalize(const DevParams &P, Ctl *ctl)
 {
     __threadfence();
-    const double t = ctl->t;
     const double Smax = __longlong_as_double((long long)atomicAdd(&ctl->smax_bits, 0ull));
-    double dt = P.cstable * P.dx / Smax;
-    if (dt > P.maxstep) dt = P.maxstep;
-    if (t + dt > P.tend) dt = P.tend - t;
-    const double courant = Smax * dt * P.oneoverdx;
-    ctl->dt = dt;
-    ctl->courant = courant;
-    ctl->cfl = courant > 1;
+    const StepSize s = step_size(P, ctl->t, Smax);
+    ctl->dt = s.dt;
+    ctl->courant = s.courant;
+    ctl->cfl = s.courant > 1;
     ctl->smax_bits = 0ull;
     ctl->wave_ticket = 0u;
     ctl->pending = 1;
 }
 
 template <class PP, class RS>
-__global__ void __launch_bounds__(TILE_THREADS, PP::kWaveMinBlocks) k_wave_cells(const __grid_constant__ DevParams P, const BufsT<RS> B, Ctl *ctl)
+__global__ void __launch_bounds__(TILE_THREADS, PP::kWaveMinBlocks) k_wave_cells(const __grid_constant__ DevParams P, const __grid_constant__ BufsT<RS> B,
+                                                                              Ctl *ctl)
 {
     typedef typename PP::R R;
     if (!ctl->active) return;
@@ -1145,38 +1197,11 @@ __global__ void __launch_bounds__(TILE_THREADS, PP::kWaveMinBlocks) k_wave_cells
     __shared__ bool last;
     const int64_t n = ctl->step;
     const double t = ctl->t;
-    const SetV<RS> src = B.set[n & 1];
+    const SetV<RS> &src = B.set[n & 1];
     double inh = 0, inhv = 0, insed = 0;
     if (P.inflow) inflow_ghost(t, inh, inhv, insed);
-    /* cells in i-major order, j contiguous; (i, j) advanced by the stride */
-    /* the cells of the rows this context updates; a face belongs to the
-     * row of its lower (left) cell, face 1/2 to row 1 */
-    R smax = 0;
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    const int64_t c0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (!P.has_solid) {
-        /* V cells per thread and 16-byte loads (the pass is bound by load latency) */
-        constexpr int V = Cols<RS>::pad;
-        const int nv = (P.ny + V - 1) / V;
-        const int64_t total = (int64_t)(P.own_hi - P.own_lo + 1) * nv;
-        for (int64_t c = c0; c < total; c += stride) {
-            const int r = (int)(c / nv);
-            const int i = r + P.own_lo, j0 = (int)(c - (int64_t)r * nv) * V + 1;
-            const R s = wave_vec_any<PP, RS>(P, src, i, j0, (R)inh, (R)inhv);
-            smax = (s > smax) ? s : smax;
-        }
-    } else {
-        const int64_t total = (int64_t)(P.own_hi - P.own_lo + 1) * P.ny;
-        const int si = (int)(stride / P.ny), sj = (int)(stride - (int64_t)si * P.ny);
-        int i = (int)(c0 / P.ny) + P.own_lo, j = (int)(c0 - (int64_t)(i - P.own_lo) * P.ny) + 1;
-        for (int64_t c = c0; c < total; c += stride) {
-            const R s = wave_cell<PP, RS>(P, src, i, j, (R)inh, (R)inhv, B.solid);
-            smax = (s > smax) ? s : smax;
-            i += si;
-            j += sj;
-            if (j > P.ny) { j -= P.ny; i++; }
-        }
-    }
+    const R smax = wave_rows<PP, RS, false>(P, src, (int64_t)blockIdx.x * blockDim.x + threadIdx.x,
+                                            (int64_t)gridDim.x * blockDim.x, (R)inh, (R)inhv, B.solid);
     const double m = block_max((double)smax, red8);
     if (threadIdx.x == 0) {
         atomicMax(&ctl->smax_bits, (unsigned long long)__double_as_longlong(m));
@@ -1223,7 +1248,7 @@ struct FailArgs {
     const double *z0;          /* set-up topography: a solid neighbour's slopes */
 };
 
-__device__ __forceinline__ double fa_slope_x(const FailArgs &A, const double *__restrict__ z, int i, int j)
+__device__ __forceinline__ double fa_slope_x(const FailArgs &A, const double *z, int i, int j)
 {
     const int64_t p = A.pitch;
     const int64_t q = (int64_t)(i - 1) * p + (j - 1);
@@ -1232,7 +1257,7 @@ __device__ __forceinline__ double fa_slope_x(const FailArgs &A, const double *__
     return A.oneoverdx * (z[q + p] - z[q]);
 }
 
-__device__ __forceinline__ double fa_slope_y(const FailArgs &A, const double *__restrict__ z, int i, int j)
+__device__ __forceinline__ double fa_slope_y(const FailArgs &A, const double *z, int i, int j)
 {
     const int64_t q = (int64_t)(i - 1) * A.pitch + (j - 1);
     if (j != 1 && j != A.ny) return A.half_odx * (z[q + 1] - z[q - 1]);
@@ -1243,8 +1268,8 @@ __device__ __forceinline__ double fa_slope_y(const FailArgs &A, const double *__
 /* Exact slope-failure test, SWEHR.c:1292-1312, in the form's arithmetic
  * (rarely needed: see the bound in tile_cell). */
 template <class PP, class RS>
-__device__ __noinline__ typename PP::R fail_exact(const FailArgs A, const RS *__restrict__ dep_plane,
-                                                  const double *__restrict__ zp, const double *__restrict__ zc,
+__device__ __noinline__ typename PP::R fail_exact(const FailArgs A, const RS *dep_plane,
+                                                  const double *zp, const double *zc,
                                                   int i, int j, typename PP::R sx, typename PP::R sy,
                                                   typename PP::R gz, typename PP::R dep0, typename PP::R rho0c,
                                                   typename PP::R h0v)
@@ -1297,7 +1322,7 @@ __device__ __forceinline__ typename PP::R storm_r(PP &pp, const DevParams &P, do
  * memory in every thread.) */
 template <class PP, class RS, int MAXS, bool BUDGET>
 __device__ __forceinline__ void solid_cell(const DevParams &P, const SetV<RS> &src, const SetV<RS> &dst,
-                                        const double *__restrict__ zc, double *__restrict__ zn, int64_t q,
+                                        const double *zc, double *zn, int64_t q,
                                         Acc2<MAXS, BUDGET> &acc)
 {
     const int64_t pl = P.plane;
@@ -1328,8 +1353,8 @@ __device__ __forceinline__ void solid_cell(const DevParams &P, const SetV<RS> &s
  * whose slots already hold new values). */
 template <class PP, class RS, int MAXS, bool BUDGET, int NS, bool FRESH>
 __device__ __forceinline__ void tile_cell_pp(PP &pp, const DevParams &P, const SetV<RS> &src, const SetV<RS> &dst,
-                                          const double *__restrict__ zp, const double *__restrict__ zc,
-                                          double *__restrict__ zn, const unsigned char *smb, const StagedLayout &L,
+                                          const double *zp, const double *zc,
+                                          double *zn, const unsigned char *smb, const StagedLayout &L,
                                           TileCoord tc, double t, double dt, double Rr, Acc2<MAXS, BUDGET> &acc,
                                           const uint8_t *__restrict__ solid, const double *__restrict__ z0)
 {
@@ -1520,7 +1545,7 @@ __device__ __forceinline__ void tile_cell_pp(PP &pp, const DevParams &P, const S
             uflux = (R)u_in - dtdx * (fxr0 * sk[uxr] - fxl0 * sk[uxl]) - dtdx * (fyr0 * sk[uyr] - fyl0 * sk[uyl]);
         else
             uflux = Ureg[kSlot ? 0 : k];
-        const double Mk0 = stage_m ? celld[(CD_M + k) * T_I * T_J + cs] : __ldg(src.M + qm);
+        const double Mk0 = stage_m ? celld[(CD_M + k) * T_I * T_J + cs] : __ldcg(src.M + qm);
         const R Mk0r = (R)Mk0;
         /* Rain-splash detachment of the original soil is the only source the
          * shallow branch uses; the other sources and the settling velocity
@@ -1711,8 +1736,8 @@ __device__ __noinline__ void tile_cell_again(const DevParams &P, const CellArgs<
  * to its sums as it goes, so it keeps the plain operators. */
 template <class PP, class RS, int MAXS, bool BUDGET, int NS = 0>
 __device__ __forceinline__ void tile_cell(const DevParams &P, const SetV<RS> &src, const SetV<RS> &dst,
-                                          const double *__restrict__ zp, const double *__restrict__ zc,
-                                          double *__restrict__ zn, const unsigned char *smb, const StagedLayout &L,
+                                          const double *zp, const double *zc,
+                                          double *zn, const unsigned char *smb, const StagedLayout &L,
                                           TileCoord tc, double t, double dt, double Rr, Acc2<MAXS, BUDGET> &acc,
                                           const uint8_t *__restrict__ solid, const double *__restrict__ z0)
 {
@@ -2029,6 +2054,132 @@ __global__ void __launch_bounds__(TILE_THREADS, PP::kMinBlocks) k_update_tile(co
     }
     if (threadIdx.x == 0) ctl->rain_now = Rr;
     update_finalize<PP, RS>(P, B.set[(n + 1) & 1], ctl, stage, saveflow, smb);
+}
+
+/* ------------------------------------------------------------- run ------
+ * Up to `steps` whole steps of one domain in one cooperative launch: wave
+ * pass, grid barrier, update pass, grid barrier, with the two kernels' per-cell
+ * arithmetic, so the results are the same bits.
+ *
+ * A small domain's step is latency: of the 28 us that the 200 x 50 hillslope's
+ * 50 tiles take as two kernels (FP64), a cell's chain of dependent operations
+ * is 13, staging, face states and faces 4, and launching, reading the control
+ * block, tickets and the last block's work 11.  Here the step state stays in
+ * shared memory and the two barriers take about 1.5 us each (see
+ * RUN_TILES_PER_SM for times).
+ *
+ * What one launch's blocks write and others read -- the state planes, the
+ * topography -- is read from L2 (ld.cg) or by the copy engine after a proxy
+ * fence on both sides of the barrier, never through the read-only path.  The
+ * barriers give up after a bounded number of polls (SWEHR_TIMEOUT). */
+#define RUN_MAX_POLLS (1u << 24)
+
+/* count: arrivals of all launches of this grid, a multiple of the grid size
+ * between launches; target: the count that ends this barrier.  The whole
+ * block calls it; `ok` is shared.  then() runs in thread 0 before the block
+ * goes on, and says whether it does. */
+template <class Then>
+__device__ __forceinline__ bool grid_barrier(Ctl *ctl, unsigned long long target, bool *ok, Then then)
+{
+    fence_proxy_async();                 /* this thread's stores before any block's tile copies */
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        atomicAdd(&ctl->run_count, 1ull);
+        bool done = false;
+        for (uint32_t k = 0; k < RUN_MAX_POLLS && !done; k++) {
+            unsigned long long v;
+            asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(&ctl->run_count) : "memory");
+            done = v >= target;
+        }
+        __threadfence();
+        if (!done) {
+            ctl->dev_error = 1;
+            ctl->status = 3;
+            ctl->active = 0;
+        } else
+            done = then();
+        *ok = done;
+    }
+    __syncthreads();
+    fence_proxy_async();
+    return *ok;
+}
+
+template <class PP, class RS, int MAXS, bool STAGE_M, int NS>
+__global__ void __launch_bounds__(TILE_THREADS, PP::kMinBlocks)
+k_run_tile(const __grid_constant__ DevParams P, const __grid_constant__ BufsT<RS> B, Ctl *ctl,
+           const double *__restrict__ rain, double *stage, double *saveflow, const __grid_constant__ TmaMaps tm,
+           int steps)
+{
+    typedef typename PP::R R;
+    if (!ctl->active) return;            /* written only after this launch's first barrier */
+    extern __shared__ __align__(128) unsigned char smb_raw[];
+    unsigned char *smb = smb_raw + ((128u - (smem_addr(smb_raw) & 127u)) & 127u);
+    __shared__ double red8[TILE_THREADS / 32];
+    __shared__ __align__(8) uint64_t tma_bar;
+    __shared__ bool ok;
+    __shared__ StepSize size;
+    __shared__ double rate;
+    uint32_t tma_phase = 0;
+    if (threadIdx.x == 0) {
+        mbar_init(&tma_bar, 1);
+        mbar_init_fence();
+    }
+    __syncthreads();
+    const StagedLayout L = StagedLayout::make(P.S, sizeof(R), STAGE_M);
+    int64_t n = ctl->step;
+    double t = ctl->t;
+    const double t_stop = ctl->t_stop;
+    const int64_t max_step = ctl->max_step;
+    const unsigned grid = gridDim.x;
+    /* fewer than `grid` arrivals of this launch can have come before this read */
+    unsigned long long target = *(volatile unsigned long long *)&ctl->run_count / grid * grid;
+    const int64_t ntiles = (int64_t)((P.own_hi - P.own_lo + T_I) / T_I) * ((P.ny + T_J - 1) / T_J);
+    for (int k = 0; k < steps; k++) {
+        double inh = 0, inhv = 0, insed = 0;
+        if (P.inflow) inflow_ghost(t, inh, inhv, insed);
+        const R smax = wave_rows<PP, RS, true>(P, B.set[n & 1], (int64_t)blockIdx.x * TILE_THREADS + threadIdx.x,
+                                               (int64_t)grid * TILE_THREADS, (R)inh, (R)inhv, B.solid);
+        const double m = block_max((double)smax, red8);
+        unsigned long long *slot = &ctl->run_smax[n & 1];
+        if (threadIdx.x == 0) atomicMax(slot, (unsigned long long)__double_as_longlong(m));
+        target += grid;
+        const bool go = grid_barrier(ctl, target, &ok, [&] {
+            size = step_size(P, t, __longlong_as_double((long long)__ldcg(slot)));
+            rate = P.storm ? 0.0 : rain_at(P, rain, t);
+            return __ldcg(&ctl->dev_error) == 0;      /* a tile load of the last step gave up: no further step */
+        });
+        if (!go) return;
+        const double dt = size.dt, Rr = rate;
+        const bool cfl = size.courant > 1;
+        Acc2<MAXS, false> none;
+        for (int64_t tile = blockIdx.x; tile < ntiles; tile += grid)
+            update_tile<PP, RS, MAXS, false, true, NS>(P, B, n, t, dt, Rr, tile_coord(P, tile), smb, L, none, &tm,
+                                                       &tma_bar, &tma_phase, ctl);
+        target += grid;
+        if (!grid_barrier(ctl, target, &ok, [] { return true; })) return;
+        const double courant = size.courant;
+        if (blockIdx.x == 0) {
+            /* the step's end, while the other blocks begin the next wave pass:
+             * it only reads the state they read, and its own fields */
+            if (threadIdx.x == 0) {
+                *slot = 0ull;
+                ctl->dt = dt;
+                ctl->courant = courant;
+                ctl->cfl = cfl;
+                ctl->rain_now = Rr;
+            }
+            __syncthreads();
+            update_finalize<PP, RS>(P, B.set[(n + 1) & 1], ctl, stage, saveflow, smb);
+            __syncthreads();
+        }
+        /* what update_finalize has just stored, in every block */
+        const double tnew = (cfl ? 2 * P.tend : t) + dt;
+        n++;
+        t = tnew;
+        if (cfl || !(dt > 0) || !(tnew < P.tend) || !(tnew < t_stop) || n >= max_step) return;
+    }
 }
 
 /* ------------------------------------------------------------- batched ---

@@ -78,6 +78,9 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity)
 /* order this CTA's earlier shared-memory accesses before copies that write it */
 __device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
+/* order this thread's accesses to any memory and those of the copy engine */
+__device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async;" ::: "memory"); }
+
 /* box (x, y, z) of a 3-D tensor map into shared memory (x is the
  * contiguous coordinate and must be a multiple of 16 bytes) */
 __device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, uint64_t *bar, int x, int y, int z)
