@@ -718,33 +718,46 @@ struct SetPlanes<float> {
 };
 
 /* The same staging as stage_load as tensor-map box copies (planes of one
- * domain), issued by one thread onto the tile's mbarrier: halo boxes of
+ * domain), onto two mbarriers, each announced and issued by one thread of a
+ * warp of its own: the halo planes that the face states are formed from, and
+ * the rest, which is waited for only before the cells.  Halo boxes of
  * Cols<RS>::rj columns x halo rows at column j0-1-pad, row i0-2 (0-based),
  * the z_prev window of the tile's rows (doubles, column j0-3), cell
  * boxes T_J x T_I at (j0-1, i0-1).  j0-1 is a multiple of T_J and pad is 16
  * bytes of the plane's type, so every box starts on a 16-byte column
  * boundary; rows or columns outside the grid arrive as zeros. */
 template <class RS>
-__device__ __forceinline__ void stage_load_tma(const DevParams &P, const TmaMaps &tm, int set, int64_t n,
-                                               TileCoord tc, unsigned char *smb, const StagedLayout &L,
-                                               uint64_t *bar)
+__device__ __forceinline__ void stage_halo_tma(const DevParams &P, const TmaMaps &tm, int set, TileCoord tc,
+                                               unsigned char *smb, const StagedLayout &L, uint64_t *bar)
 {
     typedef SetPlanes<RS> SP;
-    const uint32_t hb = (uint32_t)(HALO_ROWS * Cols<RS>::rj * sizeof(RS));
-    const uint32_t cbr = (uint32_t)(T_I * T_J * sizeof(RS)), cbd = (uint32_t)(T_I * T_J * sizeof(double));
-    const uint32_t bytes = (uint32_t)(HP_U + P.S) * hb + (uint32_t)((ZP_ROWS + ZC_ROWS) * R_J * sizeof(double)) +
-                           (3u + (P.has_ks ? 1u : 0u)) * cbr + (1u + (L.stage_m ? (uint32_t)P.S : 0u)) * cbd;
-    mbar_expect_tx(bar, bytes);
-    const CUtensorMap *mh = &tm.m[TM_HALO0 + set], *mc = &tm.m[TM_CELL0 + set], *md = &tm.m[TM_CELLD0 + set];
-    const int hx = tc.j0 - 1 - Cols<RS>::pad, hy = tc.i0 - 2, zx = tc.j0 - 3, cx = tc.j0 - 1, cy = tc.i0 - 1;
+    mbar_expect_tx(bar, (4u + (uint32_t)P.S) * (uint32_t)(HALO_ROWS * Cols<RS>::rj * sizeof(RS)));
+    const CUtensorMap *mh = &tm.m[TM_HALO0 + set];
+    const int hx = tc.j0 - 1 - Cols<RS>::pad, hy = tc.i0 - 2;
     RS *halo = reinterpret_cast<RS *>(smb + L.halo);
     tma_load_3d(halo + HP_H * L.hps, mh, bar, hx, hy, SP::h);
     tma_load_3d(halo + HP_HU * L.hps, mh, bar, hx, hy, SP::hu);
     tma_load_3d(halo + HP_HV * L.hps, mh, bar, hx, hy, SP::hv);
-    tma_load_3d(halo + HP_TS * L.hps, mh, bar, hx, hy, SP::totsed);
-    tma_load_3d(halo + HP_DEP * L.hps, mh, bar, hx, hy, SP::dep);
     tma_load_3d(halo + HP_GZ * L.hps, mh, bar, hx, hy, SP::gz);
     for (int k = 0; k < P.S; k++) tma_load_3d(halo + (HP_U + k) * L.hps, mh, bar, hx, hy, SP::U + k);
+}
+
+/* the rest, which only the cells need: TOTSED and DEP with their halo, the
+ * topography windows and the cell planes */
+template <class RS>
+__device__ __forceinline__ void stage_cell_tma(const DevParams &P, const TmaMaps &tm, int set, int64_t n, TileCoord tc,
+                                               unsigned char *smb, const StagedLayout &L, uint64_t *bar)
+{
+    typedef SetPlanes<RS> SP;
+    const uint32_t cbr = (uint32_t)(T_I * T_J * sizeof(RS)), cbd = (uint32_t)(T_I * T_J * sizeof(double));
+    mbar_expect_tx(bar, 2u * (uint32_t)(HALO_ROWS * Cols<RS>::rj * sizeof(RS)) +
+                            (uint32_t)((ZP_ROWS + ZC_ROWS) * R_J * sizeof(double)) + (3u + (P.has_ks ? 1u : 0u)) * cbr +
+                            (1u + (L.stage_m ? (uint32_t)P.S : 0u)) * cbd);
+    const CUtensorMap *mc = &tm.m[TM_CELL0 + set], *md = &tm.m[TM_CELLD0 + set];
+    const int hx = tc.j0 - 1 - Cols<RS>::pad, hy = tc.i0 - 2, zx = tc.j0 - 3, cx = tc.j0 - 1, cy = tc.i0 - 1;
+    RS *halo = reinterpret_cast<RS *>(smb + L.halo);
+    tma_load_3d(halo + HP_TS * L.hps, &tm.m[TM_HALO0 + set], bar, hx, hy, SP::totsed);
+    tma_load_3d(halo + HP_DEP * L.hps, &tm.m[TM_HALO0 + set], bar, hx, hy, SP::dep);
     tma_load_3d(smb + L.zp, &tm.m[TM_ZP], bar, zx, cy, (int)((n + 2) % 3));
     tma_load_3d(smb + L.zc, &tm.m[TM_ZC], bar, zx, hy, (int)(n % 3));
     RS *cr = reinterpret_cast<RS *>(smb + L.cell_r);
@@ -1847,12 +1860,14 @@ __device__ __forceinline__ void update_tile(const DevParams &P, const BufsT<RS> 
          * (the barrier ending it); order them before the copies that land */
         if (threadIdx.x == 0) {
             fence_proxy_async_smem();
-            stage_load_tma<RS>(P, *tm, (int)(n & 1), n, tc, smb, L, bar);
+            stage_halo_tma<RS>(P, *tm, (int)(n & 1), tc, smb, L, bar);
+        } else if (threadIdx.x == 32) {
+            fence_proxy_async_smem();
+            stage_cell_tma<RS>(P, *tm, (int)(n & 1), n, tc, smb, L, bar + 1);
         }
         /* one warp polls, the others wait at the block's barrier: eight polling
          * warps take issue slots from the SM's other blocks */
         if (threadIdx.x < 32 && !mbar_wait_bounded(bar, *phase & 1u) && threadIdx.x == 0) ctl->dev_error = 1;
-        *phase += 1;
         __syncthreads();
     } else {
         stage_load<RS, NS>(P, src, zp, zc, B.ks, tc, smb, L);
@@ -1913,6 +1928,10 @@ __device__ __forceinline__ void update_tile(const DevParams &P, const BufsT<RS> 
         face[1] = yface ? T2 : T1;
         face[2] = yface ? T1 : T2;
         upb[f] = (T0 > 0) ? 0 : 1;
+    }
+    if constexpr (TMA) {
+        if (threadIdx.x < 32 && !mbar_wait_bounded(bar + 1, *phase & 1u) && threadIdx.x == 0) ctl->dev_error = 1;
+        *phase += 1;
     }
     __syncthreads();
     tile_cell<PP, RS, MAXS, BUDGET, NS>(P, src, dst, zp, zc, zn, smb, L, tc, t, dt, Rr, acc, B.solid, B.z0);
@@ -2014,11 +2033,12 @@ __global__ void __launch_bounds__(TILE_THREADS, PP::kMinBlocks) k_update_tile(co
      * with the polling below: FP64 update 4.24 -> 4.04 ms, mixed 2.24 -> 2.12) */
     unsigned char *smb = smb_raw + (TMA ? (128u - (smem_addr(smb_raw) & 127u)) & 127u : 0u);
     __shared__ bool last;
-    __shared__ __align__(8) uint64_t tma_bar;
+    __shared__ __align__(8) uint64_t tma_bar[2];
     uint32_t tma_phase = 0;
     if constexpr (TMA) {
         if (threadIdx.x == 0) {
-            mbar_init(&tma_bar, 1);
+            mbar_init(&tma_bar[0], 1);
+            mbar_init(&tma_bar[1], 1);
             mbar_init_fence();
         }
         __syncthreads();
@@ -2031,7 +2051,7 @@ __global__ void __launch_bounds__(TILE_THREADS, PP::kMinBlocks) k_update_tile(co
     acc_zero(acc);
     const int64_t ntiles = (int64_t)((P.own_hi - P.own_lo + T_I) / T_I) * ((P.ny + T_J - 1) / T_J);
     for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x)
-        update_tile<PP, RS, MAXS, BUDGET, TMA, NS>(P, B, n, t, dt, Rr, tile_coord(P, tile), smb, L, acc, &tm, &tma_bar,
+        update_tile<PP, RS, MAXS, BUDGET, TMA, NS>(P, B, n, t, dt, Rr, tile_coord(P, tile), smb, L, acc, &tm, tma_bar,
                                                &tma_phase, ctl);
     double *red = reinterpret_cast<double *>(smb + L.red);
     if (BUDGET) budget_block_sum(acc, red);
@@ -2117,13 +2137,14 @@ k_run_tile(const __grid_constant__ DevParams P, const __grid_constant__ BufsT<RS
     extern __shared__ __align__(128) unsigned char smb_raw[];
     unsigned char *smb = smb_raw + ((128u - (smem_addr(smb_raw) & 127u)) & 127u);
     __shared__ double red8[TILE_THREADS / 32];
-    __shared__ __align__(8) uint64_t tma_bar;
+    __shared__ __align__(8) uint64_t tma_bar[2];
     __shared__ bool ok;
     __shared__ StepSize size;
     __shared__ double rate;
     uint32_t tma_phase = 0;
     if (threadIdx.x == 0) {
-        mbar_init(&tma_bar, 1);
+        mbar_init(&tma_bar[0], 1);
+            mbar_init(&tma_bar[1], 1);
         mbar_init_fence();
     }
     __syncthreads();
@@ -2156,7 +2177,7 @@ k_run_tile(const __grid_constant__ DevParams P, const __grid_constant__ BufsT<RS
         Acc2<MAXS, false> none;
         for (int64_t tile = blockIdx.x; tile < ntiles; tile += grid)
             update_tile<PP, RS, MAXS, false, true, NS>(P, B, n, t, dt, Rr, tile_coord(P, tile), smb, L, none, &tm,
-                                                       &tma_bar, &tma_phase, ctl);
+                                                       tma_bar, &tma_phase, ctl);
         target += grid;
         if (!grid_barrier(ctl, target, &ok, [] { return true; })) return;
         const double courant = size.courant;
