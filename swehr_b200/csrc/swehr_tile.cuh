@@ -86,6 +86,8 @@ struct PolicyF64 {
     static __device__ __forceinline__ R quotz(R a, R b) { return divz(a, b); }
     static __device__ __forceinline__ R quotn(R a, R b) { return divz(a, b); }
     static __device__ __forceinline__ R root1(R x) { return sw_sqrt_pow(x); }
+    static __device__ __forceinline__ R quot_in(R a, R b) { return a / b; }
+    static __device__ __forceinline__ R divk_in(R a, R c, R yc, int ok) { return divk(a, c, yc, ok); }
     /* wave pass: two cells per thread (16-byte loads) at 3 CTAs per SM (80
      * registers); measured against one cell per thread at 5 CTAs: wet steps
      * -0.06 ms, early steps +0.03 ms per 4096^2 step */
@@ -174,7 +176,7 @@ struct PolicyF64 {
  * PolicyF64 from the branch-free sequences of swehr_ieee.h, so that the
  * compiler interleaves a cell's independent quotients, roots and exponentials
  * and quotients by one divisor share its reciprocal.  ok is cleared by an
- * operand outside [2^-500, 2^501) that is not a zero dividend or radicand, a
+ * operand outside [2^-300, 2^301) that is not a zero dividend or radicand, a
  * divisor that is not positive, an exponent beyond 700 or a NaN; the caller
  * then computes again with PolicyF64.  Constants need no test here:
  * DevParams::fast_ok says that the run's are in range (ok starts as it). */
@@ -211,6 +213,14 @@ struct FastF64 {
     {
         ok &= sw_mid_or_zero(a);
         return sw_quot(a, c, yc);
+    }
+    /* a dividend that is in range with what has been tested: a quotient of
+     * tested operands, a difference of settling velocities */
+    static __device__ __forceinline__ R divk_in(R a, R c, R yc, int) { return sw_quot(a, c, yc); }
+    __device__ __forceinline__ R quot_in(R a, const Recip &r)
+    {
+        ok &= sw_mid_pos(r.b);
+        return sw_quot(a, r.b, r.y);
     }
     __device__ __forceinline__ R sqrtp(R x)
     {
@@ -250,7 +260,6 @@ struct FastF64 {
      * quotient's sign without the quotient */
     __device__ __forceinline__ R e3_term(R num, R J, R yJ, int, R m)
     {
-        ok &= sw_small(num);
         if (m == 0)
             return PolicyF64::zero_xor(__double_as_longlong(num) ^ __double_as_longlong(m));
         return divk(num, J, yJ, 1) * m;
@@ -365,6 +374,8 @@ struct PolicyF32 {
     static __device__ __forceinline__ R divz(R a, R b) { return div(a, b); }
     static __device__ __forceinline__ R sqrtz(R x) { return sqrtp(x); }
     static __device__ __forceinline__ R divk(R a, R c, R, int) { return div(a, c); }
+    static __device__ __forceinline__ R divk_in(R a, R c, R, int) { return div(a, c); }
+    static __device__ __forceinline__ R quot_in(R a, R y) { return quot(a, y); }
     static __device__ __forceinline__ R e3_term(R num, R J, R yJ, int ok, R m) { return divk(num, J, yJ, ok) * m; }
     static __device__ __forceinline__ R e4_term(R A, R T, R F, R e, R m) { return quot(quot(A, T) * F, e) * m; }
     static __device__ __forceinline__ R qnan() { return __int_as_float(0x7fc00000); }
@@ -1590,13 +1601,13 @@ __device__ __forceinline__ void tile_cell_pp(PP &pp, const DevParams &P, const S
                 VF = pp.settle(K.a13[k], K.a13sq[k], K.c109s * gz * K.ds[k]);
                 VF = VF * vfconc;
                 if (K.ds[k] > R(0.0001) && h0v < K.h0x9)
-                    VF = R(2e-3) + pp.divk(fmax(h0v - K.h0x3, R(0)) * (VF - R(2e-3)), K.h0x6, (R)P.inv_h0x6, P.divk_ok);
+                    VF = R(2e-3) + pp.divk_in(fmax(h0v - K.h0x3, R(0)) * (VF - R(2e-3)), K.h0x6, (R)P.inv_h0x6, P.divk_ok);
                 if (K.ds[k] > R(0.002) && h0v < K.h0x9)
-                    VF = R(2e-3) + pp.divk(fmax(h0v - K.h0x3, R(0)) * (VF - R(2e-3)), K.h0x6, (R)P.inv_h0x6, P.divk_ok);
+                    VF = R(2e-3) + pp.divk_in(fmax(h0v - K.h0x3, R(0)) * (VF - R(2e-3)), K.h0x6, (R)P.inv_h0x6, P.divk_ok);
             }
             chtemp = u;
             const R redetach = fmin(Mk0r, dtr * (E2 + E4));
-            const R dec = pp.exp(pp.div(-VF, h) * (half * dtr));
+            const R dec = pp.exp(pp.quot_in(-VF, PP::recip(h)) * (half * dtr));
             u = dec * u;
             u = u + dtr * (E1 + E3) + redetach;
             u = dec * u;
@@ -1643,7 +1654,7 @@ __device__ __forceinline__ void tile_cell_pp(PP &pp, const DevParams &P, const S
         for (int k = 0; k < MAXS; k++) {
             if (k >= S) break;
             const R uk = kSlot ? (R)Uslot[k * hps] : Ureg[kSlot ? 0 : k];
-            totsed += pp.divk(pp.quotz(uk, rh), rhos, (R)P.inv_rhos, P.divk_ok);
+            totsed += pp.divk_in(pp.quotz(uk, rh), rhos, (R)P.inv_rhos, P.divk_ok);
             dst.U[k * pl + q] = (RS)uk;
             if (stage_m) dst.M[k * pl + q] = celld[(CD_M + k) * T_I * T_J + cs];
         }
