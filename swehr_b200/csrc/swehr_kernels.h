@@ -56,24 +56,29 @@ struct BatchHdr {
     unsigned long long *grab;
 };
 
-/* the batched kernels of one form (both take one argument: the header) */
+/* the batched kernels of one form (the wave pass takes the header, the update
+ * the header and the common constants) */
 struct BatchConfig {
-    void *fn_wave = nullptr, *fn_update = nullptr;
-    size_t smem_wave = 0, smem_update = 0;
-    int occ_wave = 1, occ_update = 1;   /* resident blocks per SM */
+    void *fn_wave = nullptr;
+    size_t smem_wave = 0;
+    int occ_wave = 1;                   /* resident blocks per SM */
     int threads = 0;                    /* threads per block */
     int tile_i = 0, tile_j = 0;         /* cells per tile */
-    /* update kernel: dynamic shared memory and resident blocks per SM when
-     * the largest class count among the scenarios is S (index S = 0..16) */
-    size_t smem_update_s[17] = {};
-    int occ_update_s[17] = {};
-    int stage_m_s[17] = {};             /* stage M_k in shared memory at this class count */
-    void *fn_update_s[17] = {};         /* the update kernel for that choice */
-    /* kernels built for exactly S classes (S = 7, 10; null elsewhere), used
-     * when every running scenario has S classes */
-    void *fn_update_x[17] = {};
-    size_t smem_update_x[17] = {};
-    int occ_update_x[17] = {};
+    /* update kernels with each scenario's own constants, and with common ones
+     * (pools without budgets) */
+    struct Update {
+        /* dynamic shared memory and resident blocks per SM when the largest
+         * class count among the scenarios is S (index S = 0..16) */
+        void *fn_s[17] = {};
+        size_t smem_s[17] = {};
+        int occ_s[17] = {};
+        /* kernels built for exactly S classes (S = 7, 10; null elsewhere), used
+         * when every running scenario has S classes */
+        void *fn_x[17] = {};
+        size_t smem_x[17] = {};
+        int occ_x[17] = {};
+    };
+    Update own, common;
 };
 
 int configure_batch_f64(int max_classes, bool budget, BatchConfig &cfg);

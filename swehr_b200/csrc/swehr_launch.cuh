@@ -234,61 +234,76 @@ struct FormLauncher {
         return 0;
     }
 
-    template <int MAXS, bool BUDGET, bool SM, int NS = 0>
-    static void *ubatch_fn() { return (void *)k_update_batch<PP, RS, MAXS, BUDGET, SM, NS>; }
+    template <int MAXS, bool BUDGET, bool SM, int NS, bool COMMON>
+    static void *ubatch_fn() { return (void *)k_update_batch<PP, RS, MAXS, BUDGET, SM, NS, COMMON>; }
 
-    /* batched kernels for exactly NS classes (every running scenario has NS) */
-    template <int MAXS, int NS>
-    static cudaError_t exact_batch(bool budget, BatchConfig &cfg)
+    /* batched kernel for exactly NS classes (every running scenario has NS):
+     * M_k staged where that leaves the resident blocks the kernel is
+     * register-budgeted for */
+    template <int MAXS, int NS, bool COMMON>
+    static cudaError_t exact_batch(bool budget, BatchConfig::Update &u)
     {
-        void *fw = budget ? ubatch_fn<MAXS, true, true, NS>() : ubatch_fn<MAXS, false, true, NS>();
-        void *fo = budget ? ubatch_fn<MAXS, true, false, NS>() : ubatch_fn<MAXS, false, false, NS>();
-        int sm = 1;
-        return pick_staging(fw, fo, NS, cfg.smem_update_x[NS], cfg.occ_update_x[NS], sm, cfg.fn_update_x[NS]);
+        constexpr int blocks = COMMON ? PP::kCommonMinBlocks : PP::kBatchMinBlocks;
+        constexpr bool sm = NS == 7 || (NS == 10 && sizeof(RS) == 4 && blocks == 2);
+        void *f = ubatch_fn<MAXS, false, sm, NS, COMMON>();
+        if constexpr (!COMMON)
+            if (budget) f = ubatch_fn<MAXS, true, sm, NS, COMMON>();
+        u.smem_x[NS] = update_smem(NS, sm);
+        cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)u.smem_x[NS]);
+        if (e == cudaSuccess)
+            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&u.occ_x[NS], f, TILE_THREADS, u.smem_x[NS]);
+        if (u.occ_x[NS] < 1) u.occ_x[NS] = 1;
+        u.fn_x[NS] = f;
+        return e;
     }
 
-    template <bool SM>
+    template <bool SM, bool COMMON>
     static void *pick_ub(int max_classes, bool budget)
     {
-        if (max_classes <= 4) return budget ? ubatch_fn<4, true, SM>() : ubatch_fn<4, false, SM>();
-        if (max_classes <= 8) return budget ? ubatch_fn<8, true, SM>() : ubatch_fn<8, false, SM>();
-        return budget ? ubatch_fn<16, true, SM>() : ubatch_fn<16, false, SM>();
+        if constexpr (!COMMON)
+            if (budget) {
+                if (max_classes <= 4) return ubatch_fn<4, true, SM, 0, false>();
+                if (max_classes <= 8) return ubatch_fn<8, true, SM, 0, false>();
+                return ubatch_fn<16, true, SM, 0, false>();
+            }
+        if (max_classes <= 4) return ubatch_fn<4, false, SM, 0, COMMON>();
+        if (max_classes <= 8) return ubatch_fn<8, false, SM, 0, COMMON>();
+        return ubatch_fn<16, false, SM, 0, COMMON>();
+    }
+
+    template <bool COMMON>
+    static cudaError_t configure_updates(int max_classes, bool budget, BatchConfig::Update &u)
+    {
+        void *with = pick_ub<true, COMMON>(max_classes, budget), *without = pick_ub<false, COMMON>(max_classes, budget);
+        cudaError_t e = cudaSuccess;
+        for (int S = 0; S <= 16 && e == cudaSuccess; S++) {
+            const int Sc = S < 1 ? 1 : (S > max_classes ? max_classes : S);
+            int stage_m = 1;
+            e = pick_staging(with, without, Sc, u.smem_s[S], u.occ_s[S], stage_m, u.fn_s[S]);
+        }
+        if (e == cudaSuccess && max_classes >= 7) e = exact_batch<8, 7, COMMON>(budget, u);
+        if (e == cudaSuccess && max_classes >= 10) e = exact_batch<16, 10, COMMON>(budget, u);
+        /* limits for the largest shape either kernel is launched with */
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(with, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)update_smem(max_classes));
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(without, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)update_smem(max_classes, 0));
+        return e;
     }
 
     static int configure_batch(int max_classes, bool budget, BatchConfig &cfg)
     {
-        void *fu_with = pick_ub<true>(max_classes, budget), *fu_without = pick_ub<false>(max_classes, budget);
         void *fw = (void *)k_wave_batch<PP, RS>;
-        const size_t su = update_smem(max_classes), sw = wave_smem();
+        const size_t sw = wave_smem();
         cudaError_t e = cudaFuncSetAttribute(fw, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sw);
         if (e != cudaSuccess) return (int)e;
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&cfg.occ_wave, fw, TILE_THREADS, sw);
         if (e != cudaSuccess) return (int)e;
         if (cfg.occ_wave < 1) cfg.occ_wave = 1;
-        cfg.occ_update = 1;
-        for (int S = 0; S <= 16; S++) {
-            const int Sc = S < 1 ? 1 : (S > max_classes ? max_classes : S);
-            e = pick_staging(fu_with, fu_without, Sc, cfg.smem_update_s[S], cfg.occ_update_s[S], cfg.stage_m_s[S],
-                             cfg.fn_update_s[S]);
-            if (e != cudaSuccess) return (int)e;
-            if (cfg.occ_update_s[S] > cfg.occ_update) cfg.occ_update = cfg.occ_update_s[S];
-        }
-        if (max_classes >= 7) {
-            e = exact_batch<8, 7>(budget, cfg);
-            if (e != cudaSuccess) return (int)e;
-        }
-        if (max_classes >= 10) {
-            e = exact_batch<16, 10>(budget, cfg);
-            if (e != cudaSuccess) return (int)e;
-        }
-        /* limits for the largest shape either kernel is launched with */
-        e = cudaFuncSetAttribute(fu_with, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)su);
+        e = configure_updates<false>(max_classes, budget, cfg.own);
+        if (e == cudaSuccess && !budget) e = configure_updates<true>(max_classes, budget, cfg.common);
         if (e != cudaSuccess) return (int)e;
-        e = cudaFuncSetAttribute(fu_without, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)update_smem(max_classes, 0));
-        if (e != cudaSuccess) return (int)e;
-        cfg.fn_update = cfg.fn_update_s[max_classes];
         cfg.fn_wave = fw;
-        cfg.smem_update = su;
         cfg.smem_wave = sw;
         cfg.threads = TILE_THREADS;
         cfg.tile_i = T_I;

@@ -61,11 +61,17 @@ struct swehr_pool {
     int min_s = 1;                       /* smallest class count running */
     size_t smem_update = 0;              /* update kernel's dynamic shared memory now */
     void *fn_update = nullptr;           /* update kernel now (staging choice for max_s) */
+    /* the constants all running scenarios share, when they share them (the
+     * update kernel's parameter), and the number of the set: graphs hold it */
+    DevParams common = {};
+    bool has_common = false;
+    int common_id = 0;
     cudaStream_t stream = nullptr;
     struct GraphEntry {
         size_t smem;
         int gw, gu;
         void *fn;
+        int common_id;                   /* 0: the scenarios' own constants */
         cudaGraphExec_t exec;
     };
     std::vector<GraphEntry> graphs;      /* one per launch shape seen (class count x grids) */
@@ -203,13 +209,50 @@ static void fill_desc(const PoolScen &s, const BufsT<RS> &B, ScenSummary *d_sum,
 
 static void apply_shape(swehr_pool *pl);
 
+/* the constants a batch's update kernel can take from its parameter (see
+ * k_update_batch): a scenario's parameters without its own grid, rain, storm,
+ * output, roughness and class data */
+static DevParams common_constants(const DevParams &P)
+{
+    DevParams c = P;
+    c.nx = c.ny = c.S = c.pitch = c.rnum = c.inflow = c.storm = c.budget = 0;
+    memset(c.bndry, 0, sizeof c.bndry);
+    c.outlet_row = c.npoints = 0;
+    memset(c.xpoint, 0, sizeof c.xpoint);
+    memset(c.ypoint, 0, sizeof c.ypoint);
+    c.has_ks = c.has_solid = c.own_lo = c.own_hi = c.row0 = c.slab = 0;
+    c.plane = 0;
+    c.dx = c.oneoverdx = c.half_odx = c.tend = c.rint = c.stageint = 0;
+    c.nu = c.roughness = c.ks = c.cstable = c.maxstep = 0;
+    c.storm_peak = c.storm_r2 = c.storm_x0 = c.storm_y0 = c.storm_vx = c.storm_vy = 0;
+    auto classes = [](auto &k) {
+        memset(k.ds, 0, sizeof k.ds);
+        memset(k.pf, 0, sizeof k.pf);
+        memset(k.a13, 0, sizeof k.a13);
+        memset(k.a13sq, 0, sizeof k.a13sq);
+    };
+    classes(c);
+    classes(c.kd);
+    classes(c.kf);
+    c.kd.oneoverdx = c.kd.half_odx = c.kd.roughness = 0;
+    c.kf.oneoverdx = c.kf.half_odx = c.kf.roughness = 0;
+    return c;
+}
+
 /* write the running scenarios into the device table and header */
 static int rebuild_table(swehr_pool *pl)
 {
     int k = 0, max_s = 1, min_s = 16;
     int64_t tile0 = 0, cells = 0;
+    DevParams first;
+    bool same = pl->budget == 0;
     for (auto &s : pl->scen) {
         if (!s.running) continue;
+        if (k == 0) first = common_constants(s.ctx->P);
+        else if (same) {
+            const DevParams c = common_constants(s.ctx->P);
+            same = memcmp(&c, &first, sizeof c) == 0;
+        }
         max_s = std::max(max_s, (int)s.ctx->P.S);
         min_s = std::min(min_s, (int)s.ctx->P.S);
         s.ntiles = tiles_of(s.ctx->P, pl->cfg);     /* in the tile shape in use */
@@ -264,6 +307,19 @@ static int rebuild_table(swehr_pool *pl)
     pl->running_cells = cells;
     pl->max_s = max_s;
     pl->min_s = std::min(min_s, max_s);
+    pl->has_common = same && k > 0;
+    if (pl->has_common && (pl->common_id == 0 || memcmp(&first, &pl->common, sizeof first) != 0)) {
+        /* other constants than the graphs hold: those are never launched again */
+        for (auto it = pl->graphs.begin(); it != pl->graphs.end();) {
+            if (it->common_id) {
+                cudaGraphExecDestroy(it->exec);
+                it = pl->graphs.erase(it);
+            } else
+                ++it;
+        }
+        pl->common = first;
+        pl->common_id++;
+    }
     pl->dirty = false;
     apply_shape(pl);
     return SWEHR_OK;
@@ -271,7 +327,7 @@ static int rebuild_table(swehr_pool *pl)
 
 static void launch_pool_step(swehr_pool *pl, cudaEvent_t e0, cudaEvent_t e1, cudaEvent_t e2)
 {
-    void *args[] = {(void *)&pl->d_hdr};
+    void *args[] = {(void *)&pl->d_hdr, (void *)&pl->common};
     if (e0) cudaEventRecord(e0, pl->stream);
     cudaLaunchKernel(pl->cfg.fn_wave, dim3(pl->grid_wave), dim3(pl->cfg.threads), args, pl->cfg.smem_wave, pl->stream);
     if (e1) cudaEventRecord(e1, pl->stream);
@@ -286,7 +342,8 @@ static void launch_pool_step(swehr_pool *pl, cudaEvent_t e0, cudaEvent_t e1, cud
 static int pool_graph(swehr_pool *pl, cudaGraphExec_t *out)
 {
     for (auto &g : pl->graphs)
-        if (g.smem == pl->smem_update && g.gw == pl->grid_wave && g.gu == pl->grid_update && g.fn == pl->fn_update) {
+        if (g.smem == pl->smem_update && g.gw == pl->grid_wave && g.gu == pl->grid_update && g.fn == pl->fn_update &&
+            g.common_id == (pl->has_common ? pl->common_id : 0)) {
             *out = g.exec;
             return SWEHR_OK;
         }
@@ -298,7 +355,8 @@ static int pool_graph(swehr_pool *pl, cudaGraphExec_t *out)
     cudaError_t e = cudaGraphInstantiate(&ex, g, 0);
     cudaGraphDestroy(g);
     if (e != cudaSuccess) return swehr_err(SWEHR_CUDA_ERROR, std::string("cudaGraphInstantiate: ") + cudaGetErrorString(e));
-    pl->graphs.push_back({pl->smem_update, pl->grid_wave, pl->grid_update, pl->fn_update, ex});
+    pl->graphs.push_back({pl->smem_update, pl->grid_wave, pl->grid_update, pl->fn_update,
+                          pl->has_common ? pl->common_id : 0, ex});
     *out = ex;
     return SWEHR_OK;
 }
@@ -313,24 +371,31 @@ static void set_grids(swehr_pool *pl, int kw, int ku)
  * kernel's staging is sized by the largest class count present, so a pool
  * that admits up to 16 classes still runs 7-class batches at the 7-class
  * occupancy */
+static const BatchConfig::Update &updates(const swehr_pool *pl, const BatchConfig &c)
+{
+    return pl->has_common ? c.common : c.own;
+}
+
 /* the running scenarios all have the class count of a kernel built for
  * exactly that many classes */
-static bool exact_classes(const swehr_pool *pl, const BatchConfig &c)
+static bool exact_classes(const swehr_pool *pl, const BatchConfig::Update &u)
 {
-    return pl->min_s == pl->max_s && c.fn_update_x[pl->max_s] != nullptr;
+    return pl->min_s == pl->max_s && u.fn_x[pl->max_s] != nullptr;
 }
 
 static int update_occupancy(const swehr_pool *pl, const BatchConfig &c)
 {
-    return exact_classes(pl, c) ? c.occ_update_x[pl->max_s] : c.occ_update_s[pl->max_s];
+    const BatchConfig::Update &u = updates(pl, c);
+    return exact_classes(pl, u) ? u.occ_x[pl->max_s] : u.occ_s[pl->max_s];
 }
 
 static void apply_shape(swehr_pool *pl)
 {
     const int S = pl->max_s;
-    const bool exact = exact_classes(pl, pl->cfg);
-    pl->smem_update = exact ? pl->cfg.smem_update_x[S] : pl->cfg.smem_update_s[S];
-    pl->fn_update = exact ? pl->cfg.fn_update_x[S] : pl->cfg.fn_update_s[S];
+    const BatchConfig::Update &u = updates(pl, pl->cfg);
+    const bool exact = exact_classes(pl, u);
+    pl->smem_update = exact ? u.smem_x[S] : u.smem_s[S];
+    pl->fn_update = exact ? u.fn_x[S] : u.fn_s[S];
     const int occ_u = update_occupancy(pl, pl->cfg);
     const int ku = pl->ku_sel ? std::min(pl->ku_sel, occ_u) : occ_u;
     const int kw = pl->kw_sel ? pl->kw_sel : pl->cfg.occ_wave;

@@ -79,6 +79,7 @@ struct PolicyF64 {
     static constexpr bool ok = true;
     static constexpr int kMinBlocks = 2;      /* CTAs per SM the update kernel is register-budgeted for */
     static constexpr int kBatchMinBlocks = 2; /* ... and the batched update kernel */
+    static constexpr int kCommonMinBlocks = 2; /* ... with common constants */
     static constexpr bool kRollClasses = true;    /* one division and exp sequence in the code, not eight */
     typedef double Recip;
     static __device__ __forceinline__ R recip(R b) { return b; }
@@ -294,6 +295,9 @@ struct PolicyF32 {
      * spilled ~260 B per thread; at 2 (128 registers) the 256-scenario
      * ensemble steps 1.2 % faster */
     static constexpr int kBatchMinBlocks = 2;
+    /* with the constants in the constant bank again (k_update_batch) it fits
+     * three blocks as the single-domain update does */
+    static constexpr int kCommonMinBlocks = 3;
     /* unrolled: 17 % faster than rolled with the class count exact */
     static constexpr bool kRollClasses = false;
     static constexpr int kWaveMinBlocks = 5;      /* 48 registers: four cells per thread without spills */
@@ -802,14 +806,14 @@ __device__ __forceinline__ double sslope_y(const DevParams &P, const double *zs,
 /* Derived halo values from the staged planes: h, u = hu/h, v = hv/h (0 when
  * dry), sqrt(GZ h) with GZ of the previous step, SED_k.  Ghost cells read their source cell (SWEHR.c:816-1035). */
 template <class PP, class RS, int NS = 0>
-__device__ __forceinline__ void stage_derive(const DevParams &P, const SetV<RS> &src, TileCoord tc, unsigned char *smb,
+__device__ __forceinline__ void stage_derive(const DevParams &P, const DevParams &C, const SetV<RS> &src, TileCoord tc, unsigned char *smb,
                                              const StagedLayout &L, typename PP::R inh, typename PP::R inhv,
                                              typename PP::R insed)
 {
     typedef typename PP::R R;
     typedef typename PP::Fast F;
     const int S = NS ? NS : P.S;
-    const RealC<R> &K = kc<R>(P);
+    const RealC<R> &K = kc<R>(C);
     const RS *halo = reinterpret_cast<const RS *>(smb + L.halo);
     R *su = reinterpret_cast<R *>(smb + L.u), *sv = reinterpret_cast<R *>(smb + L.v);
     R *sc = reinterpret_cast<R *>(smb + L.c);
@@ -835,7 +839,7 @@ __device__ __forceinline__ void stage_derive(const DevParams &P, const SetV<RS> 
             if ((gi == 0 && P.bndry[0] == 1) || (gi == P.nx + 1 && P.bndry[2] == 1)) hu = -hu;
             if ((gj == 0 && P.bndry[1] == 1) || (gj == P.ny + 1 && P.bndry[3] == 1)) hv = -hv;
         }
-        F pp = make_fast<F>(P);
+        F pp = make_fast<F>(C);
         const bool flow = h > K.hfilm;
         const typename F::Recip rh = F::recip(h);
         R u = 0, v = 0;
@@ -1376,14 +1380,14 @@ __device__ __forceinline__ void solid_cell(const DevParams &P, const SetV<RS> &s
  * from the source set instead of their staged slots (a cell computed again,
  * whose slots already hold new values). */
 template <class PP, class RS, int MAXS, bool BUDGET, int NS, bool FRESH>
-__device__ __forceinline__ void tile_cell_pp(PP &pp, const DevParams &P, const SetV<RS> &src, const SetV<RS> &dst,
+__device__ __forceinline__ void tile_cell_pp(PP &pp, const DevParams &P, const DevParams &C, const SetV<RS> &src, const SetV<RS> &dst,
                                           const double *zp, const double *zc,
                                           double *zn, const unsigned char *smb, const StagedLayout &L,
                                           TileCoord tc, double t, double dt, double Rr, Acc2<MAXS, BUDGET> &acc,
                                           const uint8_t *__restrict__ solid, const double *__restrict__ z0)
 {
     typedef typename PP::R R;
-    const RealC<R> &K = kc<R>(P);
+    const RealC<R> &K = kc<R>(C), &own = kc<R>(P);
     const int ti = threadIdx.x / T_J, tj = threadIdx.x % T_J;
     const int i = tc.i0 + ti, j = tc.j0 + tj;
     const int64_t pl = P.plane;
@@ -1445,10 +1449,10 @@ __device__ __forceinline__ void tile_cell_pp(PP &pp, const DevParams &P, const S
                2 * rho0c >= R(0x1p-100);
     };
     if (i > 1 && i < P.nx && !zero_gradient(so + RJ, so - RJ))
-        gammax -= pp.div((rhos - rho0c) * gz * h0v * h0v, 2 * rho0c) * half * K.oneoverdx
+        gammax -= pp.div((rhos - rho0c) * gz * h0v * h0v, 2 * rho0c) * half * own.oneoverdx
                   * ((R)sTS[so + RJ] - (R)sTS[so - RJ]);
     if (j > 1 && j < P.ny && !zero_gradient(so + 1, so - 1))
-        gammay -= pp.div((rhos - rho0c) * gz * h0v * h0v, 2 * rho0c) * half * K.oneoverdx
+        gammay -= pp.div((rhos - rho0c) * gz * h0v * h0v, 2 * rho0c) * half * own.oneoverdx
                   * ((R)sTS[so + 1] - (R)sTS[so - 1]);
     /* slope stability: provable "no failure" first, exact test otherwise */
     R fail = 0;
@@ -1458,7 +1462,7 @@ __device__ __forceinline__ void tile_cell_pp(PP &pp, const DevParams &P, const S
         const R s = fabs(sy);
         const R depx = fabs((R)sDEP[i < P.nx ? so + RJ : so]) + fabs((R)sDEP[i > 1 ? so - RJ : so]);
         const R depy = fabs((R)sDEP[j < P.ny ? so + 1 : so]) + fabs((R)sDEP[j > 1 ? so - 1 : so]);
-        const R pb = fabs(dep0) * rho0 * fabs(gz) * half * K.oneoverdx * fmax(depx, depy);
+        const R pb = fabs(dep0) * rho0 * fabs(gz) * half * own.oneoverdx * fmax(depx, depy);
         const R w = rhow * gz * (dep0 + h0v);
         const R lhs_ub = A * s;
         const R rhs_lb = K.cohesion + (A * (1 - half * s * s) - w) * K.fa - pb;
@@ -1467,13 +1471,13 @@ __device__ __forceinline__ void tile_cell_pp(PP &pp, const DevParams &P, const S
         if (!safe) {
             FailArgs fa;
             fa.nx = P.nx; fa.ny = P.ny; fa.pitch = P.pitch; fa.pad_ = 0; fa.plane = P.plane;
-            fa.oneoverdx = P.oneoverdx; fa.half_odx = P.half_odx; fa.rho0 = P.rho0; fa.rhow = P.rhow;
-            fa.cohesion = P.cohesion; fa.fa = P.fa;
+            fa.oneoverdx = P.oneoverdx; fa.half_odx = P.half_odx; fa.rho0 = C.rho0; fa.rhow = C.rhow;
+            fa.cohesion = C.cohesion; fa.fa = C.fa;
             fa.solid = P.has_solid ? solid : nullptr; fa.z0 = z0;
             fail = fail_exact<typename PP::Plain, RS>(fa, src.dep, zp, zc, i, j, sx, sy, gz, dep0, rho0c, h0v);
         }
     }
-    R dfmask = fmin(one, pp.divk(totsed0 - R(0.2), R(0.2), (R)P.inv_p2, P.divk_ok));
+    R dfmask = fmin(one, pp.divk(totsed0 - R(0.2), R(0.2), (R)C.inv_p2, C.divk_ok));
     if (h0v < K.h0x9 || totsed0 < R(0.2)) dfmask = 0;
     R betax = K.neg1ml * gz * h0v * K.fa;
     R betay = K.neg1ml * gz * h0v * K.fa;
@@ -1493,7 +1497,7 @@ __device__ __forceinline__ void tile_cell_pp(PP &pp, const DevParams &P, const S
     const bool swash = (h0v > K.hfx10 && totsed0 < R(0.6));
     R E3b = 0, E4b = 0, e4den = 1;
     if (swash) {
-        const R manning = (h0v <= K.hc) ? K.roughness * pp.pow(pp.div(h0v, K.hc), K.dde) : K.roughness;
+        const R manning = (h0v <= K.hc) ? own.roughness * pp.pow(pp.div(h0v, K.hc), K.dde) : own.roughness;
         const R qq = pp.sqrtp(hu0 * hu0 + hv0 * hv0);
         const R SF = pp.div(manning * manning * qq * qq, pp.pow(h0v, R(3.333)));
         /* streampowererosion (SWEHR.c:412-426): omega is the same for every
@@ -1501,14 +1505,14 @@ __device__ __forceinline__ void tile_cell_pp(PP &pp, const DevParams &P, const S
         const R omega = rho0c * gz * SF * qq;
         if (omega > K.uc && totsed0 < R(0.6)) E3b = K.af * (omega - K.uc);
         if (omega > K.uc2 && totsed0 < R(0.6)) E4b = K.afr * (omega - K.uc2);
-        e4den = pp.divk(rhos - rho0c, rhos, (R)P.inv_rhos, P.divk_ok) * gz * h0v;
+        e4den = pp.divk(rhos - rho0c, rhos, (R)C.inv_rhos, C.divk_ok) * gz * h0v;
     }
     const typename PP::Recip rtotm = PP::recip(totm0), re4 = PP::recip(e4den);
     const R vfconc = pp.pow(1 - fmin(totsed0, R(0.99)), R(4.0));
     const bool debris = (h0v > K.h0x9 && totsed0 > K.cthreshold);
 
     /* conservative update, SWEHR.c:1424-1446 */
-    const R dtdx = dtr * K.oneoverdx;
+    const R dtdx = dtr * own.oneoverdx;
     R h = h0v - dtdx * (fxr0 - fxl0) - dtdx * (fyr0 - fyl0) + dtr * Rc;
     R hu = hu0 - dtdx * (fxr1 - fxl1) - dtdx * (fyr1 - fyl1) + dtr * SXf + dtr * gammax + dtr * dfmask * betax;
     R hv = hv0 - dtdx * (fxr2 - fxl2) - dtdx * (fyr2 - fyl2) + dtr * SYf + dtr * gammay + dtr * dfmask * betay;
@@ -1518,19 +1522,19 @@ __device__ __forceinline__ void tile_cell_pp(PP &pp, const DevParams &P, const S
     const double hd = (double)h;
     double zf, need;
     if constexpr (PP::kGuarded) {
-        zf = pp.divk(vinf0, P.thetas - P.theta0, P.inv_dtheta, 1);
-        need = pp.div(dt * ks * (zf + P.hf + hd), zf);
+        zf = pp.divk(vinf0, C.thetas - C.theta0, C.inv_dtheta, 1);
+        need = pp.div(dt * ks * (zf + C.hf + hd), zf);
     } else {
-        zf = sw_quot(vinf0, P.thetas - P.theta0, P.inv_dtheta);
-        double num = dt * ks * (zf + P.hf + hd);
+        zf = sw_quot(vinf0, C.thetas - C.theta0, C.inv_dtheta);
+        double num = dt * ks * (zf + C.hf + hd);
         need = sw_quot(num, zf, sw_rcp(zf));
-        if (!(P.fast_ok & sw_mid_pos(vinf0) & sw_mid_pos(zf) & sw_mid_or_zero(num))) {
-            zf = vinf0 / (P.thetas - P.theta0);
-            num = dt * ks * (zf + P.hf + hd);
+        if (!(C.fast_ok & sw_mid_pos(vinf0) & sw_mid_pos(zf) & sw_mid_or_zero(num))) {
+            zf = vinf0 / (C.thetas - C.theta0);
+            num = dt * ks * (zf + C.hf + hd);
             need = num / zf;
         }
     }
-    const double infl = fmin(hd - P.hfilm, need);
+    const double infl = fmin(hd - C.hfilm, need);
     const double vinf = vinf0 + infl;
     h = (R)(hd - infl);
 
@@ -1577,7 +1581,7 @@ __device__ __forceinline__ void tile_cell_pp(PP &pp, const DevParams &P, const S
          * values, computed only when needed). */
         R E1 = 0;
         if (swash && !debris) {
-            E1 = (1 - Hs) * K.pf[k] * K.a * Rc;
+            E1 = (1 - Hs) * own.pf[k] * K.a * Rc;
             if (deepv) E1 = E1 * depthfac;
         }
 
@@ -1593,17 +1597,17 @@ __device__ __forceinline__ void tile_cell_pp(PP &pp, const DevParams &P, const S
             if (swash && !debris) {
                 if (totm0 > R(1e-8) && Mk0r > R(1e-8)) E2 = pp.quot(Hs * Mk0r, rtotm) * K.ad * Rc;
                 if (deepv) E2 = E2 * depthfac;
-                E3 = pp.e3_term((1 - Hs) * K.pf[k] * K.F, K.J, (R)P.inv_J, P.divk_ok, h0v > K.ds[k] ? E3b : R(0));
+                E3 = pp.e3_term((1 - Hs) * own.pf[k] * K.F, K.J, (R)C.inv_J, C.divk_ok, h0v > own.ds[k] ? E3b : R(0));
                 if (totm0 > R(1e-6) && Mk0r > 0)
-                    E4 = pp.e4_term(K.one_m_bb * Hs * Mk0r, rtotm, K.F, re4, h0v > K.ds[k] ? E4b : R(0));
+                    E4 = pp.e4_term(K.one_m_bb * Hs * Mk0r, rtotm, K.F, re4, h0v > own.ds[k] ? E4b : R(0));
             }
             if (!debris) {
-                VF = pp.settle(K.a13[k], K.a13sq[k], K.c109s * gz * K.ds[k]);
+                VF = pp.settle(own.a13[k], own.a13sq[k], K.c109s * gz * own.ds[k]);
                 VF = VF * vfconc;
-                if (K.ds[k] > R(0.0001) && h0v < K.h0x9)
-                    VF = R(2e-3) + pp.divk_in(fmax(h0v - K.h0x3, R(0)) * (VF - R(2e-3)), K.h0x6, (R)P.inv_h0x6, P.divk_ok);
-                if (K.ds[k] > R(0.002) && h0v < K.h0x9)
-                    VF = R(2e-3) + pp.divk_in(fmax(h0v - K.h0x3, R(0)) * (VF - R(2e-3)), K.h0x6, (R)P.inv_h0x6, P.divk_ok);
+                if (own.ds[k] > R(0.0001) && h0v < K.h0x9)
+                    VF = R(2e-3) + pp.divk_in(fmax(h0v - K.h0x3, R(0)) * (VF - R(2e-3)), K.h0x6, (R)C.inv_h0x6, C.divk_ok);
+                if (own.ds[k] > R(0.002) && h0v < K.h0x9)
+                    VF = R(2e-3) + pp.divk_in(fmax(h0v - K.h0x3, R(0)) * (VF - R(2e-3)), K.h0x6, (R)C.inv_h0x6, C.divk_ok);
             }
             chtemp = u;
             const R redetach = fmin(Mk0r, dtr * (E2 + E4));
@@ -1611,22 +1615,22 @@ __device__ __forceinline__ void tile_cell_pp(PP &pp, const DevParams &P, const S
             u = dec * u;
             u = u + dtr * (E1 + E3) + redetach;
             u = dec * u;
-            z = z - P.invporo * (double)(u - chtemp);
+            z = z - C.invporo * (double)(u - chtemp);
             Mk = Mk + (double)(dtr * (E1 + E3)) - (double)(u - chtemp);
             if (BUDGET) det_k = (double)(dtr * (E1 + E3));
             if (fail == 1) {
-                z = z - 0.99 * Mk / P.porod;
+                z = z - 0.99 * Mk / C.porod;
                 u = u + (R)(0.99 * Mk);
                 totm = 0;
                 Mk = 0.01 * Mk;
                 dep = 0;
             }
         }
-        const R dh = pp.divk(u - chtemp, K.porod, (R)P.invporo, P.divk_ok);
+        const R dh = pp.divk(u - chtemp, K.porod, (R)C.invporo, C.divk_ok);
         h = h + dh;
         bulk += dh;
         totm += Mk;
-        dep += pp.dep_of(Mk, P);
+        dep += pp.dep_of(Mk, C);
         if constexpr (kSlot)
             Uslot[k * hps] = (RS)u;
         else
@@ -1654,7 +1658,7 @@ __device__ __forceinline__ void tile_cell_pp(PP &pp, const DevParams &P, const S
         for (int k = 0; k < MAXS; k++) {
             if (k >= S) break;
             const R uk = kSlot ? (R)Uslot[k * hps] : Ureg[kSlot ? 0 : k];
-            totsed += pp.divk_in(pp.quotz(uk, rh), rhos, (R)P.inv_rhos, P.divk_ok);
+            totsed += pp.divk_in(pp.quotz(uk, rh), rhos, (R)C.inv_rhos, C.divk_ok);
             dst.U[k * pl + q] = (RS)uk;
             if (stage_m) dst.M[k * pl + q] = celld[(CD_M + k) * T_I * T_J + cs];
         }
@@ -1668,7 +1672,7 @@ __device__ __forceinline__ void tile_cell_pp(PP &pp, const DevParams &P, const S
             if (k >= S) break;
             const int64_t qm = k * pl + q;
             const R uk = kSlot ? (R)Uslot[k * hps] : Ureg[kSlot ? 0 : k];
-            z = z + P.invporo * (double)uk;
+            z = z + C.invporo * (double)uk;
             const double mk = stage_m ? celld[(CD_M + k) * T_I * T_J + cs] : dst.M[qm];
             dst.M[qm] = mk + (double)uk;
             dst.U[qm] = (RS)0;
@@ -1677,7 +1681,7 @@ __device__ __forceinline__ void tile_cell_pp(PP &pp, const DevParams &P, const S
     /* implicit friction, SWEHR.c:1553-1565 */
     R vel1 = 0, vel2 = 0;
     if (h > hfilm) {
-        const R manning = (h <= K.hc) ? K.roughness * pp.pow(pp.div(h, K.hc), K.dde) : K.roughness;
+        const R manning = (h <= K.hc) ? own.roughness * pp.pow(pp.div(h, K.hc), K.dde) : own.roughness;
         const R SFf = pp.div(manning * manning * gz * pp.sqrtp(hu * hu + hv * hv) * 1, pp.pow(h, R(2.333)));
         const typename PP::Recip rf = PP::recip(1 + dtr * SFf), rh = PP::recip(h);
         hu = pp.quot(hu, rf);
@@ -1748,18 +1752,18 @@ struct CellArgs {
  * output is written again.  Its inputs are the source set and what the block
  * staged for it; of those only its own U_k and M_k slots have changed. */
 template <class PP, class RS>
-__device__ __noinline__ void tile_cell_again(const DevParams &P, const CellArgs<RS> &a)
+__device__ __noinline__ void tile_cell_again(const DevParams &P, const DevParams &C, const CellArgs<RS> &a)
 {
     PP pp;
     Acc2<16, false> none;
-    tile_cell_pp<PP, RS, 16, false, 0, true>(pp, P, a.src, a.dst, a.zp, a.zc, a.zn, a.smb, a.L, a.tc, a.t, a.dt, a.Rr,
+    tile_cell_pp<PP, RS, 16, false, 0, true>(pp, P, C, a.src, a.dst, a.zp, a.zc, a.zn, a.smb, a.L, a.tc, a.t, a.dt, a.Rr,
                                              none, a.solid, a.z0);
 }
 
 /* One thread's cell of the tile.  The budget variant of the plain form adds
  * to its sums as it goes, so it keeps the plain operators. */
 template <class PP, class RS, int MAXS, bool BUDGET, int NS = 0>
-__device__ __forceinline__ void tile_cell(const DevParams &P, const SetV<RS> &src, const SetV<RS> &dst,
+__device__ __forceinline__ void tile_cell(const DevParams &P, const DevParams &C, const SetV<RS> &src, const SetV<RS> &dst,
                                           const double *zp, const double *zc,
                                           double *zn, const unsigned char *smb, const StagedLayout &L,
                                           TileCoord tc, double t, double dt, double Rr, Acc2<MAXS, BUDGET> &acc,
@@ -1776,17 +1780,17 @@ __device__ __forceinline__ void tile_cell(const DevParams &P, const SetV<RS> &sr
     }
     typedef typename PP::Fast F;
     if constexpr (F::kGuarded && !BUDGET) {
-        F pp = make_fast<F>(P);
-        tile_cell_pp<F, RS, MAXS, BUDGET, NS, false>(pp, P, src, dst, zp, zc, zn, smb, L, tc, t, dt, Rr, acc, solid, z0);
+        F pp = make_fast<F>(C);
+        tile_cell_pp<F, RS, MAXS, BUDGET, NS, false>(pp, P, C, src, dst, zp, zc, zn, smb, L, tc, t, dt, Rr, acc, solid, z0);
         if (!pp.ok) {
             CellArgs<RS> a;
             a.src = src; a.dst = dst; a.zp = zp; a.zc = zc; a.z0 = z0; a.zn = zn; a.smb = smb; a.solid = solid;
             a.L = L; a.tc = tc; a.t = t; a.dt = dt; a.Rr = Rr;
-            tile_cell_again<typename F::Plain, RS>(P, a);
+            tile_cell_again<typename F::Plain, RS>(P, C, a);
         }
     } else {
         typename PP::Plain pp;
-        tile_cell_pp<typename PP::Plain, RS, MAXS, BUDGET, NS, false>(pp, P, src, dst, zp, zc, zn, smb, L, tc, t, dt, Rr,
+        tile_cell_pp<typename PP::Plain, RS, MAXS, BUDGET, NS, false>(pp, P, C, src, dst, zp, zc, zn, smb, L, tc, t, dt, Rr,
                                                                      acc, solid, z0);
     }
 }
@@ -1846,16 +1850,19 @@ __device__ __forceinline__ void stage_sample_tile(const DevParams &P, const SetV
 }
 
 /* Update of one tile: stages A (staging), B (faces), C (cells).  The whole
- * block calls it. */
+ * block calls it.  The constants that FailArgs, RealC and the Green-Ampt and
+ * bed terms take -- all but the grid spacing, the roughness and the classes'
+ * diameters and fractions -- are read from C, which is P or, in a batch whose
+ * scenarios agree on them, a kernel parameter. */
 template <class PP, class RS, int MAXS, bool BUDGET, bool TMA = false, int NS = 0>
-__device__ __forceinline__ void update_tile(const DevParams &P, const BufsT<RS> &B, int64_t n, double t, double dt,
+__device__ __forceinline__ void update_tile(const DevParams &P, const DevParams &C, const BufsT<RS> &B, int64_t n, double t, double dt,
                                             double Rr, TileCoord tc, unsigned char *smb, const StagedLayout &L,
                                             Acc2<MAXS, BUDGET> &acc, const TmaMaps *tm = nullptr,
                                             uint64_t *bar = nullptr, uint32_t *phase = nullptr, Ctl *ctl = nullptr)
 {
     typedef typename PP::R R;
     typedef typename PP::Fast F;
-    const RealC<R> &K = kc<R>(P);
+    const RealC<R> &K = kc<R>(C);
     const SetV<RS> src = B.set[n & 1];
     const SetV<RS> dst = B.set[(n + 1) & 1];
     const double *zp = B.z[(n + 2) % 3], *zc = B.z[n % 3];
@@ -1885,7 +1892,7 @@ __device__ __forceinline__ void update_tile(const DevParams &P, const BufsT<RS> 
         __pipeline_wait_prior(0);
         __syncthreads();
     }
-    stage_derive<PP, RS, NS>(P, src, tc, smb, L, (R)inh, (R)inhv, (R)insed);
+    stage_derive<PP, RS, NS>(P, C, src, tc, smb, L, (R)inh, (R)inhv, (R)insed);
     __syncthreads();
     const RS *sh = staged_h<RS>(smb, L), *sg = sh + HP_GZ * L.hps;
     /* stage B: every face of the tile (SWEHR.c:1099-1230) */
@@ -1928,7 +1935,7 @@ __device__ __forceinline__ void update_tile(const DevParams &P, const BufsT<RS> 
             yface = true;
         }
         R T0, T1, T2;
-        F pp = make_fast<F>(P);
+        F pp = make_fast<F>(C);
         hllc_v<F>(pp, hl, hr, nl, nr, tl, tr, g, cl, K.hfilm, T0, T1, T2);
         if constexpr (F::kGuarded)
             if (!pp.ok) {
@@ -1945,7 +1952,7 @@ __device__ __forceinline__ void update_tile(const DevParams &P, const BufsT<RS> 
         *phase += 1;
     }
     __syncthreads();
-    tile_cell<PP, RS, MAXS, BUDGET, NS>(P, src, dst, zp, zc, zn, smb, L, tc, t, dt, Rr, acc, B.solid, B.z0);
+    tile_cell<PP, RS, MAXS, BUDGET, NS>(P, C, src, dst, zp, zc, zn, smb, L, tc, t, dt, Rr, acc, B.solid, B.z0);
     __syncthreads();
 }
 
@@ -2062,7 +2069,7 @@ __global__ void __launch_bounds__(TILE_THREADS, PP::kMinBlocks) k_update_tile(co
     acc_zero(acc);
     const int64_t ntiles = (int64_t)((P.own_hi - P.own_lo + T_I) / T_I) * ((P.ny + T_J - 1) / T_J);
     for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x)
-        update_tile<PP, RS, MAXS, BUDGET, TMA, NS>(P, B, n, t, dt, Rr, tile_coord(P, tile), smb, L, acc, &tm, tma_bar,
+        update_tile<PP, RS, MAXS, BUDGET, TMA, NS>(P, P, B, n, t, dt, Rr, tile_coord(P, tile), smb, L, acc, &tm, tma_bar,
                                                &tma_phase, ctl);
     double *red = reinterpret_cast<double *>(smb + L.red);
     if (BUDGET) budget_block_sum(acc, red);
@@ -2187,7 +2194,7 @@ k_run_tile(const __grid_constant__ DevParams P, const __grid_constant__ BufsT<RS
         const bool cfl = size.courant > 1;
         Acc2<MAXS, false> none;
         for (int64_t tile = blockIdx.x; tile < ntiles; tile += grid)
-            update_tile<PP, RS, MAXS, false, true, NS>(P, B, n, t, dt, Rr, tile_coord(P, tile), smb, L, none, &tm,
+            update_tile<PP, RS, MAXS, false, true, NS>(P, P, B, n, t, dt, Rr, tile_coord(P, tile), smb, L, none, &tm,
                                                        tma_bar, &tma_phase, ctl);
         target += grid;
         if (!grid_barrier(ctl, target, &ok, [] { return true; })) return;
@@ -2374,9 +2381,15 @@ __global__ void __launch_bounds__(TILE_THREADS) k_wave_batch(const BatchHdr<RS> 
 }
 
 /* Batched update pass, with the same per-scenario runs: budget accumulators
- * carry across a run and are summed, counted and folded once per run. */
-template <class PP, class RS, int MAXS, bool BUDGET, bool STAGE_M, int NS>
-__global__ void __launch_bounds__(TILE_THREADS, PP::kBatchMinBlocks) k_update_batch(const BatchHdr<RS> *__restrict__ hdr)
+ * carry across a run and are summed, counted and folded once per run.
+ * COMMON: the running scenarios agree on the soil and flow constants (an
+ * ensemble over rain, roughness and topography, a serving mix of one soil), and
+ * those are read from the kernel parameter `common` instead of the scenario's
+ * descriptor: from shared memory every use is a load into a register, ~250 a
+ * cell, and the mixed form's registers did not fit three blocks per SM. */
+template <class PP, class RS, int MAXS, bool BUDGET, bool STAGE_M, int NS, bool COMMON>
+__global__ void __launch_bounds__(TILE_THREADS, COMMON ? PP::kCommonMinBlocks : PP::kBatchMinBlocks)
+k_update_batch(const BatchHdr<RS> *__restrict__ hdr, const __grid_constant__ DevParams common)
 {
     typedef typename PP::R R;
     extern __shared__ __align__(128) unsigned char smb[];
@@ -2443,7 +2456,7 @@ __global__ void __launch_bounds__(TILE_THREADS, PP::kBatchMinBlocks) k_update_ba
                 __syncthreads();
             }
             if (!snap.go) continue;
-            update_tile<PP, RS, MAXS, BUDGET, false, NS>(sd.P, sd.B, snap.n, snap.t, snap.dt, snap.rain,
+            update_tile<PP, RS, MAXS, BUDGET, false, NS>(sd.P, COMMON ? common : sd.P, sd.B, snap.n, snap.t, snap.dt, snap.rain,
                                               tile_coord(sd.P, g - sd.tile0), smb, L, acc);
             run++;
         }
