@@ -2061,7 +2061,7 @@ __global__ void __launch_bounds__(TILE_THREADS, PP::kMinBlocks) k_update_tile(co
         }
         __syncthreads();
     }
-    const StagedLayout L = StagedLayout::make(P.S, sizeof(R), STAGE_M);
+    const StagedLayout L = StagedLayout::make(NS ? NS : P.S, sizeof(R), STAGE_M);
     const int64_t n = ctl->step;
     const double t = ctl->t, dt = ctl->dt;
     const double Rr = P.storm ? 0.0 : rain_at(P, rain, t);
@@ -2166,7 +2166,7 @@ k_run_tile(const __grid_constant__ DevParams P, const __grid_constant__ BufsT<RS
         mbar_init_fence();
     }
     __syncthreads();
-    const StagedLayout L = StagedLayout::make(P.S, sizeof(R), STAGE_M);
+    const StagedLayout L = StagedLayout::make(NS ? NS : P.S, sizeof(R), STAGE_M);
     int64_t n = ctl->step;
     double t = ctl->t;
     const double t_stop = ctl->t_stop;
@@ -2403,10 +2403,13 @@ k_update_batch(const BatchHdr<RS> *__restrict__ hdr, const __grid_constant__ Dev
     unsigned run = 0;
     Acc2<MAXS, BUDGET> acc;
     acc_zero(acc);
-    /* the staging layout of the current scenario, uniform across the block:
-     * kept in shared memory rather than in every thread's registers */
-    __shared__ StagedLayout L;
-    if (threadIdx.x == 0) L = StagedLayout::make(1, sizeof(R), STAGE_M);
+    /* the staging layout: constants of the kernel where the class count is its
+     * own; else of the current scenario, uniform across the block and kept in
+     * shared memory rather than in every thread's registers */
+    __shared__ StagedLayout Ls;
+    if (!NS && threadIdx.x == 0) Ls = StagedLayout::make(1, sizeof(R), STAGE_M);
+    const StagedLayout Lx = StagedLayout::make(NS ? NS : 1, sizeof(R), STAGE_M);
+    const StagedLayout &L = NS ? Lx : Ls;
     auto flush = [&]() {
         Ctl *ctl = sd.ctl;
         double *red = reinterpret_cast<double *>(smb + L.red);
@@ -2452,8 +2455,10 @@ k_update_batch(const BatchHdr<RS> *__restrict__ hdr, const __grid_constant__ Dev
                 if (run) flush();
                 load_desc(tab, sid, sd, snap, true);
                 cur = sid;
-                if (threadIdx.x == 0) L = StagedLayout::make(sd.P.S, sizeof(R), STAGE_M);
-                __syncthreads();
+                if (!NS) {
+                    if (threadIdx.x == 0) Ls = StagedLayout::make(sd.P.S, sizeof(R), STAGE_M);
+                    __syncthreads();
+                }
             }
             if (!snap.go) continue;
             update_tile<PP, RS, MAXS, BUDGET, false, NS>(sd.P, COMMON ? common : sd.P, sd.B, snap.n, snap.t, snap.dt, snap.rain,
