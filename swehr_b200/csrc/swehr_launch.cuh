@@ -108,10 +108,6 @@ struct FormLauncher {
         return (int)cudaGetLastError();
     }
 
-    /* tile loads through tensor maps (both forms: every staged window starts
-     * on a 16-byte column, see Cols) */
-    static constexpr bool kHasTma = true;
-
     /* Tensor maps for the update kernel's tile loads (planes of one domain):
      * each state set's planes of the storage type with the halo box and the
      * cell box, its FP64 planes with the cell box, the three topography
@@ -142,51 +138,70 @@ struct FormLauncher {
     template <int MAXS, bool BUDGET, bool SM, bool TMA, int NS = 0>
     static void *update_fn() { return (void *)k_update_tile<PP, RS, MAXS, BUDGET, SM, TMA, NS>; }
 
-    template <bool BUDGET, bool SM, bool TMA>
-    static void *pick_u(int S)
+    /* Kernels built for one class count (1..10): their class loops have no exit
+     * tests, so the compiler interleaves the classes' independent quotient
+     * chains, and their staging layout is constant (mixed form, 7 classes: -7 %
+     * and -3.5 % against the kernels for up to 8).  Whether M_k is staged
+     * follows from the count too: where it costs no resident blocks. */
+    template <int NS>
+    static constexpr bool exact_staged()
     {
-        /* the class counts of the benchmark configurations get kernels
-         * built for exactly that many classes: their class loops have no
-         * exit tests, so the compiler interleaves the classes' independent
-         * division chains (mixed form -7 %); not for the fallback without
-         * tensor maps */
-        if constexpr (TMA) {
-            if (S == 7) return update_fn<8, BUDGET, SM, TMA, 7>();
-            if (S == 10) return update_fn<16, BUDGET, SM, TMA, 10>();
+        auto blocks = [](size_t bytes) {
+            const size_t fit = 233472 / (bytes + 1024 + 256);     /* an SM's shared memory; 1 KB a block is the system's */
+            return fit < (size_t)PP::kMinBlocks ? fit : (size_t)PP::kMinBlocks;
+        };
+        return blocks(StagedLayout::make(NS, sizeof(R), 1).total + 128) >= blocks(StagedLayout::make(NS, sizeof(R), 0).total + 128);
+    }
+    struct Exact {
+        void *update = nullptr, *run = nullptr;
+        int stage_m = 1;
+    };
+    template <int NS>
+    static Exact exact_of()
+    {
+        constexpr bool sm = exact_staged<NS>();
+        return Exact{update_fn<NS, false, sm, true, NS>(), (void *)k_run_tile<PP, RS, NS, sm, NS>, sm};
+    }
+    static Exact exact(int S)
+    {
+        switch (S) {
+        case 1: return exact_of<1>();
+        case 2: return exact_of<2>();
+        case 3: return exact_of<3>();
+        case 4: return exact_of<4>();
+        case 5: return exact_of<5>();
+        case 6: return exact_of<6>();
+        case 7: return exact_of<7>();
+        case 8: return exact_of<8>();
+        case 9: return exact_of<9>();
+        case 10: return exact_of<10>();
+        default: return Exact();
         }
-        if (S <= 4) return update_fn<4, BUDGET, SM, TMA>();
-        if (S <= 8) return update_fn<8, BUDGET, SM, TMA>();
-        return update_fn<16, BUDGET, SM, TMA>();
     }
 
-    template <int MAXS, int NS = 0>
-    static void *run_fn(bool sm)
+    /* with budgets (tensor maps) */
+    template <bool SM>
+    static void *pick_budget(int S)
     {
-        return sm ? (void *)k_run_tile<PP, RS, MAXS, true, NS> : (void *)k_run_tile<PP, RS, MAXS, false, NS>;
+        if (S == 7) return update_fn<8, true, SM, true, 7>();
+        if (S == 10) return update_fn<16, true, SM, true, 10>();
+        if (S <= 4) return update_fn<4, true, SM, true>();
+        if (S <= 8) return update_fn<8, true, SM, true>();
+        return update_fn<16, true, SM, true>();
     }
-    /* the same class counts as pick_u */
-    static void *pick_run(int S, bool sm)
+    /* without tensor maps (a driver that cannot encode them) */
+    template <bool BUDGET, bool SM>
+    static void *pick_copies(int S)
     {
-        if (S == 7) return run_fn<8, 7>(sm);
-        if (S == 10) return run_fn<16, 10>(sm);
-        if (S <= 4) return run_fn<4>(sm);
-        if (S <= 8) return run_fn<8>(sm);
-        return run_fn<16>(sm);
+        if (S <= 4) return update_fn<4, BUDGET, SM, false>();
+        if (S <= 8) return update_fn<8, BUDGET, SM, false>();
+        return update_fn<16, BUDGET, SM, false>();
     }
-
-    template <bool TMA>
-    static void *pick_update_t(int S, bool budget, bool sm)
+    template <bool SM>
+    static void *pick_update(int S, bool budget, bool tma)
     {
-        if (budget) return sm ? pick_u<true, true, TMA>(S) : pick_u<true, false, TMA>(S);
-        return sm ? pick_u<false, true, TMA>(S) : pick_u<false, false, TMA>(S);
-    }
-
-    static void *pick_update(int S, bool budget, bool sm, bool tma = false)
-    {
-        if constexpr (kHasTma) {
-            if (tma) return pick_update_t<true>(S, budget, sm);
-        }
-        return pick_update_t<false>(S, budget, sm);
+        if (!tma) return budget ? pick_copies<true, SM>(S) : pick_copies<false, SM>(S);
+        return budget ? pick_budget<SM>(S) : update_fn<16, false, SM, true>();
     }
 
     static int configure(const DevParams &P, int num_sms, StepConfig &cfg)
@@ -197,11 +212,23 @@ struct FormLauncher {
         size_t su = 0;
         const size_t sw = wave_smem();
         int occ_u = 0, occ_w = 0, stage_m = 1;
-        const bool tma = kHasTma && cfg.tma;
+        const bool tma = cfg.tma != 0;
         cfg.tma = tma ? 1 : 0;
-        cudaError_t e = pick_staging(pick_update(P.S, P.budget != 0, true, tma),
-                                     pick_update(P.S, P.budget != 0, false, tma), P.S, su, occ_u, stage_m, fu,
-                                     tma ? 128 : 0);
+        const Exact x = tma && !P.budget ? exact(P.S) : Exact();
+        void *fr = x.run;
+        cudaError_t e;
+        if (x.update) {
+            fu = x.update;
+            stage_m = x.stage_m;
+            su = update_smem(P.S, stage_m) + 128;
+            e = cudaFuncSetAttribute(fu, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)su);
+            if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_u, fu, TILE_THREADS, su);
+        } else {
+            e = pick_staging(pick_update<true>(P.S, P.budget != 0, tma), pick_update<false>(P.S, P.budget != 0, tma), P.S, su,
+                             occ_u, stage_m, fu, tma ? 128 : 0);
+            if (tma && !P.budget)
+                fr = stage_m ? (void *)k_run_tile<PP, RS, 16, true, 0> : (void *)k_run_tile<PP, RS, 16, false, 0>;
+        }
         if (e != cudaSuccess) return (int)e;
         e = cudaFuncSetAttribute(fw, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sw);
         if (e != cudaSuccess) return (int)e;
@@ -217,8 +244,7 @@ struct FormLauncher {
         cfg.fn_wave = fw;
         cfg.stage_m = stage_m;
         cfg.fn_run = nullptr;
-        if (tma && !P.budget && !P.has_solid && ntiles <= (int64_t)RUN_TILES_PER_SM * num_sms) {
-            void *fr = pick_run(P.S, stage_m != 0);
+        if (fr && !P.has_solid && ntiles <= (int64_t)RUN_TILES_PER_SM * num_sms) {
             int occ = 0, coop = 0, dev = 0;
             e = cudaFuncSetAttribute(fr, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)su);
             if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fr, TILE_THREADS, su);

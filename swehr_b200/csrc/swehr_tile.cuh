@@ -578,9 +578,9 @@ struct StagedLayout {
     /* stage_m: staging M_k costs 2 KB of shared memory per class; the
      * launcher picks the kernel that stages it only where that costs no
      * resident blocks (a compile-time choice of each kernel) */
-    __host__ __device__ static StagedLayout make(int S, size_t rs, int stage_m = 1)
+    __host__ __device__ static constexpr StagedLayout make(int S, size_t rs, int stage_m = 1)
     {
-        StagedLayout L;
+        StagedLayout L{};
         size_t o = 0;
         /* every region starts 128-byte aligned (a tile copy's destination) */
         auto take = [&](size_t bytes) { size_t at = o; o += (bytes + 127) / 128 * 128; return at; };
