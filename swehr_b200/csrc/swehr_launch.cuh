@@ -269,7 +269,7 @@ struct FormLauncher {
     template <int MAXS, int NS, bool COMMON>
     static cudaError_t exact_batch(bool budget, BatchConfig::Update &u)
     {
-        constexpr int blocks = COMMON ? PP::kCommonMinBlocks : PP::kBatchMinBlocks;
+        constexpr int blocks = COMMON ? PP::kCommonMinBlocks : PP::kBatchMinBlocks;      /* as in k_update_batch */
         constexpr bool sm = NS == 7 || (NS == 10 && sizeof(RS) == 4 && blocks == 2);
         void *f = ubatch_fn<MAXS, false, sm, NS, COMMON>();
         if constexpr (!COMMON)

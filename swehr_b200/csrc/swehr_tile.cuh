@@ -79,7 +79,7 @@ struct PolicyF64 {
     static constexpr bool ok = true;
     static constexpr int kMinBlocks = 2;      /* CTAs per SM the update kernel is register-budgeted for */
     static constexpr int kBatchMinBlocks = 2; /* ... and the batched update kernel */
-    static constexpr int kCommonMinBlocks = 2; /* ... with common constants */
+    static constexpr int kCommonMinBlocks = 2; /* ... of an exact class count with common constants */
     static constexpr bool kRollClasses = true;    /* one division and exp sequence in the code, not eight */
     typedef double Recip;
     static __device__ __forceinline__ R recip(R b) { return b; }
@@ -295,8 +295,11 @@ struct PolicyF32 {
      * spilled ~260 B per thread; at 2 (128 registers) the 256-scenario
      * ensemble steps 1.2 % faster */
     static constexpr int kBatchMinBlocks = 2;
-    /* with the constants in the constant bank again (k_update_batch) it fits
-     * three blocks as the single-domain update does */
+    /* with the constants in the constant bank again (k_update_batch) the
+     * kernels of an exact class count fit three blocks as the single-domain
+     * update does (16 pooled catchments 0.447 -> 0.428 ms a pool step); the one
+     * for any count up to 16 does not (5 to 10 classes: 0.474 ms at two blocks,
+     * 0.540 at three) */
     static constexpr int kCommonMinBlocks = 3;
     /* unrolled: 17 % faster than rolled with the class count exact */
     static constexpr bool kRollClasses = false;
@@ -2388,7 +2391,7 @@ __global__ void __launch_bounds__(TILE_THREADS) k_wave_batch(const BatchHdr<RS> 
  * descriptor: from shared memory every use is a load into a register, ~250 a
  * cell, and the mixed form's registers did not fit three blocks per SM. */
 template <class PP, class RS, int MAXS, bool BUDGET, bool STAGE_M, int NS, bool COMMON>
-__global__ void __launch_bounds__(TILE_THREADS, COMMON ? PP::kCommonMinBlocks : PP::kBatchMinBlocks)
+__global__ void __launch_bounds__(TILE_THREADS, COMMON && NS ? PP::kCommonMinBlocks : PP::kBatchMinBlocks)
 k_update_batch(const BatchHdr<RS> *__restrict__ hdr, const __grid_constant__ DevParams common)
 {
     typedef typename PP::R R;
