@@ -78,6 +78,7 @@ struct PolicyF64 {
     static constexpr bool kGuarded = false;
     static constexpr bool ok = true;
     static constexpr int kMinBlocks = 2;      /* CTAs per SM the update kernel is register-budgeted for */
+    static constexpr int kBudgetMinBlocks = 2; /* ... with budgets */
     static constexpr int kBatchMinBlocks = 2; /* ... and the batched update kernel */
     static constexpr int kCommonMinBlocks = 2; /* ... of an exact class count with common constants */
     static constexpr bool kRollClasses = true;    /* one division and exp sequence in the code, not eight */
@@ -290,6 +291,9 @@ struct PolicyF32 {
     static constexpr bool kGuarded = false;
     static constexpr bool ok = true;
     static constexpr int kMinBlocks = 3;
+    /* with the budget's sums in registers three blocks spill ~400 B a thread:
+     * 200 x 50 cells 40.5 us a step at three, 35.8 at two, 2048^2 850 and 701 */
+    static constexpr int kBudgetMinBlocks = 2;
     /* the batched update reads its scenario's parameters from shared memory,
      * not the constant bank, and needs more registers: at 3 CTAs per SM it
      * spilled ~260 B per thread; at 2 (128 registers) the 256-scenario
@@ -2038,7 +2042,7 @@ __device__ __forceinline__ void budget_fold(Ctl *ctl, int m, double hi, double l
 }
 
 template <class PP, class RS, int MAXS, bool BUDGET, bool STAGE_M, bool TMA, int NS>
-__global__ void __launch_bounds__(TILE_THREADS, PP::kMinBlocks) k_update_tile(const __grid_constant__ DevParams P, const BufsT<RS> B, Ctl *ctl,
+__global__ void __launch_bounds__(TILE_THREADS, BUDGET ? PP::kBudgetMinBlocks : PP::kMinBlocks) k_update_tile(const __grid_constant__ DevParams P, const BufsT<RS> B, Ctl *ctl,
                                                                   const double *__restrict__ rain, double *partials,
                                                                   double *stage, double *saveflow,
                                                                   const __grid_constant__ TmaMaps tm)
