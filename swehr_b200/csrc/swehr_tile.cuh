@@ -1475,7 +1475,9 @@ __device__ __forceinline__ void tile_cell_pp(PP &pp, const DevParams &P, const D
         const R rhs_lb = K.cohesion + (A * (1 - half * s * s) - w) * K.fa - pb;
         const R margin = R(1e-5) * (fabs(A) * (1 + s) + K.cohesion + fabs(w) * K.fa + pb) + R(1e-30);
         const bool safe = A >= 0 && gz > 0 && K.fa >= 0 && lhs_ub + margin < rhs_lb;
-        if (!safe) {
+        /* a NaN deposit (the inflow row's) makes the test's left side a NaN: no
+         * failure, without the test (3 x 51 example: 19.5 -> 17 us a step) */
+        if (!safe && dep0 == dep0) {
             FailArgs fa;
             fa.nx = P.nx; fa.ny = P.ny; fa.pitch = P.pitch; fa.pad_ = 0; fa.plane = P.plane;
             fa.oneoverdx = P.oneoverdx; fa.half_odx = P.half_odx; fa.rho0 = C.rho0; fa.rhow = C.rhow;
