@@ -102,13 +102,19 @@ SW_HD double sw_rcp(double b)
     return sw_rcp_refine(b, y);
 }
 
-/* sqrt(x), or +0 for a zero of either sign (pow(x, 0.5)) */
-SW_HD double sw_sqrt_mid(double x)
+/* sqrt(x), x > 0 */
+SW_HD double sw_sqrt_pos(double x)
 {
     double y;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double g = sw_sqrt_refine(x, y);
-    return x == 0 ? 0.0 : g;
+    return sw_sqrt_refine(x, y);
+}
+
+/* sqrt(x), or +0 for a zero of either sign (pow(x, 0.5)) */
+SW_HD double sw_sqrt_mid(double x)
+{
+    const double g = sw_sqrt_pos(x);
+    return ((__double2hiint(x) & 0x7fffffff) | __double2loint(x)) == 0 ? 0.0 : g;
 }
 
 /* Sizes, tested on the high word read as a float: its order is that of the
@@ -223,7 +229,7 @@ SW_HD double sw_cos_atan_mid(double x, bool *ok)
     const double sh = 1.0 + p;
     const double bb = sh - 1.0;
     const double sl = ((1.0 - (sh - bb)) + (p - bb)) + pe;
-    const double root = sw_sqrt_mid(sh);
+    const double root = sw_sqrt_pos(sh);
     *ok &= sw_below(x, 0x58F00000);
     const double r0 = sw_quot(1.0, root, sw_rcp(root));
     const double q = r0 * r0;

@@ -234,7 +234,7 @@ struct FastF64 {
     __device__ __forceinline__ R root1(R x)
     {
         ok &= sw_small(x);
-        return sw_sqrt_mid(x);
+        return sw_sqrt_pos(x);
     }
     __device__ __forceinline__ R pow(R x, R y)
     {
@@ -276,7 +276,7 @@ struct FastF64 {
     }
     /* A^2 and c = 1.09 (rhos/rhow - 1) gz d are in range with the run's
      * constants: gz = g / root, root >= 1 tested where it was formed */
-    static __device__ __forceinline__ R settle(R A, R A2, R c) { return sw_sqrt_mid(A2 + c) - A; }
+    static __device__ __forceinline__ R settle(R A, R A2, R c) { return sw_sqrt_pos(A2 + c) - A; }
     __device__ __forceinline__ double dep_of(double M, const DevParams &P)
     {
         ok &= sw_mid_or_zero(M) | (M != M);

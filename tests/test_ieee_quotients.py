@@ -47,7 +47,7 @@ int64_t check_sqrt(const double *x, int64_t n, int rounds, uint64_t seed)
 """
 
 
-def random_pairs(n, seed, span=400):
+def random_pairs(n, seed, span=299):
     rng = np.random.default_rng(seed)
     a = rng.uniform(1, 2, n) * np.exp2(rng.integers(-span, span, n)) * rng.choice([-1.0, 1.0], n)
     b = rng.uniform(1, 2, n) * np.exp2(rng.integers(-span, span, n))
