@@ -1273,6 +1273,39 @@ struct Acc2 {
     double det[BUDGET ? MAXS : 1], sout[BUDGET ? MAXS : 1], sround[BUDGET ? MAXS : 1];
 };
 
+template <int MAXS, bool BUDGET>
+__device__ __forceinline__ void acc_zero(Acc2<MAXS, BUDGET> &acc)
+{
+    acc.rain = acc.out = acc.clamp = acc.bulk = acc.inf = acc.round = 0;
+#pragma unroll
+    for (int k = 0; k < (BUDGET ? MAXS : 1); k++) acc.det[k] = acc.sout[k] = acc.sround[k] = 0;
+}
+
+template <int MAXS, bool BUDGET>
+__device__ __forceinline__ void acc_add(Acc2<MAXS, BUDGET> &a, const Acc2<MAXS, BUDGET> &b)
+{
+    a.rain += b.rain; a.out += b.out; a.clamp += b.clamp; a.bulk += b.bulk; a.inf += b.inf; a.round += b.round;
+#pragma unroll
+    for (int k = 0; k < (BUDGET ? MAXS : 1); k++) {
+        a.det[k] += b.det[k];
+        a.sout[k] += b.sout[k];
+        a.sround[k] += b.sround[k];
+    }
+}
+
+/* b's first MAXS classes */
+template <int MAXS, bool BUDGET>
+__device__ __forceinline__ void acc_copy(Acc2<MAXS, BUDGET> &a, const Acc2<16, BUDGET> &b)
+{
+    a.rain = b.rain; a.out = b.out; a.clamp = b.clamp; a.bulk = b.bulk; a.inf = b.inf; a.round = b.round;
+#pragma unroll
+    for (int k = 0; k < (BUDGET ? MAXS : 1); k++) {
+        a.det[k] = b.det[k];
+        a.sout[k] = b.sout[k];
+        a.sround[k] = b.sround[k];
+    }
+}
+
 /* Parameters of the exact slope-failure test (passed by value: a pointer to
  * the kernel's parameter block would force a local copy of all of it). */
 struct FailArgs {
@@ -1760,17 +1793,18 @@ struct CellArgs {
 /* A cell whose operands FastF64 does not take, with plain operators: every
  * output is written again.  Its inputs are the source set and what the block
  * staged for it; of those only its own U_k and M_k slots have changed. */
-template <class PP, class RS>
-__device__ __noinline__ void tile_cell_again(const DevParams &P, const DevParams &C, const CellArgs<RS> &a)
+template <class PP, class RS, bool BUDGET>
+__device__ __noinline__ void tile_cell_again(const DevParams &P, const DevParams &C, const CellArgs<RS> &a,
+                                             Acc2<16, BUDGET> &add)
 {
     PP pp;
-    Acc2<16, false> none;
-    tile_cell_pp<PP, RS, 16, false, 0, true>(pp, P, C, a.src, a.dst, a.zp, a.zc, a.zn, a.smb, a.L, a.tc, a.t, a.dt, a.Rr,
-                                             none, a.solid, a.z0);
+    acc_zero(add);
+    tile_cell_pp<PP, RS, 16, BUDGET, 0, true>(pp, P, C, a.src, a.dst, a.zp, a.zc, a.zn, a.smb, a.L, a.tc, a.t, a.dt, a.Rr,
+                                              add, a.solid, a.z0);
 }
 
-/* One thread's cell of the tile.  The budget variant of the plain form adds
- * to its sums as it goes, so it keeps the plain operators. */
+/* One thread's cell of the tile.  A cell that may be computed again adds to
+ * sums of its own first. */
 template <class PP, class RS, int MAXS, bool BUDGET, int NS = 0>
 __device__ __forceinline__ void tile_cell(const DevParams &P, const DevParams &C, const SetV<RS> &src, const SetV<RS> &dst,
                                           const double *zp, const double *zc,
@@ -1788,15 +1822,20 @@ __device__ __forceinline__ void tile_cell(const DevParams &P, const DevParams &C
         }
     }
     typedef typename PP::Fast F;
-    if constexpr (F::kGuarded && !BUDGET) {
+    if constexpr (F::kGuarded) {
         F pp = make_fast<F>(C);
-        tile_cell_pp<F, RS, MAXS, BUDGET, NS, false>(pp, P, C, src, dst, zp, zc, zn, smb, L, tc, t, dt, Rr, acc, solid, z0);
+        Acc2<MAXS, BUDGET> add;
+        acc_zero(add);
+        tile_cell_pp<F, RS, MAXS, BUDGET, NS, false>(pp, P, C, src, dst, zp, zc, zn, smb, L, tc, t, dt, Rr, add, solid, z0);
         if (!pp.ok) {
             CellArgs<RS> a;
             a.src = src; a.dst = dst; a.zp = zp; a.zc = zc; a.z0 = z0; a.zn = zn; a.smb = smb; a.solid = solid;
             a.L = L; a.tc = tc; a.t = t; a.dt = dt; a.Rr = Rr;
-            tile_cell_again<typename F::Plain, RS>(P, C, a);
+            Acc2<16, BUDGET> plain;
+            tile_cell_again<typename F::Plain, RS, BUDGET>(P, C, a, plain);
+            if (BUDGET) acc_copy(add, plain);
         }
+        if (BUDGET) acc_add(acc, add);
     } else {
         typename PP::Plain pp;
         tile_cell_pp<typename PP::Plain, RS, MAXS, BUDGET, NS, false>(pp, P, C, src, dst, zp, zc, zn, smb, L, tc, t, dt, Rr,
@@ -1992,14 +2031,6 @@ __device__ __forceinline__ void budget_block_sum(const Acc2<MAXS, BUDGET> &acc, 
             red[m] = s;
         }
     __syncthreads();
-}
-
-template <int MAXS, bool BUDGET>
-__device__ __forceinline__ void acc_zero(Acc2<MAXS, BUDGET> &acc)
-{
-    acc.rain = acc.out = acc.clamp = acc.bulk = acc.inf = acc.round = 0;
-#pragma unroll
-    for (int k = 0; k < (BUDGET ? MAXS : 1); k++) acc.det[k] = acc.sout[k] = acc.sround[k] = 0;
 }
 
 /* End of a step once every cell is written (whole block): time, step
