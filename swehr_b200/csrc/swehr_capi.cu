@@ -5,8 +5,9 @@
  * device memory of a context is one allocation (state sets, topography
  * planes, Ks, rain, control block, reduction partials, stage rows), sized by
  * swehr_footprint_bytes().  Stepping is enqueued as CUDA graphs of whole
- * steps; the device decides when to stop (t >= tend, t_stop, step limit,
- * CFL error), so a bounded advance is one host synchronisation at the end.
+ * steps, on a small domain as launches of many steps; the device decides when
+ * to stop (t >= tend, t_stop, step limit, CFL error), so a bounded advance is
+ * one host synchronisation at the end.
  */
 #include <cuda_runtime.h>
 
@@ -402,19 +403,26 @@ static int d2h_chunks(swehr_ctx *c, char *stage, double *host, const void *dev, 
     return SWEHR_OK;
 }
 
+/* straight to the pageable destination */
+static int d2h_direct(swehr_ctx *c, double *host, const void *dev, size_t spitch, size_t esize, int64_t nrows,
+                      int64_t ncols)
+{
+    const size_t row_in = (size_t)ncols * esize;
+    std::vector<float> tmp(esize == sizeof(double) ? 0 : (size_t)(nrows * ncols));
+    void *dst = esize == sizeof(double) ? (void *)host : (void *)tmp.data();
+    CK(cudaMemcpy2DAsync(dst, row_in, dev, spitch, row_in, (size_t)nrows, cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaStreamSynchronize(c->stream));
+    for (size_t q = 0; q < tmp.size(); q++) host[q] = (double)tmp[q];
+    return SWEHR_OK;
+}
+
 /* the rows are in host when it returns (SWEHR_OK) */
 static int d2h_rows(swehr_ctx *c, double *host, const void *dev, size_t spitch, size_t esize, int64_t nrows,
                     int64_t ncols)
 {
     const size_t row_in = (size_t)ncols * esize;
-    if (row_in > kStageBytes) {          /* a single row beyond the buffer: straight to the pageable destination */
-        std::vector<float> tmp(esize == sizeof(double) ? 0 : (size_t)(nrows * ncols));
-        void *dst = esize == sizeof(double) ? (void *)host : (void *)tmp.data();
-        CK(cudaMemcpy2DAsync(dst, row_in, dev, spitch, row_in, (size_t)nrows, cudaMemcpyDeviceToHost, c->stream));
-        CK(cudaStreamSynchronize(c->stream));
-        for (size_t q = 0; q < tmp.size(); q++) host[q] = (double)tmp[q];
-        return SWEHR_OK;
-    }
+    if (row_in > kStageBytes)            /* a single row beyond the buffer */
+        return d2h_direct(c, host, dev, spitch, esize, nrows, ncols);
     /* one pinned buffer per process, used by one read at a time, as large as
      * the largest read needed (pinning 32 MB takes ~0.1 s) */
     static std::mutex mu;
@@ -428,7 +436,12 @@ static int d2h_rows(swehr_ctx *c, double *host, const void *dev, size_t spitch, 
         if (stage) CK(cudaFreeHost(stage));
         stage = nullptr;
         held = 0;
-        CK(cudaHostAlloc((void **)&stage, want, cudaHostAllocPortable));
+        if (cudaHostAlloc((void **)&stage, want, cudaHostAllocPortable) != cudaSuccess) {
+            /* no page-locked memory (a limit of the process): the read needs none */
+            cudaGetLastError();
+            stage = nullptr;
+            return d2h_direct(c, host, dev, spitch, esize, nrows, ncols);
+        }
         held = want;
     }
     for (int e = 0; e < kStageThreadsMax; e++)

@@ -3,7 +3,8 @@
  * Compiled with --fmad=false: no contraction, so every cell is bit-identical
  * to the CPU restatement built with the project's math.
  *
- * A step is two stream-ordered launches and needs no grid barrier:
+ * A step is two stream-ordered launches and needs no grid barrier (a small
+ * domain takes many steps in one cooperative launch, k_run_tile):
  *   k_wave_cells  largest wave speed over every face (SWEHR.c:1092-1230's
  *                 Smax), one cell's faces per thread straight from global
  *                 memory; the last block to finish computes dt and the
@@ -16,7 +17,8 @@
  *                 t_stop, the step limit or a CFL error.
  * Both kernels read the step counter from the control block to pick their
  * buffers, so every step is the same pair of launches and a chunk of steps
- * is captured once as a CUDA graph.  Nothing spins or waits on the device.
+ * is captured once as a CUDA graph.  The waits on the device (a tile's loads,
+ * k_run_tile's grid barriers) give up after a fixed number of polls.
  */
 #include "swehr_launch.cuh"
 

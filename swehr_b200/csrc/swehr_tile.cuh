@@ -16,7 +16,7 @@
  *      SWEHR.c:816-1035) is staged in shared memory: h, the velocities
  *      u = hu/h and v = hv/h (0 when dry, SWEHR.c:333-352), the previous
  *      step's gravity GZ and sqrt(GZ h) of every cell that is the left/lower
- *      cell of a face, SED_k, TOTSED and DEP;
+ *      cell of a face (GZ is a plane of the state), SED_k, TOTSED and DEP;
  *   B. every face of the tile is solved once (SWEHR.c:327-409) into shared
  *      memory: 9x32 x-faces and 8x33 y-faces for 256 cells;
  *   C. one thread per cell: sources (SWEHR.c:1239-1401), the conservative,
@@ -26,7 +26,7 @@
  * The slope-failure test (SWEHR.c:1292-1312) costs six cos/sin(atan) and
  * neighbour slopes per cell but can only fire on steep, thick deposits: a
  * bound that needs none of them (sin(atan s) <= s, cos(atan s) >= 1 - s^2/2,
- * cos <= 1 in the pressure-gradient term) proves "no failure" with a 1e-6
+ * cos <= 1 in the pressure-gradient term) proves "no failure" with a 1e-5
  * relative margin for nearly every cell; the exact test runs otherwise.
  */
 #pragma once
@@ -1509,7 +1509,8 @@ __device__ __forceinline__ void tile_cell_pp(PP &pp, const DevParams &P, const D
         const R margin = R(1e-5) * (fabs(A) * (1 + s) + K.cohesion + fabs(w) * K.fa + pb) + R(1e-30);
         const bool safe = A >= 0 && gz > 0 && K.fa >= 0 && lhs_ub + margin < rhs_lb;
         /* a NaN deposit (the inflow row's) makes the test's left side a NaN: no
-         * failure, without the test (3 x 51 example: 19.5 -> 17 us a step) */
+         * failure, without the test (3 x 51 example, whose inflow row has one:
+         * with the one-class kernel 19.5 -> 17 us a step) */
         if (!safe && dep0 == dep0) {
             FailArgs fa;
             fa.nx = P.nx; fa.ny = P.ny; fa.pitch = P.pitch; fa.pad_ = 0; fa.plane = P.plane;
