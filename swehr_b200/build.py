@@ -82,10 +82,11 @@ def build_probe(verbose: bool = False) -> str:
     """The benchmark's device-peak probe (FP64 pipe ceiling) and the arithmetic
     probe of the tests, their own library."""
     src = os.path.join(CSRC, "swehr_probe.cu")
-    deps = [src] + [os.path.join(CSRC, f) for f in ("swehr_ieee.h", "swehr_math.h", "swehr_math_tables.h")]
+    deps = [src] + [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".h", ".cuh"))]
     if os.path.exists(PROBE) and all(os.path.getmtime(PROBE) >= os.path.getmtime(d) for d in deps):
         return PROBE
-    cmd = [nvcc()] + ARCH + ["-O3", "-std=c++17", "--fmad=false", "-Xcompiler", "-fPIC", "-shared", src, "-o", PROBE, "-lcudart"]
+    cmd = [nvcc()] + ARCH + ["-O3", "-std=c++17", "--fmad=false", "-Xcompiler", "-fPIC",
+                           "-I", os.path.join(HERE, "..", "include"), "-shared", src, "-o", PROBE, "-lcudart"]
     if verbose:
         print(" ".join(cmd))
     subprocess.check_call(cmd)

@@ -764,6 +764,15 @@ extern "C" int swehr_advance(swehr_ctx *c, double t_stop, int64_t max_steps, swe
         }
         return SWEHR_CFL_ERROR;
     }
+    if (h->status == SWEHR_TIMEOUT || h->dev_error) {
+        /* a wait on the device gave up in an earlier step: its cells are not all written */
+        if (pr) {
+            memset(pr, 0, sizeof *pr);
+            pr->t = h->t; pr->steps = h->step; pr->status = SWEHR_TIMEOUT;
+            pr->dt = h->dt; pr->courant = h->courant; pr->rain = h->rain_now; pr->t_step = h->t_prev;
+        }
+        return set_err(SWEHR_TIMEOUT, "a wait on the device gave up; the state is not that of a whole step");
+    }
     double kernel_ms = 0;
     int64_t launched = 0;
     bool run = h->t < c->p.tend && h->t < t_stop && max_steps != 0;

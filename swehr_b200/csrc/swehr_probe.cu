@@ -13,6 +13,7 @@
  */
 #include <cuda_runtime.h>
 
+#include "swehr_ctx.h"
 #include "swehr_ieee.h"
 
 static const int PROBE_THREADS = 256;
@@ -104,4 +105,12 @@ extern "C" int swehr_probe_ieee(int op, const double *a, const double *b, long l
     cudaMemcpy(refused, d + 4 * n, bytes, cudaMemcpyDeviceToHost);
     cudaFree(d);
     return cudaGetLastError() == cudaSuccess ? 0 : 3;
+}
+
+/* swehr_probe_give_up: the flag that a wait on the device sets when it gives
+ * up, set from the host, for the tests of what follows it. */
+extern "C" int swehr_probe_give_up(swehr_ctx *c)
+{
+    const int32_t one = 1;
+    return c && cudaMemcpy(&c->d_ctl->dev_error, &one, sizeof one, cudaMemcpyHostToDevice) == cudaSuccess ? 0 : 1;
 }

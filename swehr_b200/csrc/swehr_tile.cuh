@@ -2156,7 +2156,9 @@ __global__ void __launch_bounds__(TILE_THREADS, BUDGET ? PP::kBudgetMinBlocks : 
 /* count: arrivals of all launches of this grid, a multiple of the grid size
  * between launches; target: the count that ends this barrier.  The whole
  * block calls it; `ok` is shared.  then() runs in thread 0 before the block
- * goes on, and says whether it does. */
+ * goes on, and says whether it does; a block that does not ends the run with
+ * SWEHR_TIMEOUT, after which swehr_advance takes no further step (the arrivals
+ * counted here need not be whole then). */
 template <class Then>
 __device__ __forceinline__ bool grid_barrier(Ctl *ctl, unsigned long long target, bool *ok, Then then)
 {
@@ -2172,12 +2174,12 @@ __device__ __forceinline__ bool grid_barrier(Ctl *ctl, unsigned long long target
             done = v >= target;
         }
         __threadfence();
-        if (!done) {
+        done = done && then();
+        if (!done) {                     /* the same values from every block that gives up */
             ctl->dev_error = 1;
             ctl->status = 3;
             ctl->active = 0;
-        } else
-            done = then();
+        }
         *ok = done;
     }
     __syncthreads();
@@ -2203,7 +2205,7 @@ k_run_tile(const __grid_constant__ DevParams P, const __grid_constant__ BufsT<RS
     uint32_t tma_phase = 0;
     if (threadIdx.x == 0) {
         mbar_init(&tma_bar[0], 1);
-            mbar_init(&tma_bar[1], 1);
+        mbar_init(&tma_bar[1], 1);
         mbar_init_fence();
     }
     __syncthreads();
