@@ -7,6 +7,7 @@
 #include <cuda_runtime.h>
 
 #include <cstring>
+#include <mutex>
 #include <type_traits>
 
 #include "swehr_kernels.h"
@@ -53,6 +54,19 @@ static inline bool encode_planes(TensorMapEncodeFn enc, CUtensorMap *m, const vo
            CUDA_SUCCESS;
 }
 
+/* A kernel's dynamic shared memory limit belongs to the process (on one
+ * device), not to the simulation or pool that sets it: one that needs less,
+ * made later, must leave the others' launches possible, so it is only raised. */
+static inline cudaError_t raise_smem_limit(const void *fn, size_t bytes)
+{
+    static std::mutex mu;
+    std::lock_guard<std::mutex> lock(mu);
+    cudaFuncAttributes a;
+    const cudaError_t e = cudaFuncGetAttributes(&a, fn);
+    if (e != cudaSuccess || (size_t)a.maxDynamicSharedSizeBytes >= bytes) return e;
+    return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+}
+
 inline namespace SWEHR_TILE_NS {
 
 /* Tiles per SM up to which a domain is stepped by k_run_tile.  Measured (B200,
@@ -85,9 +99,9 @@ struct FormLauncher {
     {
         const size_t with = update_smem(S, 1) + extra, without = update_smem(S, 0) + extra;
         int ow = 0, oo = 0;
-        cudaError_t e = cudaFuncSetAttribute(f_with, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)with);
+        cudaError_t e = raise_smem_limit(f_with, with);
         if (e != cudaSuccess) return e;
-        e = cudaFuncSetAttribute(f_without, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)without);
+        e = raise_smem_limit(f_without, without);
         if (e != cudaSuccess) return e;
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ow, f_with, TILE_THREADS, with);
         if (e != cudaSuccess) return e;
@@ -221,7 +235,7 @@ struct FormLauncher {
             fu = x.update;
             stage_m = x.stage_m;
             su = update_smem(P.S, stage_m) + 128;
-            e = cudaFuncSetAttribute(fu, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)su);
+            e = raise_smem_limit(fu, su);
             if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_u, fu, TILE_THREADS, su);
         } else {
             e = pick_staging(pick_update<true>(P.S, P.budget != 0, tma), pick_update<false>(P.S, P.budget != 0, tma), P.S, su,
@@ -230,7 +244,7 @@ struct FormLauncher {
                 fr = stage_m ? (void *)k_run_tile<PP, RS, 16, true, 0> : (void *)k_run_tile<PP, RS, 16, false, 0>;
         }
         if (e != cudaSuccess) return (int)e;
-        e = cudaFuncSetAttribute(fw, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sw);
+        e = raise_smem_limit(fw, sw);
         if (e != cudaSuccess) return (int)e;
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_w, fw, TILE_THREADS, sw);
         if (e != cudaSuccess) return (int)e;
@@ -246,7 +260,7 @@ struct FormLauncher {
         cfg.fn_run = nullptr;
         if (fr && !P.has_solid && ntiles <= (int64_t)RUN_TILES_PER_SM * num_sms) {
             int occ = 0, coop = 0, dev = 0;
-            e = cudaFuncSetAttribute(fr, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)su);
+            e = raise_smem_limit(fr, su);
             if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fr, TILE_THREADS, su);
             if (e == cudaSuccess) e = cudaGetDevice(&dev);
             if (e == cudaSuccess) e = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
@@ -275,7 +289,7 @@ struct FormLauncher {
         if constexpr (!COMMON)
             if (budget) f = ubatch_fn<MAXS, true, sm, NS, COMMON>();
         u.smem_x[NS] = update_smem(NS, sm);
-        cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)u.smem_x[NS]);
+        cudaError_t e = raise_smem_limit(f, u.smem_x[NS]);
         if (e == cudaSuccess)
             e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&u.occ_x[NS], f, TILE_THREADS, u.smem_x[NS]);
         if (u.occ_x[NS] < 1) u.occ_x[NS] = 1;
@@ -311,9 +325,9 @@ struct FormLauncher {
         if (e == cudaSuccess && max_classes >= 10) e = exact_batch<16, 10, COMMON>(budget, u);
         /* limits for the largest shape either kernel is launched with */
         if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(with, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)update_smem(max_classes));
+            e = raise_smem_limit(with, update_smem(max_classes));
         if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(without, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)update_smem(max_classes, 0));
+            e = raise_smem_limit(without, update_smem(max_classes, 0));
         return e;
     }
 
@@ -321,7 +335,7 @@ struct FormLauncher {
     {
         void *fw = (void *)k_wave_batch<PP, RS>;
         const size_t sw = wave_smem();
-        cudaError_t e = cudaFuncSetAttribute(fw, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sw);
+        cudaError_t e = raise_smem_limit(fw, sw);
         if (e != cudaSuccess) return (int)e;
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&cfg.occ_wave, fw, TILE_THREADS, sw);
         if (e != cudaSuccess) return (int)e;
