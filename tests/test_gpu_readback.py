@@ -68,3 +68,24 @@ def test_planes_read_in_parts(nx, ny, precision):
         assert np.array_equal(s.field("h"), a if precision == FP64 else a.astype(np.float32).astype(np.float64))
         s.write_field("z", a)
         assert np.array_equal(s.field("z"), a)
+
+
+def test_small_reads_do_not_wait_for_another_threads_large_ones():
+    """While one thread reads a 256 MB plane over and over, another reads a
+    64 x 64 one: thousands of times, not once between two of the large reads."""
+    import threading
+    from swehr_b200.lib import Simulation
+    large = W.tiny_case(nx=4096, ny=8192, S=1, per_cell_ks=False)
+    small = W.tiny_case(nx=64, ny=64, S=1, per_cell_ks=False)
+    a = np.random.default_rng(1).uniform(0.0, 1.0, (64, 64))
+    reads = 0
+    with Simulation(large) as big, Simulation(small) as s:
+        s.write_field("h", a)
+        big.field("h")
+        t = threading.Thread(target=lambda: [big.field("h") for _ in range(8)])
+        t.start()
+        while t.is_alive():
+            assert np.array_equal(s.field("h"), a)
+            reads += 1
+        t.join()
+    assert reads > 100
