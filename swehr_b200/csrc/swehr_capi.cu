@@ -258,7 +258,7 @@ static void make_devparams(const swehr_params *p, const swehr_inputs *in, const 
     }
     {
         auto in_range = [](double c) { return c >= 0x1p-100 && c <= 0x1p100; };
-        bool ok = P.divk_ok && in_range(P.g) && in_range(P.rhos) && in_range(P.rhow) && in_range(P.h0) && P.F >= 0 &&
+        bool ok = P.divk_ok && P.rhos <= 0x1p50 && P.porod <= 0x1p50 && in_range(P.g) && in_range(P.rhos) && in_range(P.rhow) && in_range(P.h0) && P.F >= 0 &&
                   P.F <= 0x1p100;
         for (int k = 0; k < p->sclass; k++)
             ok = ok && in_range(P.a13sq[k]) && in_range(P.ds[k]) && P.c109s >= 0 && P.c109s <= 0x1p100;

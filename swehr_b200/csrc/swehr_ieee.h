@@ -81,6 +81,21 @@ SW_HD double sw_quot(double a, double b, double y)
     return fma(r, y, q);
 }
 
+/* the same for any dividend below 2^501, a subnormal result included, and b in
+ * [2^-200, 2^52): the quotient of a 2^400, which lies in the normal range, is scaled
+ * back, which rounds a second time where the result is subnormal (last place
+ * 2^-1074, 2^-674 scaled).  The remainder there, a multiple of ulp(b) 2^-674
+ * below b 2^-674, is exact and says whether the nearest place is the next one; a
+ * tie is one of the first quotient too, rounded to even by the scaling. */
+SW_HD double sw_quot_tiny(double a, double b, double y)
+{
+    const double s = a * 0x1p400;
+    double q = sw_quot(s, b, y) * 0x1p-400;
+    const double r = fma(-b, q * 0x1p400, s);
+    if (fabs(q) < 0x1p-1022 && fabs(r) > b * 0x1p-675) q += copysign(0x1p-1074, r);
+    return q;
+}
+
 /* sqrt(x) from an estimate y within 2^-18 of 1/sqrt(x), relatively; x > 0 of
  * middling size */
 SW_HD double sw_sqrt_refine(double x, double y)
@@ -139,6 +154,26 @@ SW_HD bool sw_mid_or_zero(double x)
     return ((fabsf(sw_hi_float(x)) >= __int_as_float(SW_MID_LO)) | sw_zero(x)) & sw_small(x);
 }
 
+/* A dividend may be as small as 2^-860 over a divisor below 2^52: the quotient
+ * is above 2^-913, its remainder a multiple of 2^-965, and the same holds once
+ * more for that quotient over a constant below 2^50.  What suspended mass
+ * settles to after the rain lies below that too (sw_tiny), down to the smallest
+ * subnormals, where a decay by less than a half rounds to no decay at all. */
+#define SW_LOW 0x0A300000
+#define SW_DEPTH_LO 0x33700000
+#define SW_DEPTH_HI 0x43300000
+SW_HD bool sw_tiny(double x) { return sw_below(x, SW_LOW) & !sw_zero(x); }
+SW_HD bool sw_low_or_zero(double x)
+{
+    return ((fabsf(sw_hi_float(x)) >= __int_as_float(SW_LOW)) | sw_zero(x)) & sw_small(x);
+}
+/* a divisor in [2^-200, 2^52) */
+SW_HD bool sw_mid_depth(double x)
+{
+    const float f = sw_hi_float(x);
+    return (f >= __int_as_float(SW_DEPTH_LO)) & (f < __int_as_float(SW_DEPTH_HI));
+}
+
 /* The polynomials' coefficients in the constant bank: a multiply-add takes its
  * operand from there, while an immediate double is moved into a register pair
  * at every use (4096^2, ponded flow: FP64 update -0.7 %). */
@@ -171,6 +206,10 @@ SW_HD double sw_exp_mid(double x, double xlo)
 
 /* |x| <= 700 (false for a NaN) */
 SW_HD bool sw_exp_fits(double x) { return sw_below(x, 0x4085E000); }
+
+/* x below -746 (by 2^-10 or more: the high word decides), where exp rounds to
+ * zero */
+SW_HD bool sw_exp_gone(double x) { return sw_hi_float(x) < __int_as_float(0xC0875000); }
 
 /* sw_pow's general case for middling x > 0 (sw_log_dd, then exp of y log x),
  * its two quotients by the same divisor in [2, 4) sharing a reciprocal; *ok

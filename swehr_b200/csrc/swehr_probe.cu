@@ -71,7 +71,8 @@ extern "C" int swehr_probe_fp64_peak(double *tflops)
 /* swehr_probe_ieee: the branch-free sequences of swehr_ieee.h beside the
  * compiler's operators and the plain bodies of swehr_math.h, element by
  * element, for the tests.  op: 0 a/b, 1 root of a, 2 exp(a), 3 a^b, 4
- * cos(atan a); host arrays of n doubles.  refused: 1 where the operands are
+ * cos(atan a), 5 a/b of small a, 6 a/b of any small a, 7 exp(a) down to zero;
+ * host arrays of n doubles.  refused: 1 where the operands are
  * not ones the sequences take. */
 __global__ void k_ieee(int op, const double *__restrict__ a, const double *__restrict__ b, long long n, double *fast,
                        double *plain, double *refused)
@@ -84,7 +85,10 @@ __global__ void k_ieee(int op, const double *__restrict__ a, const double *__res
         case 1: fast[q] = sw_sqrt_mid(x); plain[q] = sw_sqrt_pow(x); ok = sw_mid_pos(x) || sw_zero(x); break;
         case 2: fast[q] = sw_exp_mid(x, 0.0); plain[q] = sw_exp(x); ok = sw_exp_fits(x); break;
         case 3: fast[q] = sw_pow_mid(x, y, &ok); plain[q] = sw_pow(x, y); break;
-        default: fast[q] = sw_cos_atan_mid(x, &ok); plain[q] = sw_cos_atan(x); break;
+        case 4: fast[q] = sw_cos_atan_mid(x, &ok); plain[q] = sw_cos_atan(x); break;
+        case 5: fast[q] = sw_quot(x, y, sw_rcp(y)); plain[q] = x / y; ok = sw_low_or_zero(x) && sw_mid_depth(y); break;
+        case 6: fast[q] = sw_quot_tiny(x, y, sw_rcp(y)); plain[q] = x / y; ok = sw_small(x) && sw_mid_depth(y); break;
+        default: fast[q] = sw_exp_gone(x) ? 0.0 : sw_exp_mid(x, 0.0); plain[q] = sw_exp(x); ok = sw_exp_gone(x); break;
         }
         refused[q] = !ok;
     }
@@ -93,7 +97,7 @@ __global__ void k_ieee(int op, const double *__restrict__ a, const double *__res
 extern "C" int swehr_probe_ieee(int op, const double *a, const double *b, long long n, double *fast, double *plain,
                                 double *refused)
 {
-    if (!a || !b || !fast || !plain || !refused || n < 1 || op < 0 || op > 4) return 1;
+    if (!a || !b || !fast || !plain || !refused || n < 1 || op < 0 || op > 7) return 1;
     const size_t bytes = (size_t)n * sizeof(double);
     double *d = nullptr;
     if (cudaMalloc(&d, 5 * bytes) != cudaSuccess) return 2;

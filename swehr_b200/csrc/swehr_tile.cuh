@@ -87,6 +87,10 @@ struct PolicyF64 {
     static __device__ __forceinline__ R quot(R a, R b) { return a / b; }
     static __device__ __forceinline__ R quotz(R a, R b) { return divz(a, b); }
     static __device__ __forceinline__ R quotn(R a, R b) { return divz(a, b); }
+    static __device__ __forceinline__ R quotu(R a, R b) { return divz(a, b); }
+    static __device__ __forceinline__ void shallow(R, R) {}
+    template <bool SUMMED>
+    static __device__ __forceinline__ R bulking(R a, R c, R yc, int ok) { return divk(a, c, yc, ok); }
     static __device__ __forceinline__ R root1(R x) { return sw_sqrt_pow(x); }
     static __device__ __forceinline__ R quot_in(R a, R b) { return a / b; }
     static __device__ __forceinline__ R divk_in(R a, R c, R yc, int ok) { return divk(a, c, yc, ok); }
@@ -100,6 +104,7 @@ struct PolicyF64 {
     static __device__ __forceinline__ R sqrtp(R x) { return sw_sqrt_pow(x); }
     static __device__ __forceinline__ R pow(R x, R y) { return sw_pow(x, y); }
     static __device__ __forceinline__ R exp(R x) { return sw_exp(x); }
+    static __device__ __forceinline__ R exp_any(R x) { return sw_exp(x); }
     static __device__ __forceinline__ R cos_atan(R x) { return sw_cos_atan(x); }
     static __device__ __forceinline__ R sin_atan(R x) { return sw_sin_atan(x); }
     static __device__ __forceinline__ R div(R a, R b) { return a / b; }
@@ -179,9 +184,14 @@ struct PolicyF64 {
  * compiler interleaves a cell's independent quotients, roots and exponentials
  * and quotients by one divisor share its reciprocal.  ok is cleared by an
  * operand outside [2^-300, 2^301) that is not a zero dividend or radicand, a
- * divisor that is not positive, an exponent beyond 700 or a NaN; the caller
- * then computes again with PolicyF64.  Constants need no test here:
- * DevParams::fast_ok says that the run's are in range (ok starts as it). */
+ * divisor that is not positive, an exponent above 700 or where exp is subnormal,
+ * or a NaN; the caller then computes again with PolicyF64.  Suspended and
+ * deposited mass may be smaller: quotients of U_k below 2^-860 set tiny, and the
+ * caller forms just those again (200 x 50 hillslope after its rain, when two
+ * thirds of the warps hold such a U_k: 69 us a step with the cells formed again,
+ * 32 with those quotients, 30 in the rain).  Constants
+ * need no test here: DevParams::fast_ok says that the run's are in range (ok
+ * starts as it). */
 struct FastF64 {
     typedef double R;
     typedef FastF64 Fast;
@@ -191,7 +201,7 @@ struct FastF64 {
      * bodies would not fit the instruction cache */
     static constexpr bool kRollClasses = false;
     static constexpr bool kKnownResults = true;
-    bool ok;
+    bool ok = true, tiny = false;
     struct Recip {
         R b, y;
     };
@@ -209,11 +219,34 @@ struct FastF64 {
         ok &= sw_mid_pos(r.b) & (sw_mid_or_zero(a) | (a != a));
         return sw_quot(a, r.b, r.y);
     }
+    /* U_k / h, wrong where it sets tiny */
+    __device__ __forceinline__ R quotu(R a, const Recip &r)
+    {
+        ok &= sw_mid_depth(r.b) & sw_small(a);
+        tiny |= sw_tiny(a);
+        return sw_quot(a, r.b, r.y);
+    }
     __device__ __forceinline__ R div(R a, R b) { return quot(a, recip(b)); }
     __device__ __forceinline__ R divz(R a, R b) { return div(a, b); }
     __device__ __forceinline__ R divk(R a, R c, R yc, int)
     {
         ok &= sw_mid_or_zero(a);
+        return sw_quot(a, c, yc);
+    }
+    /* (u - chtemp) / c, to be added to h: below 2^-860 it is less than 2^-760 and
+     * changes no h of middling size, so its bits do not matter there unless it is
+     * SUMMED on its own, for the budget.  The deep branch has tested h as a
+     * divisor; in the shallow one u is 0 and chtemp an earlier class's */
+    __device__ __forceinline__ void shallow(R chtemp, R h) { ok &= !sw_tiny(chtemp) | sw_mid_pos(h); }
+    template <bool SUMMED>
+    __device__ __forceinline__ R bulking(R a, R c, R yc, int)
+    {
+        if constexpr (SUMMED) {
+            ok &= sw_small(a);
+            if (sw_tiny(a)) return sw_quot_tiny(a, c, yc);
+        } else {
+            ok &= sw_small(a);
+        }
         return sw_quot(a, c, yc);
     }
     /* a dividend that is in range with what has been tested: a quotient of
@@ -250,9 +283,13 @@ struct FastF64 {
     }
     __device__ __forceinline__ R exp(R x)
     {
-        ok &= sw_exp_fits(x);
-        return sw_exp_mid(x, 0.0);
+        const bool gone = sw_exp_gone(x);
+        ok &= sw_exp_fits(x) | gone;
+        const R y = sw_exp_mid(x, 0.0);
+        return gone ? R(0) : y;
     }
+    /* once a cell, and in a storm's wake far below -700 */
+    __device__ __forceinline__ R exp_any(R x) { return PolicyF64::exp(x); }
     __device__ __forceinline__ R cos_atan(R x)
     {
         return sw_cos_atan_mid(x, &ok);
@@ -279,7 +316,7 @@ struct FastF64 {
     static __device__ __forceinline__ R settle(R A, R A2, R c) { return sw_sqrt_pos(A2 + c) - A; }
     __device__ __forceinline__ double dep_of(double M, const DevParams &P)
     {
-        ok &= sw_mid_or_zero(M) | (M != M);
+        ok &= sw_low_or_zero(M) | (M != M);
         return sw_quot(M, P.rhos, P.inv_rhos);
     }
 };
@@ -374,6 +411,7 @@ struct PolicyF32 {
         return powf(x, y);
     }
     static __device__ __forceinline__ R exp(R x) { return exp2(__fmul_rn(x, 1.4426950408889634f)); }
+    static __device__ __forceinline__ R exp_any(R x) { return exp(x); }
     static __device__ __forceinline__ R cos_atan(R x) { return rsqrt(1.f + x * x); }
     static __device__ __forceinline__ R sin_atan(R x) { return x * rsqrt(1.f + x * x); }
     typedef R Recip;                                /* the reciprocal */
@@ -381,6 +419,10 @@ struct PolicyF32 {
     static __device__ __forceinline__ R quot(R a, R y) { return __fmul_rn(a, y); }
     static __device__ __forceinline__ R quotz(R a, R y) { return quot(a, y); }
     static __device__ __forceinline__ R quotn(R a, R y) { return quot(a, y); }
+    static __device__ __forceinline__ R quotu(R a, R y) { return quot(a, y); }
+    static __device__ __forceinline__ void shallow(R, R) {}
+    template <bool SUMMED>
+    static __device__ __forceinline__ R bulking(R a, R c, R yc, int ok) { return divk(a, c, yc, ok); }
     static __device__ __forceinline__ R div(R a, R b) { return quot(a, rcp(b)); }
     static __device__ __forceinline__ R divz(R a, R b) { return div(a, b); }
     static __device__ __forceinline__ R sqrtz(R x) { return sqrtp(x); }
@@ -402,8 +444,9 @@ struct PolicyF32 {
 template <class F>
 __device__ __forceinline__ F make_fast(const DevParams &P)
 {
-    if constexpr (F::kGuarded) return F{P.fast_ok != 0};
-    else return F{};
+    F pp;
+    if constexpr (F::kGuarded) pp.ok = P.fast_ok != 0;
+    return pp;
 }
 
 /* hllc of SWEHR.c:327-409 with the velocities already formed
@@ -869,10 +912,10 @@ __device__ __forceinline__ void stage_derive(const DevParams &P, const DevParams
         const RS *U = halo + HP_U * L.hps + so;
         if constexpr (NS > 0) {
 #pragma unroll
-            for (int k = 0; k < NS; k++) sed_k(k, flow ? pp.quot((R)U[k * L.hps], rh) : R(0));
+            for (int k = 0; k < NS; k++) sed_k(k, flow ? pp.quotu((R)U[k * L.hps], rh) : R(0));
         } else {
 #pragma unroll 4
-            for (int k = 0; k < S; k++) sed_k(k, flow ? pp.quot((R)U[k * L.hps], rh) : R(0));
+            for (int k = 0; k < S; k++) sed_k(k, flow ? pp.quotu((R)U[k * L.hps], rh) : R(0));
         }
         const R g = (R)halo[HP_GZ * L.hps + so];
         R c = pp.sqrtp(g * h);
@@ -884,6 +927,12 @@ __device__ __forceinline__ void stage_derive(const DevParams &P, const DevParams
 #pragma unroll 1
                 for (int k = 0; k < S; k++) sed_k(k, flow ? Q::div((R)U[k * L.hps], h) : R(0));
                 c = Q::sqrtp(g * h);
+            } else if (pp.tiny) {
+#pragma unroll 1
+                for (int k = 0; k < S; k++) {
+                    const R Uk = (R)U[k * L.hps];
+                    if (sw_tiny(Uk)) sed_k(k, sw_quot_tiny(Uk, rh.b, rh.y));
+                }
             }
         }
         su[idx] = u;
@@ -1379,7 +1428,7 @@ __device__ __forceinline__ typename PP::R storm_r(PP &pp, const DevParams &P, do
     const double x = ((double)(i + P.row0) - 0.5) * P.dx - (P.storm_x0 + P.storm_vx * t);
     const double y = ((double)j - 0.5) * P.dx - (P.storm_y0 + P.storm_vy * t);
     const double r2 = (x * x + y * y) / P.storm_r2;
-    return (R)P.storm_peak * pp.exp(R(-0.5 * r2));
+    return (R)P.storm_peak * pp.exp_any(R(-0.5 * r2));
 }
 
 /* A solid cell in the update (SWEHR.c:1421 false branch, 1566-1574): no
@@ -1414,6 +1463,30 @@ __device__ __forceinline__ void solid_cell(const DevParams &P, const SetV<RS> &s
     dst.totsed[q] = src.totsed[q];
     dst.gz[q] = src.gz[q];
     zn[q] = zc[q];
+}
+
+/* TOTSED of a cell some of whose U_k (k-th at U[k stride]) are below 2^-860, sum
+ * being their sum with the wrong quotients of those.  They only matter where
+ * nothing much larger is added: with no negative U_k, one of 2^-796 or more and
+ * none in between, every partial sum of the tiny ones, at most 16 of them and
+ * 2^60 times smaller, is lost in the rounding of the large, whatever its bits. */
+static __device__ __noinline__ double totsed_tiny(const double *U, int stride, int S, double h, double y, double rhos,
+                                           double inv_rhos, double sum)
+{
+    const int large = SW_LOW + (64 << 20);
+    bool between = false;
+    int top = 0;
+#pragma unroll 4
+    for (int k = 0; k < S; k++) {
+        const int hi = __double2hiint(U[k * stride]);
+        between |= hi < 0 || (hi >= SW_LOW && hi < large);
+        top = max(top, hi);
+    }
+    if (!between && top >= large) return sum;
+    sum = 0;
+#pragma unroll 4
+    for (int k = 0; k < S; k++) sum += sw_quot_tiny(sw_quot_tiny(U[k * stride], h, y), rhos, inv_rhos);
+    return sum;
 }
 
 /* One cell of the tile with the arithmetic PP.  FRESH: U_k and M_k are read
@@ -1634,6 +1707,7 @@ __device__ __forceinline__ void tile_cell_pp(PP &pp, const DevParams &P, const D
         if (h < K.hfx10) {
             Mk += (double)(dtr * E1 + u);
             u = 0;
+            pp.shallow(chtemp, h);
             if (BUDGET) det_k = (double)(dtr * E1);
         } else {
             R E2 = 0, E3 = 0, E4 = 0, VF = 0;
@@ -1669,7 +1743,7 @@ __device__ __forceinline__ void tile_cell_pp(PP &pp, const DevParams &P, const D
                 dep = 0;
             }
         }
-        const R dh = pp.divk(u - chtemp, K.porod, (R)C.invporo, C.divk_ok);
+        const R dh = pp.template bulking<BUDGET>(u - chtemp, K.porod, (R)C.invporo, C.divk_ok);
         h = h + dh;
         bulk += dh;
         totm += Mk;
@@ -1701,10 +1775,21 @@ __device__ __forceinline__ void tile_cell_pp(PP &pp, const DevParams &P, const D
         for (int k = 0; k < MAXS; k++) {
             if (k >= S) break;
             const R uk = kSlot ? (R)Uslot[k * hps] : Ureg[kSlot ? 0 : k];
-            totsed += pp.divk_in(pp.quotz(uk, rh), rhos, (R)C.inv_rhos, C.divk_ok);
+            totsed += pp.divk_in(pp.quotu(uk, rh), rhos, (R)C.inv_rhos, C.divk_ok);
             dst.U[k * pl + q] = (RS)uk;
             if (stage_m) dst.M[k * pl + q] = celld[(CD_M + k) * T_I * T_J + cs];
         }
+        if constexpr (PP::kGuarded)
+            if (pp.tiny) {
+                if constexpr (!kSlot) {
+#pragma unroll
+                    for (int k = 0; k < MAXS; k++) {
+                        if (k >= S) break;
+                        Uslot[k * hps] = Ureg[kSlot ? 0 : k];
+                    }
+                }
+                totsed = totsed_tiny(Uslot, hps, S, rh.b, rh.y, rhos, C.inv_rhos, totsed);
+            }
     } else {
         clamp = hfilm - h;
         h = hfilm;
