@@ -32,6 +32,8 @@ SOURCES = [
     ("swehr_batch16_f64.cu", ["--fmad=false"]),
     ("swehr_batch16_f32.cu", []),
     ("swehr_slab.cu", ["--fmad=false"]),
+    ("swehr_wide_f64.cu", ["--fmad=false"]),
+    ("swehr_wide16_f64.cu", ["--fmad=false"]),
 ]
 
 

@@ -79,7 +79,20 @@ struct BatchConfig {
         int occ_x[17] = {};
     };
     Update own, common;
+    /* both passes' kernels for pools with a scenario whose constants are out of
+     * the ordinary kernels' range */
+    Update wide;
+    void *fn_wave_wide = nullptr;
+    int occ_wave_wide = 1;
 };
+
+/* The kernels of runs whose constants are out of the ordinary kernels' range
+ * (Policy::Wide), for any class count: update[tensor maps][budgets] */
+struct WideKernels {
+    void *wave, *update[2][2], *wave_batch, *update_batch[2];
+};
+WideKernels wide_kernels_f64();
+WideKernels wide_kernels_f64_t16();
 
 int configure_batch_f64(int max_classes, bool budget, BatchConfig &cfg);
 int configure_batch_f32(int max_classes, bool budget, BatchConfig &cfg);

@@ -218,7 +218,22 @@ struct FormLauncher {
         return budget ? pick_budget<SM>(S) : update_fn<16, false, SM, true>();
     }
 
-    static int configure(const DevParams &P, int num_sms, StepConfig &cfg)
+    /* Policy::Wide's kernels (one instantiation, in a translation unit of its
+     * own); M_k stays in global memory */
+    static WideKernels wide_kernels()
+    {
+        typedef typename PP::Wide W;
+        return WideKernels{(void *)k_wave_cells<W, RS>,
+                           {{(void *)k_update_tile<W, RS, 16, false, false, false, 0>,
+                             (void *)k_update_tile<W, RS, 16, true, false, false, 0>},
+                            {(void *)k_update_tile<W, RS, 16, false, false, true, 0>,
+                             (void *)k_update_tile<W, RS, 16, true, false, true, 0>}},
+                           (void *)k_wave_batch<W, RS>,
+                           {(void *)k_update_batch<W, RS, 16, false, false, 0, false>,
+                            (void *)k_update_batch<W, RS, 16, true, false, 0, false>}};
+    }
+
+    static int configure(const DevParams &P, int num_sms, StepConfig &cfg, const WideKernels &wide)
     {
         const int64_t ntiles = (int64_t)((P.nx + T_I - 1) / T_I) * ((P.ny + T_J - 1) / T_J);
         void *fu = nullptr;
@@ -226,13 +241,22 @@ struct FormLauncher {
         size_t su = 0;
         const size_t sw = wave_smem();
         int occ_u = 0, occ_w = 0, stage_m = 1;
+        const bool ordinary = PP::ordinary(P);
         const bool tma = cfg.tma != 0;
         cfg.tma = tma ? 1 : 0;
-        const Exact x = tma && !P.budget ? exact(P.S) : Exact();
-        void *fr = x.run;
+        const Exact x = ordinary && tma && !P.budget ? exact(P.S) : Exact();
+        void *fr = nullptr;                    /* the many-step kernel of fu's layout */
         cudaError_t e;
-        if (x.update) {
+        if (!ordinary) {
+            fu = wide.update[tma][P.budget != 0];
+            fw = wide.wave;
+            stage_m = 0;
+            su = update_smem(P.S, 0) + (tma ? 128 : 0);
+            e = raise_smem_limit(fu, su);
+            if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_u, fu, TILE_THREADS, su);
+        } else if (x.update) {
             fu = x.update;
+            fr = x.run;
             stage_m = x.stage_m;
             su = update_smem(P.S, stage_m) + 128;
             e = raise_smem_limit(fu, su);
@@ -331,7 +355,25 @@ struct FormLauncher {
         return e;
     }
 
-    static int configure_batch(int max_classes, bool budget, BatchConfig &cfg)
+    static cudaError_t configure_wide(int max_classes, bool budget, BatchConfig &cfg, const WideKernels &wide)
+    {
+        void *f = wide.update_batch[budget];
+        cudaError_t e = raise_smem_limit(f, update_smem(max_classes, 0));
+        for (int S = 0; S <= 16 && e == cudaSuccess; S++) {
+            BatchConfig::Update &u = cfg.wide;
+            u.fn_s[S] = f;
+            u.smem_s[S] = update_smem(S < 1 ? 1 : (S > max_classes ? max_classes : S), 0);
+            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&u.occ_s[S], f, TILE_THREADS, u.smem_s[S]);
+            if (u.occ_s[S] < 1) u.occ_s[S] = 1;
+        }
+        cfg.fn_wave_wide = wide.wave_batch;
+        if (e == cudaSuccess)
+            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&cfg.occ_wave_wide, wide.wave_batch, TILE_THREADS, wave_smem());
+        if (cfg.occ_wave_wide < 1) cfg.occ_wave_wide = 1;
+        return e;
+    }
+
+    static int configure_batch(int max_classes, bool budget, BatchConfig &cfg, const WideKernels &wide)
     {
         void *fw = (void *)k_wave_batch<PP, RS>;
         const size_t sw = wave_smem();
@@ -342,6 +384,7 @@ struct FormLauncher {
         if (cfg.occ_wave < 1) cfg.occ_wave = 1;
         e = configure_updates<false>(max_classes, budget, cfg.own);
         if (e == cudaSuccess && !budget) e = configure_updates<true>(max_classes, budget, cfg.common);
+        if (e == cudaSuccess && wide.wave_batch) e = configure_wide(max_classes, budget, cfg, wide);
         if (e != cudaSuccess) return (int)e;
         cfg.fn_wave = fw;
         cfg.smem_wave = sw;

@@ -66,6 +66,7 @@ struct swehr_pool {
     DevParams common = {};
     bool has_common = false;
     int common_id = 0;
+    bool has_wide = false;               /* a running scenario's constants are out of the ordinary kernels' range */
     cudaStream_t stream = nullptr;
     struct GraphEntry {
         size_t smem;
@@ -245,9 +246,10 @@ static int rebuild_table(swehr_pool *pl)
     int k = 0, max_s = 1, min_s = 16;
     int64_t tile0 = 0, cells = 0;
     DevParams first;
-    bool same = pl->budget == 0;
+    bool same = pl->budget == 0, wide = false;
     for (auto &s : pl->scen) {
         if (!s.running) continue;
+        wide |= !swehr_ctx_ordinary(s.ctx);
         if (k == 0) first = common_constants(s.ctx->P);
         else if (same) {
             const DevParams c = common_constants(s.ctx->P);
@@ -307,7 +309,8 @@ static int rebuild_table(swehr_pool *pl)
     pl->running_cells = cells;
     pl->max_s = max_s;
     pl->min_s = std::min(min_s, max_s);
-    pl->has_common = same && k > 0;
+    pl->has_wide = wide;
+    pl->has_common = same && k > 0 && !wide;
     if (pl->has_common && (pl->common_id == 0 || memcmp(&first, &pl->common, sizeof first) != 0)) {
         /* other constants than the graphs hold: those are never launched again */
         for (auto it = pl->graphs.begin(); it != pl->graphs.end();) {
@@ -329,7 +332,7 @@ static void launch_pool_step(swehr_pool *pl, cudaEvent_t e0, cudaEvent_t e1, cud
 {
     void *args[] = {(void *)&pl->d_hdr, (void *)&pl->common};
     if (e0) cudaEventRecord(e0, pl->stream);
-    cudaLaunchKernel(pl->cfg.fn_wave, dim3(pl->grid_wave), dim3(pl->cfg.threads), args, pl->cfg.smem_wave, pl->stream);
+    cudaLaunchKernel(pl->has_wide ? pl->cfg.fn_wave_wide : pl->cfg.fn_wave, dim3(pl->grid_wave), dim3(pl->cfg.threads), args, pl->cfg.smem_wave, pl->stream);
     if (e1) cudaEventRecord(e1, pl->stream);
     cudaLaunchKernel(pl->fn_update, dim3(pl->grid_update), dim3(pl->cfg.threads), args, pl->smem_update, pl->stream);
     if (e2) cudaEventRecord(e2, pl->stream);
@@ -373,7 +376,12 @@ static void set_grids(swehr_pool *pl, int kw, int ku)
  * occupancy */
 static const BatchConfig::Update &updates(const swehr_pool *pl, const BatchConfig &c)
 {
-    return pl->has_common ? c.common : c.own;
+    return pl->has_wide ? c.wide : pl->has_common ? c.common : c.own;
+}
+
+static int wave_occupancy(const swehr_pool *pl, const BatchConfig &c)
+{
+    return pl->has_wide ? c.occ_wave_wide : c.occ_wave;
 }
 
 /* the running scenarios all have the class count of a kernel built for
@@ -398,7 +406,7 @@ static void apply_shape(swehr_pool *pl)
     pl->fn_update = exact ? u.fn_x[S] : u.fn_s[S];
     const int occ_u = update_occupancy(pl, pl->cfg);
     const int ku = pl->ku_sel ? std::min(pl->ku_sel, occ_u) : occ_u;
-    const int kw = pl->kw_sel ? pl->kw_sel : pl->cfg.occ_wave;
+    const int kw = pl->kw_sel ? pl->kw_sel : wave_occupancy(pl, pl->cfg);
     set_grids(pl, kw, ku);
 }
 
@@ -653,7 +661,7 @@ int swehr_pool_tune(swehr_pool *pl, int64_t steps_per_trial, swehr_pool_stats *s
     std::vector<std::pair<int, int>> cand;
     for (int sh = 0; sh < nsh; sh++) {
         occ_u[sh] = update_occupancy(pl, pl->shapes[sh]);
-        trials[sh] = std::max(pl->shapes[sh].occ_wave, occ_u[sh]);
+        trials[sh] = std::max(wave_occupancy(pl, pl->shapes[sh]), occ_u[sh]);
         for (int k = 1; k <= trials[sh]; k++) cand.push_back({sh, k});
     }
     std::vector<double> bw[2], bu[2];
@@ -675,7 +683,7 @@ int swehr_pool_tune(swehr_pool *pl, int64_t steps_per_trial, swehr_pool_stats *s
             if (rc) return rc;
         }
         if (pl->nrun == 0) break;
-        const int kw = std::min(k, pl->cfg.occ_wave), ku = std::min(k, occ_u[sh]);
+        const int kw = std::min(k, wave_occupancy(pl, pl->cfg)), ku = std::min(k, occ_u[sh]);
         set_grids(pl, kw, ku);
         const double cells = (double)std::max<int64_t>(pl->running_cells, 1);
         for (int64_t s = 0; s < steps_per_trial; s++)
@@ -699,7 +707,7 @@ int swehr_pool_tune(swehr_pool *pl, int64_t steps_per_trial, swehr_pool_stats *s
     int best_sh = 0, kw_best[2], ku_best[2];
     double best_t = INFINITY;
     for (int sh = 0; sh < nsh; sh++) {
-        kw_best[sh] = pl->shapes[sh].occ_wave;
+        kw_best[sh] = std::min(trials[sh], wave_occupancy(pl, pl->shapes[sh]));
         ku_best[sh] = occ_u[sh];
         for (int k = 1; k <= trials[sh]; k++) {
             if (bw[sh][k] < bw[sh][kw_best[sh]]) kw_best[sh] = k;

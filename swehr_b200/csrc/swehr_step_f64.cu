@@ -26,7 +26,7 @@ namespace swehr {
 
 int configure_step_f64(const DevParams &P, int num_sms, StepConfig &cfg)
 {
-    return FormLauncher<PolicyF64, double>::configure(P, num_sms, cfg);
+    return FormLauncher<PolicyF64, double>::configure(P, num_sms, cfg, wide_kernels_f64());
 }
 
 int launch_wave_f64(const DevParams &P, const BufsT<double> &B, Ctl *ctl, const StepConfig &cfg, cudaStream_t s)
@@ -66,7 +66,7 @@ int encode_tma_f64(const DevParams &P, const BufsT<double> &B, TmaMaps &tm)
 
 int configure_batch_f64(int max_classes, bool budget, BatchConfig &cfg)
 {
-    return FormLauncher<PolicyF64, double>::configure_batch(max_classes, budget, cfg);
+    return FormLauncher<PolicyF64, double>::configure_batch(max_classes, budget, cfg, wide_kernels_f64());
 }
 
 }  // namespace swehr

@@ -69,12 +69,17 @@ inline namespace SWEHR_TILE_NS {
  * forms' kernels; Fast is the arithmetic their cells, faces and wave speeds
  * run on.  Fast of the plain form collects in ok whether every operand was
  * one its branch-free sequences are exact for; where it was not, the caller
- * computes the cell (face, vector) again with Plain. */
+ * computes the cell (face, vector) again with Plain.  Wide is the arithmetic of
+ * runs whose constants are out of the range that Fast takes untested
+ * (ordinary); they have kernels of their own (swehr_wide_*.cu). */
 struct FastF64;
+struct WideF64;
 struct PolicyF64 {
     typedef double R;
     typedef FastF64 Fast;
     typedef PolicyF64 Plain;
+    typedef WideF64 Wide;
+    __host__ __device__ static bool ordinary(const DevParams &P) { return P.fast_ok != 0; }
     static constexpr bool kGuarded = false;
     static constexpr bool ok = true;
     static constexpr int kMinBlocks = 2;      /* CTAs per SM the update kernel is register-budgeted for */
@@ -190,8 +195,7 @@ struct PolicyF64 {
  * caller forms just those again (200 x 50 hillslope after its rain, when two
  * thirds of the warps hold such a U_k: 69 us a step with the cells formed again,
  * 32 with those quotients, 30 in the rain).  Constants
- * need no test here: DevParams::fast_ok says that the run's are in range (ok
- * starts as it). */
+ * need no test here: DevParams::fast_ok says that the run's are in range. */
 struct FastF64 {
     typedef double R;
     typedef FastF64 Fast;
@@ -321,8 +325,15 @@ struct FastF64 {
     }
 };
 
+/* every cell with the plain operators, once */
+struct WideF64 : PolicyF64 {
+    typedef WideF64 Fast;
+    typedef WideF64 Plain;
+};
+
 struct PolicyF32 {
     typedef float R;
+    __host__ __device__ static bool ordinary(const DevParams &) { return true; }
     typedef PolicyF32 Fast;
     typedef PolicyF32 Plain;
     static constexpr bool kGuarded = false;
@@ -439,15 +450,6 @@ struct PolicyF32 {
     /* DEP is stored in FP32 here: a reciprocal multiply is exact enough */
     static __device__ __forceinline__ double dep_of(double M, const DevParams &P) { return M * P.inv_rhos; }
 };
-
-/* the arithmetic of a routine that recomputes with Plain where it has to */
-template <class F>
-__device__ __forceinline__ F make_fast(const DevParams &P)
-{
-    F pp;
-    if constexpr (F::kGuarded) pp.ok = P.fast_ok != 0;
-    return pp;
-}
 
 /* hllc of SWEHR.c:327-409 with the velocities already formed
  * (nl = normal/ul, tl = tangential/vl; both 0 for a dry side) and the left
@@ -889,7 +891,7 @@ __device__ __forceinline__ void stage_derive(const DevParams &P, const DevParams
             if ((gi == 0 && P.bndry[0] == 1) || (gi == P.nx + 1 && P.bndry[2] == 1)) hu = -hu;
             if ((gj == 0 && P.bndry[1] == 1) || (gj == P.ny + 1 && P.bndry[3] == 1)) hv = -hv;
         }
-        F pp = make_fast<F>(C);
+        F pp;
         const bool flow = h > K.hfilm;
         const typename F::Recip rh = F::recip(h);
         R u = 0, v = 0;
@@ -1058,7 +1060,7 @@ __device__ __forceinline__ typename PP::R wave_cell(const DevParams &P, const Se
                                                     const uint8_t *__restrict__ solid)
 {
     typedef typename PP::Fast F;
-    F pp = make_fast<F>(P);
+    F pp;
     /* GZ of the previous step, written by its update */
     const typename PP::R s =
         wave_cell_g<F, RS>(pp, P, src, i, j, inh, inhv, (typename PP::R)src.gz[cidx(P, i, j)], solid);
@@ -1179,7 +1181,7 @@ __device__ __forceinline__ typename PP::R wave_vec_any(const DevParams &P, const
 {
     typedef typename PP::R R;
     typedef typename PP::Fast F;
-    F pp = make_fast<F>(P);
+    F pp;
     R s = wave_vec<F, RS, LIVE>(pp, P, src, i, j0, inh, inhv);
     if constexpr (F::kGuarded)
         if (!pp.ok) {
@@ -1909,7 +1911,7 @@ __device__ __forceinline__ void tile_cell(const DevParams &P, const DevParams &C
     }
     typedef typename PP::Fast F;
     if constexpr (F::kGuarded) {
-        F pp = make_fast<F>(C);
+        F pp;
         Acc2<MAXS, BUDGET> add;
         acc_zero(add);
         tile_cell_pp<F, RS, MAXS, BUDGET, NS, false>(pp, P, C, src, dst, zp, zc, zn, smb, L, tc, t, dt, Rr, add, solid, z0);
@@ -2069,7 +2071,7 @@ __device__ __forceinline__ void update_tile(const DevParams &P, const DevParams 
             yface = true;
         }
         R T0, T1, T2;
-        F pp = make_fast<F>(C);
+        F pp;
         hllc_v<F>(pp, hl, hr, nl, nr, tl, tr, g, cl, K.hfilm, T0, T1, T2);
         if constexpr (F::kGuarded)
             if (!pp.ok) {
