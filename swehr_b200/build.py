@@ -34,6 +34,8 @@ SOURCES = [
     ("swehr_slab.cu", ["--fmad=false"]),
     ("swehr_wide_f64.cu", ["--fmad=false"]),
     ("swehr_wide16_f64.cu", ["--fmad=false"]),
+    ("swehr_wide_f32.cu", []),
+    ("swehr_wide16_f32.cu", []),
 ]
 
 

@@ -14,7 +14,7 @@ namespace swehr {
 
 int configure_batch_f32_t16(int max_classes, bool budget, BatchConfig &cfg)
 {
-    return FormLauncher<PolicyF32, float>::configure_batch(max_classes, budget, cfg, WideKernels());
+    return FormLauncher<PolicyF32, float>::configure_batch(max_classes, budget, cfg, wide_kernels_f32_t16());
 }
 
 }  // namespace swehr

@@ -264,6 +264,17 @@ static void make_devparams(const swehr_params *p, const swehr_inputs *in, const 
             ok = ok && in_range(P.a13sq[k]) && in_range(P.ds[k]) && P.c109s >= 0 && P.c109s <= 0x1p100;
         P.fast_ok = ok;
     }
+    {
+        /* a film and constants that leave every divisor of the mixed form normal:
+         * the smallest are (film)^2.333, (10 film)^3.333 and, for depths below
+         * 2^20, mtstar0 (h0 / depth)^b */
+        auto middling = [](double c) { return c == 0 || (fabs(c) >= 0x1p-100 && fabs(c) <= 0x1p100); };
+        bool ok = P.hfilm >= 0x1p-40 && P.hfilm <= 0x1p40 && middling(P.g * 0x1p70) && middling(P.rhos) && middling(P.J) &&
+                  middling(P.porod) && middling(P.hc) && P.h0 >= 0x1p-30 && P.h0 <= 0x1p97 && P.b <= 2 &&
+                  (P.mtstar0 == 0 || fabs(P.mtstar0) >= 0x1p-20) && middling(P.c109s);
+        for (int k = 0; k < p->sclass; k++) ok = ok && middling(P.a13sq[k]);
+        P.mixed_ok = ok;
+    }
     fill_realc(P, P.kd);
     fill_realc(P, P.kf);
 }

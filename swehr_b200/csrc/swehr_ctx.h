@@ -72,7 +72,7 @@ int swehr_ctx_create(const swehr_params *p, const swehr_inputs *in, int precisio
 size_t swehr_ctx_footprint(const swehr_params *p, int has_ks, int has_solid, int precision, int num_sms);
 
 /* whether the run's constants are in the range of its form's ordinary kernels */
-inline bool swehr_ctx_ordinary(const swehr_ctx *c) { return c->precision == SWEHR_MIXED || c->P.fast_ok; }
+inline bool swehr_ctx_ordinary(const swehr_ctx *c) { return c->precision == SWEHR_MIXED ? c->P.mixed_ok : c->P.fast_ok; }
 
 /* free a context (pools use this for their scenarios) */
 void swehr_ctx_destroy(swehr_ctx *c);

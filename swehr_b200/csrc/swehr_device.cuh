@@ -66,6 +66,8 @@ struct DevParams {
     /* every constant a branch-free sequence takes untested is positive and of
      * middling size (FastF64); 0: the plain operators throughout */
     int32_t fast_ok;
+    /* the mixed form's divisors are normal numbers (FormF32::rcp) */
+    int32_t mixed_ok, pad_ok;
     double storm_peak, storm_r2, storm_x0, storm_y0, storm_vx, storm_vy;
     double ds[16], pf[16], a13[16], a13sq[16];
     RealC<double> kd;     /* the constants above, for templated kernels */

@@ -93,6 +93,8 @@ struct WideKernels {
 };
 WideKernels wide_kernels_f64();
 WideKernels wide_kernels_f64_t16();
+WideKernels wide_kernels_f32();
+WideKernels wide_kernels_f32_t16();
 
 int configure_batch_f64(int max_classes, bool budget, BatchConfig &cfg);
 int configure_batch_f32(int max_classes, bool budget, BatchConfig &cfg);

@@ -384,7 +384,7 @@ struct FormLauncher {
         if (cfg.occ_wave < 1) cfg.occ_wave = 1;
         e = configure_updates<false>(max_classes, budget, cfg.own);
         if (e == cudaSuccess && !budget) e = configure_updates<true>(max_classes, budget, cfg.common);
-        if (e == cudaSuccess && wide.wave_batch) e = configure_wide(max_classes, budget, cfg, wide);
+        if (e == cudaSuccess) e = configure_wide(max_classes, budget, cfg, wide);
         if (e != cudaSuccess) return (int)e;
         cfg.fn_wave = fw;
         cfg.smem_wave = sw;

@@ -11,7 +11,7 @@ namespace swehr {
 
 int configure_step_f32(const DevParams &P, int num_sms, StepConfig &cfg)
 {
-    return FormLauncher<PolicyF32, float>::configure(P, num_sms, cfg, WideKernels());
+    return FormLauncher<PolicyF32, float>::configure(P, num_sms, cfg, wide_kernels_f32());
 }
 
 int launch_wave_f32(const DevParams &P, const BufsT<float> &B, Ctl *ctl, const StepConfig &cfg, cudaStream_t s)
@@ -49,7 +49,7 @@ int encode_tma_f32(const DevParams &P, const BufsT<float> &B, TmaMaps &tm)
 
 int configure_batch_f32(int max_classes, bool budget, BatchConfig &cfg)
 {
-    return FormLauncher<PolicyF32, float>::configure_batch(max_classes, budget, cfg, WideKernels());
+    return FormLauncher<PolicyF32, float>::configure_batch(max_classes, budget, cfg, wide_kernels_f32());
 }
 
 }  // namespace swehr

@@ -127,6 +127,8 @@ struct PolicyF64 {
         if (x == 0) return R(0);
         return sqrtp(x);
     }
+    /* sqrtp of squared momenta and velocities */
+    static __device__ __forceinline__ R sqrtw(R x) { return sqrtz(x); }
     static __device__ __forceinline__ R qnan() { return __longlong_as_double(0x7ff8000000000000LL); }
     /* a / c for a constant divisor c in [2^-100, 2^100] whose correctly
      * rounded reciprocal yc the host computed, without the division
@@ -267,6 +269,7 @@ struct FastF64 {
         return sw_sqrt_mid(x);
     }
     __device__ __forceinline__ R sqrtz(R x) { return sqrtp(x); }
+    __device__ __forceinline__ R sqrtw(R x) { return sqrtp(x); }
     /* root of a sum of squares plus one */
     __device__ __forceinline__ R root1(R x)
     {
@@ -331,11 +334,14 @@ struct WideF64 : PolicyF64 {
     typedef WideF64 Plain;
 };
 
-struct PolicyF32 {
+/* WIDE: also where divisors and radicands may be subnormal (see rcp) */
+template <bool WIDE>
+struct FormF32 {
     typedef float R;
-    __host__ __device__ static bool ordinary(const DevParams &) { return true; }
-    typedef PolicyF32 Fast;
-    typedef PolicyF32 Plain;
+    typedef FormF32 Fast;
+    typedef FormF32 Plain;
+    typedef FormF32<true> Wide;
+    __host__ __device__ static bool ordinary(const DevParams &P) { return P.mixed_ok != 0; }
     static constexpr bool kGuarded = false;
     static constexpr bool ok = true;
     static constexpr int kMinBlocks = 3;
@@ -357,15 +363,14 @@ struct PolicyF32 {
     static constexpr bool kRollClasses = false;
     static constexpr int kWaveMinBlocks = 5;      /* 48 registers: four cells per thread without spills */
     static constexpr bool kKnownResults = false;
-    /* The SFU's functions in the form that takes no denormal operand.  The
-     * other form tests every operand and scales it there and back (two
-     * multiplications and a compare around each of a wet cell's ~100 uses, a
-     * fifth of the mixed update's instructions).  The divisors and radicands
-     * here are depths above the film, sums with one or with such a depth's
-     * wave speed, and constants: normal numbers, for which both forms are the
-     * same.  A quotient keeps a denormal dividend (the reciprocal is what the
-     * SFU computes); roots and powers below 1e-19 and exponentials below 1e-38
-     * come out as (near) zero. */
+    /* The SFU's reciprocals and reciprocal roots are taken in the form without
+     * subnormal operands: the other is 17 % of the mixed update (4096^2, ponded
+     * flow, ~100 uses a wet cell).  The divisors are depths above the film and
+     * their powers, sums with one or with such a depth's wave speed, and constants:
+     * normal numbers where DevParams::mixed_ok says that the film and the constants
+     * are of middling size.  Other runs, such as one without a film, take the WIDE
+     * form's kernels, where a divisor below 2^-100 is scaled with its dividend (the
+     * others are divided the same).  A subnormal dividend is kept in either. */
     static __device__ __forceinline__ R rcp(R b)
     {
         R y;
@@ -378,6 +383,7 @@ struct PolicyF32 {
         asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
         return y;
     }
+    /* for pow's arguments, of which none and no result is subnormal */
     static __device__ __forceinline__ R exp2(R x)
     {
         R y;
@@ -394,8 +400,14 @@ struct PolicyF32 {
      * pow(x, 0.5) of a zero).  The product is rounded on its own (never fused
      * into a later add), so the single-domain and batched kernels compute the
      * same value. */
+    static __device__ __forceinline__ R sqrtw(R x) { return x > 0.f ? __fmul_rn(x, rsqrtf(x)) : 0.f; }
+    /* ... without subnormal operands: a root below 1e-19 comes out nearer to zero.
+     * It is a slope, is added to the root of a film's depth, or goes into a stream
+     * power, its cube, that is zero either way; squared velocities and momenta take
+     * sqrtw (4096^2 in ponded flow: +0.4 %) */
     static __device__ __forceinline__ R sqrtp(R x)
     {
+        if constexpr (WIDE) return sqrtw(x);
         const R c = fmaxf(x, 0.f);
         return __fmul_rn(c, rsqrt(fmaxf(c, 1.17549435e-38f)));
     }
@@ -421,27 +433,33 @@ struct PolicyF32 {
         }
         return powf(x, y);
     }
-    static __device__ __forceinline__ R exp(R x) { return exp2(__fmul_rn(x, 1.4426950408889634f)); }
+    static __device__ __forceinline__ R exp(R x) { return __expf(x); }
     static __device__ __forceinline__ R exp_any(R x) { return exp(x); }
     static __device__ __forceinline__ R cos_atan(R x) { return rsqrt(1.f + x * x); }
     static __device__ __forceinline__ R sin_atan(R x) { return x * rsqrt(1.f + x * x); }
-    typedef R Recip;                                /* the reciprocal */
-    static __device__ __forceinline__ R recip(R b) { return rcp(b); }
-    static __device__ __forceinline__ R quot(R a, R y) { return __fmul_rn(a, y); }
-    static __device__ __forceinline__ R quotz(R a, R y) { return quot(a, y); }
-    static __device__ __forceinline__ R quotn(R a, R y) { return quot(a, y); }
-    static __device__ __forceinline__ R quotu(R a, R y) { return quot(a, y); }
+    struct Recip {
+        R y, s;                                     /* the reciprocal of the divisor times s (WIDE) */
+    };
+    static __device__ __forceinline__ Recip recip(R b)
+    {
+        const R s = WIDE && fabsf(b) < 0x1p-100f ? 0x1p60f : 1.f;
+        return Recip{rcp(WIDE ? b * s : b), s};
+    }
+    static __device__ __forceinline__ R quot(R a, Recip r) { return __fmul_rn(WIDE ? a * r.s : a, r.y); }
+    static __device__ __forceinline__ R quotz(R a, Recip r) { return quot(a, r); }
+    static __device__ __forceinline__ R quotn(R a, Recip r) { return quot(a, r); }
+    static __device__ __forceinline__ R quotu(R a, Recip r) { return quot(a, r); }
     static __device__ __forceinline__ void shallow(R, R) {}
     template <bool SUMMED>
     static __device__ __forceinline__ R bulking(R a, R c, R yc, int ok) { return divk(a, c, yc, ok); }
-    static __device__ __forceinline__ R div(R a, R b) { return quot(a, rcp(b)); }
+    static __device__ __forceinline__ R div(R a, R b) { return quot(a, recip(b)); }
     static __device__ __forceinline__ R divz(R a, R b) { return div(a, b); }
     static __device__ __forceinline__ R sqrtz(R x) { return sqrtp(x); }
     static __device__ __forceinline__ R divk(R a, R c, R, int) { return div(a, c); }
     static __device__ __forceinline__ R divk_in(R a, R c, R, int) { return div(a, c); }
-    static __device__ __forceinline__ R quot_in(R a, R y) { return quot(a, y); }
+    static __device__ __forceinline__ R quot_in(R a, Recip r) { return quot(a, r); }
     static __device__ __forceinline__ R e3_term(R num, R J, R yJ, int ok, R m) { return divk(num, J, yJ, ok) * m; }
-    static __device__ __forceinline__ R e4_term(R A, R T, R F, R e, R m) { return quot(quot(A, T) * F, e) * m; }
+    static __device__ __forceinline__ R e4_term(R A, Recip T, R F, Recip e, R m) { return quot(quot(A, T) * F, e) * m; }
     static __device__ __forceinline__ R qnan() { return __int_as_float(0x7fc00000); }
     /* settling velocity sqrt(A^2 + c) - A rewritten as c / (sqrt(A^2 + c) + A):
      * equal in exact arithmetic, but for fine classes (d = 2 um: A = 8.37,
@@ -450,6 +468,7 @@ struct PolicyF32 {
     /* DEP is stored in FP32 here: a reciprocal multiply is exact enough */
     static __device__ __forceinline__ double dep_of(double M, const DevParams &P) { return M * P.inv_rhos; }
 };
+typedef FormF32<false> PolicyF32;
 
 /* hllc of SWEHR.c:327-409 with the velocities already formed
  * (nl = normal/ul, tl = tangential/vl; both 0 for a dry side) and the left
@@ -1812,7 +1831,7 @@ __device__ __forceinline__ void tile_cell_pp(PP &pp, const DevParams &P, const D
     R vel1 = 0, vel2 = 0;
     if (h > hfilm) {
         const R manning = (h <= K.hc) ? own.roughness * pp.pow(pp.div(h, K.hc), K.dde) : own.roughness;
-        const R SFf = pp.div(manning * manning * gz * pp.sqrtp(hu * hu + hv * hv) * 1, pp.pow(h, R(2.333)));
+        const R SFf = pp.div(manning * manning * gz * pp.sqrtw(hu * hu + hv * hv) * 1, pp.pow(h, R(2.333)));
         const typename PP::Recip rf = PP::recip(1 + dtr * SFf), rh = PP::recip(h);
         hu = pp.quot(hu, rf);
         hv = pp.quot(hv, rf);
@@ -1820,7 +1839,7 @@ __device__ __forceinline__ void tile_cell_pp(PP &pp, const DevParams &P, const D
         vel2 = pp.quot(hv, rh);
     }
     R maxvel = (R)cellr[CR_MAXVEL * T_I * T_J + cs], maxdep = (R)cellr[CR_MAXDEP * T_I * T_J + cs];
-    const R vmag = pp.sqrtz(vel1 * vel1 + vel2 * vel2);
+    const R vmag = pp.sqrtw(vel1 * vel1 + vel2 * vel2);
     if (vmag > maxvel) maxvel = vmag;
     if (h > maxdep) maxdep = h;
     dst.h[q] = (RS)h;
