@@ -14,7 +14,12 @@ namespace swehr {
 
 int configure_batch_f32_t16(int max_classes, bool budget, BatchConfig &cfg)
 {
-    return FormLauncher<PolicyF32, float>::configure_batch(max_classes, budget, cfg, wide_kernels_f32_t16());
+    return FormLauncher<PolicyF32, float>::configure_batch(max_classes, budget, cfg);
+}
+
+int configure_batch_wide_f32_t16(int max_classes, bool budget, BatchConfig &cfg)
+{
+    return FormLauncher<PolicyF32, float>::configure_batch_wide(max_classes, budget, cfg, wide_kernels_f32_t16());
 }
 
 }  // namespace swehr

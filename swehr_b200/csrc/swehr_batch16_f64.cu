@@ -15,7 +15,12 @@ namespace swehr {
 
 int configure_batch_f64_t16(int max_classes, bool budget, BatchConfig &cfg)
 {
-    return FormLauncher<PolicyF64, double>::configure_batch(max_classes, budget, cfg, wide_kernels_f64_t16());
+    return FormLauncher<PolicyF64, double>::configure_batch(max_classes, budget, cfg);
+}
+
+int configure_batch_wide_f64_t16(int max_classes, bool budget, BatchConfig &cfg)
+{
+    return FormLauncher<PolicyF64, double>::configure_batch_wide(max_classes, budget, cfg, wide_kernels_f64_t16());
 }
 
 }  // namespace swehr

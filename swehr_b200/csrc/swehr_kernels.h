@@ -96,6 +96,10 @@ WideKernels wide_kernels_f64_t16();
 WideKernels wide_kernels_f32();
 WideKernels wide_kernels_f32_t16();
 
+int configure_batch_wide_f64(int max_classes, bool budget, BatchConfig &cfg);
+int configure_batch_wide_f64_t16(int max_classes, bool budget, BatchConfig &cfg);
+int configure_batch_wide_f32(int max_classes, bool budget, BatchConfig &cfg);
+int configure_batch_wide_f32_t16(int max_classes, bool budget, BatchConfig &cfg);
 int configure_batch_f64(int max_classes, bool budget, BatchConfig &cfg);
 int configure_batch_f32(int max_classes, bool budget, BatchConfig &cfg);
 /* the same kernels built for 16 x 16-cell tiles (cfg.tile_i = cfg.tile_j = 16) */

@@ -7,8 +7,10 @@
 #include <cuda_runtime.h>
 
 #include <cstring>
+#include <map>
 #include <mutex>
 #include <type_traits>
+#include <utility>
 
 #include "swehr_kernels.h"
 #include "swehr_tile.cuh"
@@ -56,15 +58,20 @@ static inline bool encode_planes(TensorMapEncodeFn enc, CUtensorMap *m, const vo
 
 /* A kernel's dynamic shared memory limit belongs to the process (on one
  * device), not to the simulation or pool that sets it: one that needs less,
- * made later, must leave the others' launches possible, so it is only raised. */
+ * made later, must leave the others' launches possible, so it is only raised.
+ * (The limit set is remembered: asking for a kernel's attributes costs a new
+ * simulation 0.4 ms a kernel.) */
 static inline cudaError_t raise_smem_limit(const void *fn, size_t bytes)
 {
     static std::mutex mu;
+    static std::map<std::pair<int, const void *>, size_t> limits;
+    int dev = 0;
+    const cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
     std::lock_guard<std::mutex> lock(mu);
-    cudaFuncAttributes a;
-    const cudaError_t e = cudaFuncGetAttributes(&a, fn);
-    if (e != cudaSuccess || (size_t)a.maxDynamicSharedSizeBytes >= bytes) return e;
-    return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    size_t &limit = limits[{dev, fn}];
+    if (limit < bytes) limit = bytes;
+    return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit);
 }
 
 inline namespace SWEHR_TILE_NS {
@@ -355,7 +362,9 @@ struct FormLauncher {
         return e;
     }
 
-    static cudaError_t configure_wide(int max_classes, bool budget, BatchConfig &cfg, const WideKernels &wide)
+    /* the wide kernels of a pool, once it has a scenario that needs them (to load
+     * them costs 50 ms) */
+    static int configure_batch_wide(int max_classes, bool budget, BatchConfig &cfg, const WideKernels &wide)
     {
         void *f = wide.update_batch[budget];
         cudaError_t e = raise_smem_limit(f, update_smem(max_classes, 0));
@@ -370,10 +379,10 @@ struct FormLauncher {
         if (e == cudaSuccess)
             e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&cfg.occ_wave_wide, wide.wave_batch, TILE_THREADS, wave_smem());
         if (cfg.occ_wave_wide < 1) cfg.occ_wave_wide = 1;
-        return e;
+        return (int)e;
     }
 
-    static int configure_batch(int max_classes, bool budget, BatchConfig &cfg, const WideKernels &wide)
+    static int configure_batch(int max_classes, bool budget, BatchConfig &cfg)
     {
         void *fw = (void *)k_wave_batch<PP, RS>;
         const size_t sw = wave_smem();
@@ -384,7 +393,6 @@ struct FormLauncher {
         if (cfg.occ_wave < 1) cfg.occ_wave = 1;
         e = configure_updates<false>(max_classes, budget, cfg.own);
         if (e == cudaSuccess && !budget) e = configure_updates<true>(max_classes, budget, cfg.common);
-        if (e == cudaSuccess) e = configure_wide(max_classes, budget, cfg, wide);
         if (e != cudaSuccess) return (int)e;
         cfg.fn_wave = fw;
         cfg.smem_wave = sw;

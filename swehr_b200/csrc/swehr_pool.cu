@@ -66,7 +66,9 @@ struct swehr_pool {
     DevParams common = {};
     bool has_common = false;
     int common_id = 0;
-    bool has_wide = false;               /* a running scenario's constants are out of the ordinary kernels' range */
+    /* a running scenario's constants are out of the ordinary kernels' range; the
+     * kernels of such pools are configured when the first one runs */
+    bool has_wide = false, wide_ready = false;
     cudaStream_t stream = nullptr;
     struct GraphEntry {
         size_t smem;
@@ -309,6 +311,15 @@ static int rebuild_table(swehr_pool *pl)
     pl->running_cells = cells;
     pl->max_s = max_s;
     pl->min_s = std::min(min_s, max_s);
+    if (wide && !pl->wide_ready) {
+        const bool b = pl->budget != 0, mixed = pl->precision == SWEHR_MIXED;
+        int ce = (mixed ? configure_batch_wide_f32 : configure_batch_wide_f64)(pl->max_classes, b, pl->shapes[0]);
+        if (!ce)
+            ce = (mixed ? configure_batch_wide_f32_t16 : configure_batch_wide_f64_t16)(pl->max_classes, b, pl->shapes[1]);
+        if (ce) return swehr_err(SWEHR_CUDA_ERROR, std::string("configure: ") + cudaGetErrorString((cudaError_t)ce));
+        pl->cfg = pl->shapes[pl->shape];
+        pl->wide_ready = true;
+    }
     pl->has_wide = wide;
     pl->has_common = same && k > 0 && !wide;
     if (pl->has_common && (pl->common_id == 0 || memcmp(&first, &pl->common, sizeof first) != 0)) {

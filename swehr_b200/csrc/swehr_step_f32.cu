@@ -49,7 +49,12 @@ int encode_tma_f32(const DevParams &P, const BufsT<float> &B, TmaMaps &tm)
 
 int configure_batch_f32(int max_classes, bool budget, BatchConfig &cfg)
 {
-    return FormLauncher<PolicyF32, float>::configure_batch(max_classes, budget, cfg, wide_kernels_f32());
+    return FormLauncher<PolicyF32, float>::configure_batch(max_classes, budget, cfg);
+}
+
+int configure_batch_wide_f32(int max_classes, bool budget, BatchConfig &cfg)
+{
+    return FormLauncher<PolicyF32, float>::configure_batch_wide(max_classes, budget, cfg, wide_kernels_f32());
 }
 
 }  // namespace swehr

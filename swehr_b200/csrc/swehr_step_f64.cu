@@ -66,7 +66,12 @@ int encode_tma_f64(const DevParams &P, const BufsT<double> &B, TmaMaps &tm)
 
 int configure_batch_f64(int max_classes, bool budget, BatchConfig &cfg)
 {
-    return FormLauncher<PolicyF64, double>::configure_batch(max_classes, budget, cfg, wide_kernels_f64());
+    return FormLauncher<PolicyF64, double>::configure_batch(max_classes, budget, cfg);
+}
+
+int configure_batch_wide_f64(int max_classes, bool budget, BatchConfig &cfg)
+{
+    return FormLauncher<PolicyF64, double>::configure_batch_wide(max_classes, budget, cfg, wide_kernels_f64());
 }
 
 }  // namespace swehr
