@@ -242,8 +242,12 @@ struct FastF64 {
     /* (u - chtemp) / c, to be added to h: below 2^-860 it is less than 2^-760 and
      * changes no h of middling size, so its bits do not matter there unless it is
      * SUMMED on its own, for the budget.  The deep branch has tested h as a
-     * divisor; in the shallow one u is 0 and chtemp an earlier class's */
-    __device__ __forceinline__ void shallow(R chtemp, R h) { ok &= !sw_tiny(chtemp) | sw_mid_pos(h); }
+     * divisor; in the shallow one u is 0 and chtemp an earlier class's, and a
+     * film that drains may be below zero */
+    __device__ __forceinline__ void shallow(R chtemp, R h)
+    {
+        ok &= sw_zero(chtemp) | (fabsf(sw_hi_float(h)) >= __int_as_float(SW_MID_LO));
+    }
     template <bool SUMMED>
     __device__ __forceinline__ R bulking(R a, R c, R yc, int)
     {
