@@ -3,21 +3,22 @@
  * branch, for operands of middling size, shared by the CUDA kernels and the
  * CPU tests.
  *
- * The compiler's double division and square root are each a short sequence
- * of fused multiply-adds, a range test and a call for the odd operands.  The
- * call ends a basic block, so two independent quotients of a cell never
- * overlap; a wet FP64 cell has about a hundred of them and its warp waits on
- * one dependent chain after the other.  Here the range test is a value that
- * the caller collects over a whole cell (FastF64 in swehr_tile.cuh), and a
- * cell with an odd operand is computed again with plain operators.
+ * A wet FP64 cell has about a hundred quotients and roots; written out as plain
+ * multiply-adds the independent ones overlap.  What they are not exact for is a
+ * value that the caller collects over a whole cell (FastF64 in swehr_tile.cuh),
+ * and a cell with such an operand is computed again with plain operators.
  * Measured on the 4096^2 domain in ponded flow (7 classes, B200): FP64
  * update 6.29 ms with the operators, 4.24 ms with these; a step on the 3 x 51
  * example 34 and 26 us.
  *
- * Method (P. W. Markstein, "Computation of elementary functions on the IBM
- * RISC System/6000 processor", IBM J. Res. Dev. 34, 1990): a reciprocal
- * estimate refined by Newton steps, q = a y, and one correction by the exact
- * remainder r = a - b q.  Why the result is the rounded quotient, for
+ * Method.  A reciprocal estimate y of 1/b with residual e = 1 - b y is refined by
+ * y (1 + e + e^2), an estimate y of x^(-1/2) with e = 1 - x y^2 by
+ * y (1 + e/2 + 3 e^2/8): the third-order iterations of the family of A. S.
+ * Householder ("The Numerical Treatment of a Single Nonlinear Equation", 1970),
+ * the binomial series of 1/(1 - e) and (1 - e)^(-1/2) cut after the square.  The
+ * quotient is q = a y corrected by the exact remainder r = a - b q (P. W.
+ * Markstein, "Computation of elementary functions on the IBM RISC System/6000
+ * processor", IBM J. Res. Dev. 34, 1990).  Why the result is the rounded quotient, for
  * 1 <= b < 2 and y the double next to 1/b, i.e. within 2^-54 of it (a scaling
  * by powers of two changes nothing while no step leaves the normal range):
  *   - away from the midpoint of two neighbouring doubles q + r y rounds

@@ -78,16 +78,18 @@ inline namespace SWEHR_TILE_NS {
 
 /* Tiles per SM up to which a domain is stepped by k_run_tile.  Measured (B200,
  * 7 classes, ponded flow, us a step, two kernels and many steps a launch):
- *   tiles      1     64    175    384    750   1536   65536
- *   FP64    35.0   32.4   33.7   48.6   74.0  139.1    4228
- *           32.3   28.2   31.4   47.1   71.7  141.4    4346
- *   mixed   22.5   21.2   23.8   26.2   37.1   60.0    1858
- *           19.9   17.8   20.3   23.1   33.7   61.6    1884
+ *   tiles      1     64    175    384    750    969   1280   1536   2816
+ *   FP64    35.1   32.0   33.2   48.8   71.6   99.5  121.8  138.2  219.7
+ *           32.3   27.4   29.4   48.1   70.1   97.7  124.4  143.7  221.2
+ *   mixed   22.3   22.0   23.3   25.5   35.0   42.6   48.7   60.1   94.8
+ *           19.2   18.4   20.7   23.2   33.5   46.2   45.7   60.5   98.7
  * What a launch saves is the same at any size, but the wave pass runs at the
  * update's occupancy and a block's tiles wait for the slowest block at every
- * barrier.  With interior solid cells (the wave pass takes one cell a thread:
- * 517 x 389, 10 classes 134 and 150 us) and with budgets (block 0 folds the
- * sums between two barriers: 200 x 50 mixed 40 and 47 us) two kernels stay. */
+ * barrier; from about 970 tiles (6.5 per SM) it depends on the last round's
+ * size which is faster.  With interior solid cells (the wave pass takes one cell
+ * a thread: 517 x 389, 10 classes 134 and 150 us) and with budgets (block 0
+ * folds the sums between two barriers: 200 x 50 mixed 40 and 47 us) two kernels
+ * stay. */
 #define RUN_TILES_PER_SM 4
 
 template <class PP, class RS>

@@ -69,7 +69,7 @@ extern "C" int swehr_probe_fp64_peak(double *tflops)
 }
 
 /* swehr_probe_ieee: the branch-free sequences of swehr_ieee.h beside the
- * compiler's operators and the plain bodies of swehr_math.h, element by
+ * plain operators and the bodies of swehr_math.h, element by
  * element, for the tests.  op: 0 a/b, 1 root of a, 2 exp(a), 3 a^b, 4
  * cos(atan a), 5 a/b of small a, 6 a/b of any small a, 7 exp(a) down to zero;
  * host arrays of n doubles.  refused: 1 where the operands are

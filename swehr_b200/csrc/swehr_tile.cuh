@@ -86,7 +86,7 @@ struct PolicyF64 {
     static constexpr int kBudgetMinBlocks = 2; /* ... with budgets */
     static constexpr int kBatchMinBlocks = 2; /* ... and the batched update kernel */
     static constexpr int kCommonMinBlocks = 2; /* ... of an exact class count with common constants */
-    static constexpr bool kRollClasses = true;    /* one division and exp sequence in the code, not eight */
+    static constexpr bool kRollClasses = true;    /* its cells are rare (computed again) or wide: one body for any count */
     typedef double Recip;
     static __device__ __forceinline__ R recip(R b) { return b; }
     static __device__ __forceinline__ R quot(R a, R b) { return a / b; }
@@ -127,7 +127,7 @@ struct PolicyF64 {
         if (x == 0) return R(0);
         return sqrtp(x);
     }
-    /* sqrtp of squared momenta and velocities */
+    /* sqrtp, in FormF32 without its loss below 1e-19 */
     static __device__ __forceinline__ R sqrtw(R x) { return sqrtz(x); }
     static __device__ __forceinline__ R qnan() { return __longlong_as_double(0x7ff8000000000000LL); }
     /* a / c for a constant divisor c in [2^-100, 2^100] whose correctly
@@ -406,9 +406,9 @@ struct FormF32 {
      * same value. */
     static __device__ __forceinline__ R sqrtw(R x) { return x > 0.f ? __fmul_rn(x, rsqrtf(x)) : 0.f; }
     /* ... without subnormal operands: a root below 1e-19 comes out nearer to zero.
-     * It is a slope, is added to the root of a film's depth, or goes into a stream
-     * power, its cube, that is zero either way; squared velocities and momenta take
-     * sqrtw (4096^2 in ponded flow: +0.4 %) */
+     * It is a slope, is added to the root of a film's depth, or is a discharge
+     * below 1e-19 m2/s in the stream power, its cube; the velocities and momenta
+     * that are results take sqrtw (4096^2 in ponded flow: +0.4 %) */
     static __device__ __forceinline__ R sqrtp(R x)
     {
         if constexpr (WIDE) return sqrtw(x);
