@@ -31,7 +31,7 @@ typedef enum swehr_status {
     SWEHR_OK = 0,
     SWEHR_CFL_ERROR = 1,    /* Courant number > 1 (SWEHR.c:1412-1413); the step completes, then stepping stops */
     SWEHR_NAN = 2,          /* non-finite water depth detected (only when params.stop_on_nan) */
-    SWEHR_TIMEOUT = 3,      /* host wall-clock limit of swehr_advance reached */
+    SWEHR_TIMEOUT = 3,      /* a bounded wait on the device gave up; no further step of this context is taken */
     SWEHR_CUDA_ERROR = 4,   /* a CUDA runtime call failed; see swehr_last_error() */
     SWEHR_INVALID = 5,      /* bad argument (sizes, NULL pointers, class count, ...) */
     SWEHR_OOM = 6,          /* device allocation failed / pool budget exceeded */
