@@ -122,3 +122,24 @@ def test_a_step_of_the_recession_takes_no_longer_than_one_of_the_rain(budget):
         after = s.advance(max_steps=700)
     ratio = (after.device_ms / after.steps_this_call) / (rain.device_ms / rain.steps_this_call)
     assert ratio < 1.35, ratio
+
+
+@pytest.mark.parametrize("timed", [False, True], ids=["", "timed"])
+@pytest.mark.parametrize("kind", ["storm", "film"])
+def test_exponents_below_minus_700_equal_the_oracle(kind, timed):
+    """Cells up to 75 radii from a storm's centre, and classes that settle out of a
+    film of 1e-8 m within a step: exp through the subnormals to zero."""
+    from harness import CLASS_FIELDS, STATE_FIELDS, OracleRun, compare
+    from swehr_b200.lib import Simulation
+    over = dict(hfilm=1e-8) if kind == "film" else dict(storm_peak=2e-4, storm_radius=0.2, storm_x0=5.0, storm_y0=6.0,
+                                                         storm_vx=0.05, storm_vy=0.02)
+    case = W.tiny_case(nx=20, ny=40, S=4, seed=12, rain_mmh=200.0, tend=1e3, **over)
+    o = OracleRun(case, "shim")
+    with Simulation(case) as s:
+        s.set_timing(timed)
+        for _ in range(4):
+            o.advance(max_steps=60)
+            pr = s.advance(max_steps=60)
+            assert pr.t == o.t
+            res = compare(s.fields(), o.fields(), STATE_FIELDS + CLASS_FIELDS)
+            assert all(v[2] for v in res.values()), {k: v for k, v in res.items() if not v[2]}

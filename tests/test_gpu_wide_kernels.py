@@ -145,3 +145,19 @@ def test_such_a_run_forms_each_cell_once():
             pr = s.advance(max_steps=700)
             us.append(pr.device_ms / pr.steps_this_call)
     assert us[1] < 2.0 * us[0], us
+
+
+@pytest.mark.parametrize("precision", [FP64, MIXED], ids=["fp64", "mixed"])
+def test_slabs_of_such_a_run_equal_the_whole(precision):
+    from swehr_b200.lib import Simulation, SlabDomain
+    case = _case(4, nx=26, ny=40, hfilm=0.0, **OUT)
+    names = ("h", "hu", "hv", "z", "vinf", "totsed", "U", "M")
+    with Simulation(case, precision=precision) as s:
+        pw = s.advance(max_steps=120)
+        want = s.fields(names)
+    with SlabDomain(case, 3, precision) as d:
+        d.step(120)
+        ps, got = d.progress(), d.fields(names)
+    assert (ps.t, ps.dt, ps.steps) == (pw.t, pw.dt, 120)
+    for n in names:
+        assert np.array_equal(got[n], want[n], equal_nan=True), n
