@@ -85,8 +85,8 @@ inline namespace SWEHR_TILE_NS {
  *           19.2   18.4   20.7   23.2   33.5   46.2   45.7   60.5   98.7
  * What a launch saves is the same at any size, but the wave pass runs at the
  * update's occupancy and a block's tiles wait for the slowest block at every
- * barrier; from about 970 tiles (6.5 per SM) it depends on the last round's
- * size which is faster.  With interior solid cells (the wave pass takes one cell
+ * barrier; from about 970 tiles (6.5 per SM) it depends on how full the last
+ * wave of tiles is which is faster.  With interior solid cells (the wave pass takes one cell
  * a thread: 517 x 389, 10 classes 134 and 150 us) and with budgets (block 0
  * folds the sums between two barriers: 200 x 50 mixed 40 and 47 us) two kernels
  * stay. */
